@@ -221,8 +221,8 @@ __global__ void __launch_bounds__(1 << LOG_NT, 1)
 #pragma unroll
         for (int e = 0; e < E; e++)
             v[e] = Stage<R>::read(buf, T, tp | (e << S0));
-        // levels LT-1 .. 0 of phase 2^K, direction fixed for the tile (the
-        // first transpose's barrier also ends the reads of the staged tile)
+        __syncthreads(); // the staged tile is overwritten by the first transpose
+        // levels LT-1 .. 0 of phase 2^K, direction fixed for the tile
         const bool asc_c = ((cta_bits >> K) & 1) == 0;
         int s = S0;
         int b = LT - 1;
