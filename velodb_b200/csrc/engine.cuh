@@ -35,18 +35,6 @@ namespace velo {
 // of y - x (limb 0 least significant); one carry chain, no branches
 // ---------------------------------------------------------------------------
 
-__device__ __forceinline__ uint32_t gt_mask2(uint32_t x0, uint32_t x1, uint32_t y0, uint32_t y1)
-{
-    uint32_t r;
-    asm("{\n\t.reg .u32 t;\n\t"
-        "sub.cc.u32 t, %1, %3;\n\t"
-        "subc.cc.u32 t, %2, %4;\n\t"
-        "subc.u32 %0, 0, 0;\n\t}"
-        : "=r"(r)
-        : "r"(y0), "r"(y1), "r"(x0), "r"(x1));
-    return r;
-}
-
 __device__ __forceinline__ uint32_t gt_mask3(uint32_t x0, uint32_t x1, uint32_t x2, uint32_t y0, uint32_t y1,
                                              uint32_t y2)
 {
@@ -83,9 +71,7 @@ __device__ __forceinline__ uint32_t hi32(uint64_t x) { return (uint32_t)(x >> 32
 template <int KW>
 __device__ __forceinline__ uint32_t key_gt_mask(const uint64_t* x, const uint64_t* y)
 {
-    if constexpr (KW == 1) {
-        return gt_mask2(lo32(x[0]), hi32(x[0]), lo32(y[0]), hi32(y[0]));
-    } else if constexpr (KW == 2) {
+    if constexpr (KW == 2) {
         return gt_mask4(lo32(x[1]), hi32(x[1]), lo32(x[0]), hi32(x[0]), lo32(y[1]), hi32(y[1]), lo32(y[0]), hi32(y[0]));
     } else {
         // lexicographic from the most significant word
@@ -165,17 +151,52 @@ struct MadSwap {
     }
 };
 
+// The exchange with one select and two multiply-adds a register: with
+// t = a + b, a' = x ? b : a (ALU pipe), b' = t - a' (FMA pipe, mod 2^32).
+// One instruction fewer than MadSwap and the pipes' shares nearly even; `one`
+// is 1 known only at run time (CTAs are one-dimensional), so that the sums
+// stay multiply-adds.
+struct AddSwap {
+    uint32_t one, neg;
+    bool x;
+    __device__ __forceinline__ explicit AddSwap(bool x_) : one(blockDim.y), neg(0u - blockDim.y), x(x_) { }
+    __device__ __forceinline__ void operator()(uint32_t& a, uint32_t& b) const
+    {
+        const uint32_t t = a * one + b;
+        const uint32_t na = x ? b : a;
+        b = na * neg + t;
+        a = na;
+    }
+    __device__ __forceinline__ void operator()(uint64_t& a, uint64_t& b) const
+    {
+        uint32_t al = lo32(a), ah = hi32(a), bl = lo32(b), bh = hi32(b);
+        (*this)(al, bl);
+        (*this)(ah, bh);
+        a = ((uint64_t)ah << 32) | al;
+        b = ((uint64_t)bh << 32) | bl;
+    }
+};
+
 // how a RowRec compares its key
 enum KeyMode : int {
     KEY_MASKED = 0, // words 0..KW-1, each AND-ed with Cols::mask (runtime)
     KEY_FULL = 1,   // words 0..KW-1 as they are
     KEY_HI32 = 2,   // the high 32 bits of word 0 only (KW == 1)
+    KEY_HI96 = 3,   // word 0 and the high 32 bits of word 1 (KW == 2, strict)
 };
 
-// (u64 key, u32 payload), ordered lexicographically on both (plain sort rows).
-// Every field is compared, so the sorted output is unique.  Registers hold
-// the key as two 32-bit halves so exchanges never repack 64-bit values.
-struct RowKP {
+// 12-byte rows: u64 key, u32 payload.  Registers hold the key as two 32-bit
+// halves so exchanges never repack 64-bit values.  Ordered as CM says:
+//   K12_ALL      key, then payload (plain sort rows): every field is compared,
+//                so the sorted output is unique
+//   K12_KEY_TAG  key, then the top bit of the payload, not strict
+//   K12_KEY      the key alone, strict; the rows of descending blocks are
+//                complemented (Flip), so one compare serves both directions
+// As compaction rows they are marked by a clear top bit of the key.
+enum K12Order : int { K12_ALL = 0, K12_KEY_TAG = 1, K12_KEY = 2 };
+
+template <int CM>
+struct RowK12 {
     uint32_t kl, kh, p;
     struct Cols {
         uint64_t* k;
@@ -183,53 +204,129 @@ struct RowKP {
     };
     static constexpr int SMEM_BYTES = 16; // one 16-byte slot per row (kl, kh, p, unused)
     static constexpr int SWZ_BITS = 3;
-    __device__ __forceinline__ static RowKP load(const Cols& c, size_t g)
+    __device__ __forceinline__ static RowK12 load(const Cols& c, size_t g)
     {
         VELO_TRACE_AT(TS_ROW_LOAD, c.k + g);
         const uint64_t k = __ldcg(c.k + g);
-        return RowKP { lo32(k), hi32(k), __ldcg(c.p + g) };
+        return RowK12 { lo32(k), hi32(k), __ldcg(c.p + g) };
     }
-    __device__ __forceinline__ static void store(const Cols& c, size_t g, const RowKP& r)
+    __device__ __forceinline__ static void store(const Cols& c, size_t g, const RowK12& r)
     {
         VELO_TRACE_AT(TS_ROW_STORE, c.k + g);
         c.k[g] = ((uint64_t)r.kh << 32) | r.kl;
         c.p[g] = r.p;
     }
-    __device__ __forceinline__ static RowKP pad(const Cols&) { return RowKP { ~0u, ~0u, ~0u }; }
-    __device__ __forceinline__ static void sstore(char* sm, int, int i, const RowKP& r)
+    __device__ __forceinline__ static RowK12 pad(const Cols&) { return RowK12 { ~0u, ~0u, ~0u }; }
+    __device__ __forceinline__ static void sstore(char* sm, int, int i, const RowK12& r)
     {
         reinterpret_cast<uint4*>(sm)[i] = make_uint4(r.kl, r.kh, r.p, 0u);
     }
     // the same at byte offset `b` = slot * SLOT_BYTES
     static constexpr int SLOT_BYTES = 16;
-    __device__ __forceinline__ static void sstore_b(char* sm, int, uint32_t b, const RowKP& r)
+    __device__ __forceinline__ static void sstore_b(char* sm, int, uint32_t b, const RowK12& r)
     {
         *reinterpret_cast<uint4*>(sm + b) = make_uint4(r.kl, r.kh, r.p, 0u);
     }
-    __device__ __forceinline__ static RowKP sload_b(const char* sm, int, uint32_t b)
+    __device__ __forceinline__ static RowK12 sload_b(const char* sm, int, uint32_t b)
     {
         const uint4 x = *reinterpret_cast<const uint4*>(sm + b);
-        return RowKP { x.x, x.y, x.z };
+        return RowK12 { x.x, x.y, x.z };
     }
-    __device__ __forceinline__ static RowKP sload(const char* sm, int, int i)
+    __device__ __forceinline__ static RowK12 sload(const char* sm, int, int i)
     {
         const uint4 x = reinterpret_cast<const uint4*>(sm)[i];
-        return RowKP { x.x, x.y, x.z };
+        return RowK12 { x.x, x.y, x.z };
     }
-    __device__ __forceinline__ static bool swap_pred(const RowKP& a, const RowKP& b, bool desc, const Cols&)
+    __device__ __forceinline__ static bool swap_pred(const RowK12& a, const RowK12& b, bool desc, const Cols&)
     {
-        return (gt_mask3(a.p, a.kl, a.kh, b.p, b.kl, b.kh) != 0u) != desc;
+        if constexpr (CM == K12_KEY) {
+            return (((uint64_t)a.kh << 32) | a.kl) > (((uint64_t)b.kh << 32) | b.kl);
+        } else if constexpr (CM == K12_KEY_TAG) {
+            // the lowest limb borrows iff a has the tag and b has not
+            return (gt_mask3(a.p & 0x80000000u, a.kl, a.kh, b.p | 0x7FFFFFFFu, b.kl, b.kh) != 0u) != desc;
+        } else {
+            return (gt_mask3(a.p, a.kl, a.kh, b.p, b.kl, b.kh) != 0u) != desc;
+        }
     }
-    // exchange a and b when x, in place: key halves on the multiply-add
-    // pipe, payload by selects
-    __device__ __forceinline__ static void cswap(RowKP& a, RowKP& b, bool x)
+    // exchange a and b when x, in place (2^24-row tile sort 538 -> 507 us,
+    // merge 104.9 -> 104.3 us against two halves as MadSwap and one by selects)
+    __device__ __forceinline__ static void cswap(RowK12& a, RowK12& b, bool x)
     {
-        const MadSwap m(x);
+        const AddSwap m(x);
         m(a.kl, b.kl);
         m(a.kh, b.kh);
-        xsel(x, a.p, b.p);
+        m(a.p, b.p);
     }
-    __device__ __forceinline__ static bool marked(const RowKP&) { return false; }
+    __device__ __forceinline__ static void flip(RowK12& r, uint32_t m)
+    {
+        r.kl ^= m;
+        r.kh ^= m;
+    }
+    __device__ __forceinline__ static bool marked(const RowK12& r) { return (r.kh >> 31) == 0; }
+};
+using RowKP = RowK12<K12_ALL>;
+
+// Types that sort with one strict compare: while a block descends its keys are
+// held complemented, where the ascending compare swaps exactly the pairs that
+// the descending one swaps on the plain keys (equal keys stay in both).
+template <class R>
+struct Flip {
+    static constexpr bool on = false;
+};
+template <>
+struct Flip<RowK12<K12_KEY>> {
+    static constexpr bool on = true;
+};
+
+// Two independent 16-bit keys a row, each lane sorted on its own: an exchange
+// is one packed minimum and one packed maximum for two keys.  The direction
+// is the only decision, so swap_pred hands it to cswap.
+struct RowU2 {
+    uint32_t k;
+    struct Cols {
+        uint32_t* k;
+    };
+    static constexpr int SMEM_BYTES = 4;
+    static constexpr int SWZ_BITS = 5;
+    static constexpr int SLOT_BYTES = 4;
+    __device__ __forceinline__ static RowU2 load(const Cols& c, size_t g)
+    {
+        VELO_TRACE_AT(TS_ROW_LOAD, c.k + g);
+        return RowU2 { __ldcg(c.k + g) };
+    }
+    __device__ __forceinline__ static void store(const Cols& c, size_t g, const RowU2& r)
+    {
+        VELO_TRACE_AT(TS_ROW_STORE, c.k + g);
+        c.k[g] = r.k;
+    }
+    __device__ __forceinline__ static RowU2 pad(const Cols&) { return RowU2 { ~0u }; }
+    __device__ __forceinline__ static void sstore(char* sm, int, int i, const RowU2& r)
+    {
+        reinterpret_cast<uint32_t*>(sm)[i] = r.k;
+    }
+    __device__ __forceinline__ static RowU2 sload(const char* sm, int, int i)
+    {
+        return RowU2 { reinterpret_cast<const uint32_t*>(sm)[i] };
+    }
+    __device__ __forceinline__ static void sstore_b(char* sm, int, uint32_t b, const RowU2& r)
+    {
+        *reinterpret_cast<uint32_t*>(sm + b) = r.k;
+    }
+    __device__ __forceinline__ static RowU2 sload_b(const char* sm, int, uint32_t b)
+    {
+        return RowU2 { *reinterpret_cast<const uint32_t*>(sm + b) };
+    }
+    __device__ __forceinline__ static bool swap_pred(const RowU2&, const RowU2&, bool desc, const Cols&)
+    {
+        return desc;
+    }
+    __device__ __forceinline__ static void cswap(RowU2& a, RowU2& b, bool desc)
+    {
+        const uint32_t lo = __vminu2(a.k, b.k), hi = __vmaxu2(a.k, b.k);
+        a.k = desc ? hi : lo;
+        b.k = desc ? lo : hi;
+    }
+    __device__ __forceinline__ static bool marked(const RowU2&) { return false; }
 };
 
 // (u64 key, u32 payload, u8 mark): compaction rows; ordered on (key, payload)
@@ -398,6 +495,15 @@ struct RowRec {
     // selects (W = 1: the high half only)
     __device__ __forceinline__ static void cswap(RowRec& a, RowRec& b, bool x)
     {
+        if constexpr (W == 2 && (KM == KEY_FULL || KM == KEY_HI96)) {
+            // whole-word keys (the join union): 2^23-row merge 69.9 -> 62.2 us,
+            // tile sort 318 -> 314 us; with a 32-bit key the tile sort's
+            // three-CTA form spills (281 -> 347 us)
+            const AddSwap m(x);
+            m(a.w[0], b.w[0]);
+            m(a.w[1], b.w[1]);
+            return;
+        }
         const MadSwap mad(x);
         if constexpr (W == 1) {
             uint32_t al = lo32(a.w[0]), ah = hi32(a.w[0]), bl = lo32(b.w[0]), bh = hi32(b.w[0]);
@@ -415,39 +521,28 @@ struct RowRec {
             }
         }
     }
-    // the same exchange with one more 32-bit half on the multiply-add pipe
-    // (two-word records compared on a whole word: three of four halves);
-    // levels alternate between the two forms so that the ALU pipe, which
-    // also carries the 64-bit compare, and the multiply-add pipe stay about
-    // even (join union sort 1.92 -> 1.87 ms; no change with a 32-bit key)
-    __device__ __forceinline__ static void cswap_fma(RowRec& a, RowRec& b, bool x)
-    {
-        if constexpr (W == 2 && KM != KEY_HI32) {
-            const MadSwap mad(x);
-            mad(a.w[0], b.w[0]);
-            uint32_t al = lo32(a.w[1]), ah = hi32(a.w[1]), bl = lo32(b.w[1]), bh = hi32(b.w[1]);
-            mad(al, bl);
-            xsel(x, ah, bh);
-            a.w[1] = ((uint64_t)ah << 32) | al;
-            b.w[1] = ((uint64_t)bh << 32) | bl;
-        } else {
-            cswap(a, b, x);
-        }
-    }
     __device__ __forceinline__ static bool swap_pred(const RowRec& a, const RowRec& b, bool desc, const Cols& c)
     {
         if constexpr (KM == KEY_HI32) {
             const uint32_t x = hi32(a.w[0]), y = hi32(b.w[0]);
             if constexpr (STRICT)
-                return desc ? (x < y) : (x > y);
+                return x > y; // Flip
             else
                 return (x > y) != desc;
         }
+        if constexpr (KM == KEY_HI96)
+            return gt_mask3(hi32(a.w[1]), lo32(a.w[0]), hi32(a.w[0]), hi32(b.w[1]), lo32(b.w[0]), hi32(b.w[0])) != 0u;
         uint64_t ka[KW], kb[KW];
 #pragma unroll
         for (int x = 0; x < KW; x++) {
             ka[x] = KM == KEY_FULL ? a.w[x] : (a.w[x] & c.mask[x]);
             kb[x] = KM == KEY_FULL ? b.w[x] : (b.w[x] & c.mask[x]);
+        }
+        if constexpr (KW == 1) {
+            if constexpr (STRICT)
+                return desc ? ka[0] < kb[0] : ka[0] > kb[0];
+            else
+                return (ka[0] > kb[0]) != desc;
         }
         if constexpr (STRICT) {
             const uint32_t gt = key_gt_mask<KW>(ka, kb);
@@ -455,6 +550,16 @@ struct RowRec {
             return (desc ? lt : gt) != 0u;
         } else {
             return (key_gt_mask<KW>(ka, kb) != 0u) != desc;
+        }
+    }
+    __device__ __forceinline__ static void flip(RowRec& r, uint32_t m)
+    {
+        if constexpr (KM == KEY_HI32) {
+            r.w[0] ^= (uint64_t)m << 32;
+        } else {
+            r.w[0] ^= ((uint64_t)m << 32) | m;
+            if constexpr (W > 1)
+                r.w[1] ^= (uint64_t)m << 32;
         }
     }
     __device__ __forceinline__ static RowRec select(bool cnd, const RowRec& a, const RowRec& b)
@@ -479,18 +584,15 @@ struct RowRec {
     }
 };
 
-// compare-exchange form of a level: ALT = 1 takes a record's cswap_fma where
-// it has one
-template <class R, int ALT>
-struct Cswap {
-    __device__ __forceinline__ static void run(R& a, R& b, bool x) { R::cswap(a, b, x); }
+// strict records keyed on the high half of a word, the low half of the last
+// one being payload
+template <int W>
+struct Flip<RowRec<W, 1, true, KEY_HI32>> {
+    static constexpr bool on = true;
 };
-template <int W, int KW, bool S, int KM>
-struct Cswap<RowRec<W, KW, S, KM>, 1> {
-    __device__ __forceinline__ static void run(RowRec<W, KW, S, KM>& a, RowRec<W, KW, S, KM>& b, bool x)
-    {
-        RowRec<W, KW, S, KM>::cswap_fma(a, b, x);
-    }
+template <>
+struct Flip<RowRec<2, 2, true, KEY_HI96>> {
+    static constexpr bool on = true;
 };
 
 template <class R>

@@ -20,20 +20,26 @@ __global__ void __launch_bounds__(256) k_count_marks(typename R::Cols c, size_t 
 
 __global__ void k_scan_tiles(const uint32_t* counts, int ntiles, uint32_t* prefix, uint64_t* d_count);
 
-// Bitonic pass list for Np = 2^logN rows and tile 2^LT; Lmax fused levels.
+// Passes of one merge phase 2^K over blocks of 2^logB rows (levels
+// 2^(logB - 1) .. 1), logB >= LT; Lmax fused levels.
+inline void plan_merge(int logB, int LT, int Lmax, int K, std::vector<NetPass>& out)
+{
+    int b = logB - 1;
+    while (b >= LT) {
+        int L = b - LT + 1;
+        L = L < Lmax ? L : Lmax;
+        out.push_back(NetPass { P_SORT_GLOBAL, K, b, L });
+        b -= L;
+    }
+    out.push_back(NetPass { P_SORT_MERGE, K, 0, 0 });
+}
+
+// Bitonic pass list for Np = 2^logN rows and tile 2^LT.
 inline void plan_sort(int logN, int LT, int Lmax, std::vector<NetPass>& out)
 {
     out.push_back(NetPass { P_SORT_TILE, logN < LT ? logN : LT, 0, 0 });
-    for (int K = LT + 1; K <= logN; K++) {
-        int b = K - 1;
-        while (b >= LT) {
-            int L = b - LT + 1;
-            L = L < Lmax ? L : Lmax;
-            out.push_back(NetPass { P_SORT_GLOBAL, K, b, L });
-            b -= L;
-        }
-        out.push_back(NetPass { P_SORT_MERGE, K, 0, 0 });
-    }
+    for (int K = LT + 1; K <= logN; K++)
+        plan_merge(K, LT, Lmax, K, out);
 }
 
 // ORCompact pass list (levels bottom-up).
@@ -114,6 +120,11 @@ inline velo_status launch_sort_records(const typename R::Cols& c, int logN, cuda
     plan_sort(logN, 12, 8, passes);
     return launch_net12<R>(c, NetGeom { (size_t)1 << logN, logN, 0 }, passes, nullptr, st);
 }
+
+// Bitonic sort of the rows [0, n) of a key-payload array of 2^logN rows (the
+// default tile of velo_osort_kp); rows n .. end of the last tile become
+// padding, with `fill` all rows from n on.  Defined in network.cu.
+velo_status sort_kp_rows(const RowKP::Cols& c, size_t n, int logN, int fill, cudaStream_t st);
 
 template <class R>
 inline velo_status launch_count_scan(const typename R::Cols& c, size_t n, int logN, int LT, uint32_t* counts,

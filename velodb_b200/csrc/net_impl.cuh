@@ -39,6 +39,11 @@ struct NetWide<RowRec<2, 1, S, KEY_FULL>> {
     static constexpr bool ok = false;
     static constexpr bool ok_global = true;
 };
+template <>
+struct NetWide<RowRec<2, 2, true, KEY_HI96>> {
+    static constexpr bool ok = false;
+    static constexpr bool ok_global = true;
+};
 template <class R, int LOG_NT>
 constexpr bool net_has_wide() { return LOG_NT <= 8 && NetWide<R>::ok; }
 template <class R, int LOG_NT>
@@ -84,9 +89,13 @@ template <class R>
 struct RowBytes {
     static constexpr int value = R::WORDS * 8;
 };
-template <>
-struct RowBytes<RowKP> {
+template <int CM>
+struct RowBytes<RowK12<CM>> {
     static constexpr int value = 12;
+};
+template <>
+struct RowBytes<RowU2> {
+    static constexpr int value = 4;
 };
 template <>
 struct RowBytes<RowKPM> {
@@ -170,7 +179,7 @@ inline unsigned merge_pipe_grid(const typename R::Cols& c, size_t ntiles, cudaSt
 #ifdef VELO_TRACE
     return 0;
 #else
-    if constexpr (!pipe_capable<R, LOG_NT, LOG_E>()) {
+    if constexpr (!pipe_capable<R, LOG_NT, LOG_E>() || Flip<R>::on) {
         return 0;
     } else {
         if (!merge_pipe_on() || ntiles < 2 || !Stage<R>::aligned(c))
@@ -214,7 +223,7 @@ velo_status launch_net(const typename R::Cols& c, const NetGeom& g, const std::v
     // without the tile-sort code: join union merges 76.5 -> 73.8 us, group-by
     // merges 65.6 -> 62.1 us; key-payload rows keep the shared kernel (2^24
     // merges 111.1 -> 112.9 us with the split)
-    constexpr bool split_merge = !std::is_same_v<R, RowKP>;
+    constexpr bool split_merge = sizeof(R) != 12;
     // the merges of records that keep a two-CTA tile sort (compared on a
     // whole word) take the global kernel's three-CTA budget from 2^21 rows:
     // 80 registers, a few spilled, join union merges 73.9 -> 71.6 us
@@ -247,28 +256,30 @@ velo_status launch_net(const typename R::Cols& c, const NetGeom& g, const std::v
         return rc;
     const int lt = N::LT;
     const size_t grid = g.logN > lt ? ((size_t)1 << (g.logN - lt)) : 1;
+    const bool whole = g.m == (size_t)1 << g.logN; // not trimmed
     // the first pass follows whatever ran before it; the later ones overlap
     // their launch with the tail of the previous pass
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
-    const unsigned pipe_grid = compact ? 0u : merge_pipe_grid<R, LOG_NT, LOG_E>(c, grid, st);
+    // (the load tunes work on whole networks)
+    const unsigned pipe_grid = compact || !whole ? 0u : merge_pipe_grid<R, LOG_NT, LOG_E>(c, grid, st);
     int* pipe_fault = nullptr;
     if (pipe_grid)
         VELO_CUDA_TRY(cudaGetSymbolAddress((void**)&pipe_fault, s_pipe_fault), "cudaGetSymbolAddress");
-    const bool tma = !compact && tma_passes_on<R, LOG_NT, LOG_E>(c);
+    const bool tma = !compact && whole && tma_passes_on<R, LOG_NT, LOG_E>(c);
     int* tma_fault = tma ? tma_fault_word() : nullptr;
     PassTimer timer(st, passes.size());
     for (size_t i = 0; i < passes.size(); i++) {
         cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3((unsigned)grid);
+        cfg.gridDim = dim3((unsigned)net_pass_tiles(g, passes[i], lt));
         cfg.blockDim = dim3(1u << LOG_NT);
         cfg.dynamicSmemBytes = smem;
         cfg.stream = st;
         cfg.attrs = attr;
         cfg.numAttrs = (i > 0 && !timer.on()) ? 1 : 0;
         if (pipe_grid && passes[i].kind == P_SORT_MERGE) {
-            if constexpr (pipe_capable<R, LOG_NT, LOG_E>()) {
+            if constexpr (pipe_capable<R, LOG_NT, LOG_E>() && !Flip<R>::on) {
                 cfg.gridDim = dim3(pipe_grid);
                 cfg.blockDim = dim3(1u << PIPE_LOG_NT);
                 cfg.dynamicSmemBytes = 2 * pipe_buf_bytes<R, PIPE_LOG_NT, PIPE_LOG_E>();

@@ -27,10 +27,39 @@ enum PassKind : int {
     P_COMPACT_GLOBAL = 4,
 };
 
+// Rows of a network.  Trimmed (m < 2^logN): rows m .. 2^logN - 1 are padding
+// that sorts last, and the passes leave them out instead of sorting them.
+// That is the network with the merge directions counted from the last block:
+// block i of phase 2^K ascends iff bit K of its rows equals bit K of m - 1,
+// so neighbouring blocks still run in opposite directions, and the one block
+// of each phase that reaches into the padding ascends: its padding, the
+// largest rows, stays at its end and no exchange moves it (an ascending
+// exchange only swaps when the lower row is strictly larger).  The order of
+// equal rows differs from the padded network's, so a caller trims only where
+// equal rows are the same in every bit or their order is not seen.
 struct NetGeom {
-    size_t n;  // real rows (public)
-    int logN;  // log2 of the padded size
-    int pad_;
+    size_t n;    // real rows (public)
+    int logN;    // log2 of the padded size
+    int fill;    // trimmed: the tile pass writes padding to rows m .. 2^logN - 1
+    size_t m;    // rows the passes work on, a multiple of the tile or 2^logN
+    size_t dirx; // XORed into the row index that gives a merge its direction
+    NetGeom() = default;
+    __host__ __device__ NetGeom(size_t n_, int logN_, int fill_ = 0)
+        : n(n_), logN(logN_), fill(fill_), m((size_t)1 << logN_), dirx(0)
+    {
+    }
+    // trimmed to the tiles of 2^lt rows that hold the n real rows
+    __host__ __device__ static NetGeom trimmed(size_t n, int logN, int lt, int fill)
+    {
+        NetGeom g(n, logN, fill);
+        const size_t t = (size_t)1 << lt;
+        const size_t m = (n + t - 1) / t * t;
+        if (m < g.m) {
+            g.m = m;
+            g.dirx = (m - 1) & ~(t - 1); // tiles keep the plain directions
+        }
+        return g;
+    }
 };
 
 struct NetPass {
@@ -40,12 +69,35 @@ struct NetPass {
     int L;    // GLOBAL: number of fused levels
 };
 
+// tiles (CTAs, work items) of pass `p` over `g` in tiles of 2^lt rows
+__host__ __device__ inline size_t net_pass_tiles(const NetGeom& g, const NetPass& p, int lt)
+{
+    if (g.logN <= lt)
+        return 1;
+    if (p.kind == P_SORT_GLOBAL) {
+        // every block of 2^(b_hi + 1) rows that holds a row below m
+        const int b = p.b_hi + 1;
+        return ((g.m + ((size_t)1 << b) - 1) >> b) << (b - lt);
+    }
+    if (p.kind == P_SORT_TILE && g.fill)
+        return (size_t)1 << (g.logN - lt);
+    return (g.m + ((size_t)1 << lt) - 1) >> lt;
+}
+
 // mark of the row stored at global index g (count pass)
 template <class R>
 struct MarkAt;
+template <int CM>
+struct MarkAt<RowK12<CM>> {
+    __device__ __forceinline__ static bool get(const typename RowK12<CM>::Cols& c, size_t g)
+    {
+        VELO_TRACE_AT(TS_MARK_LOAD, c.k + g);
+        return (__ldcg(c.k + g) >> 63) == 0;
+    }
+};
 template <>
-struct MarkAt<RowKP> {
-    __device__ __forceinline__ static bool get(const RowKP::Cols&, size_t) { return false; }
+struct MarkAt<RowU2> {
+    __device__ __forceinline__ static bool get(const RowU2::Cols&, size_t) { return false; }
 };
 template <>
 struct MarkAt<RowKPM> {
@@ -146,6 +198,7 @@ struct Net {
     static constexpr int LT = TL::LOG_T;
     static constexpr int T = TL::T;
     static constexpr int S0 = LT - LOG_E; // load/store layout (lanes <-> rows 0..31)
+    static constexpr bool FLIP = Flip<R>::on;
 
     static constexpr size_t smem_rows() { return ((size_t)T * R::SMEM_BYTES + 15) & ~(size_t)15; }
     static constexpr size_t smem_bytes_sort() { return smem_rows(); }
@@ -302,7 +355,7 @@ struct Net {
             bool d = dm;
             if constexpr (PER_E)
                 d = (dpat & (1u << e)) != 0u;
-            Cswap<R, Q & 1>::run(v[e], v[e2], R::swap_pred(v[e], v[e2], d, c));
+            R::cswap(v[e], v[e2], R::swap_pred(v[e], v[e2], d, c));
         }
     }
 
@@ -344,6 +397,29 @@ struct Net {
             }
         };
         QDown<LOG_E - 1>::run(f);
+    }
+
+    // ---- complement of the rows whose block descends (Flip types) -----------
+    // phase 2^K of a tile sort begins: a row's state goes from bit K - 1 of its
+    // index to bit K (`last`: from bit K - 1 back to plain); top = 1 if the
+    // whole tile descends in the phase K = LT
+    __device__ __forceinline__ static void flip_phase(R (&v)[E], int s, int K, uint32_t top, bool last)
+    {
+        const uint32_t tp = (uint32_t)tidpart(s);
+#pragma unroll
+        for (int e = 0; e < E; e++) {
+            const uint32_t l = tp | ((uint32_t)e << s);
+            const uint32_t from = K > 1 ? (K - 1 < LT ? (l >> (K - 1)) & 1u : top) : 0u;
+            const uint32_t to = last ? 0u : K < LT ? (l >> K) & 1u : top;
+            R::flip(v[e], 0u - (from ^ to));
+        }
+    }
+    __device__ __forceinline__ static void flip_all(R (&v)[E], bool asc)
+    {
+        const uint32_t m = asc ? 0u : ~0u;
+#pragma unroll
+        for (int e = 0; e < E; e++)
+            R::flip(v[e], m);
     }
 
     // ---- ORCompact exchange (tile-local level, block size 2^(b+1)) --------
@@ -444,7 +520,7 @@ struct Net {
     {
         constexpr bool CT = SORT && (PK == PK_LOCAL || PK == PK_MERGE);
         constexpr bool BOFF = !WIDE;
-        const size_t Np = (size_t)1 << g.logN;
+        const size_t Np = g.m;
         const bool is_global = PK == PK_GLOBAL ? true
             : PK == PK_LOCAL || PK == PK_MERGE ? false
                                                : (p.kind == P_SORT_GLOBAL) || (p.kind == P_COMPACT_GLOBAL);
@@ -462,6 +538,16 @@ struct Net {
             return (size_t)(l & ((1 << C) - 1)) | ((size_t)(l >> C) << b_lo) | cta_bits;
         };
         const int smin = is_global ? (C < S0 ? C : S0) : 0;
+        if (SORT && is_global && ((cta_bits | ((size_t)1 << b_lo)) >= Np))
+            return; // trimmed: only the lowest row of each pair exists
+        if (SORT && p.kind == P_SORT_TILE && cta_bits >= Np) {
+            // a tile of padding (trimmed, fill)
+            const int tp = tidpart(S_WARP);
+#pragma unroll
+            for (int e = 0; e < E; e++)
+                R::store(c, cta_bits | (size_t)(tp | (e << S_WARP)), R::pad(c));
+            return;
+        }
 
         R v[E];
         const bool first = (p.kind == P_SORT_TILE) || (p.kind == P_COMPACT_TILE);
@@ -482,6 +568,8 @@ struct Net {
                 const size_t gi = gidx(tp | (e << s));
                 if (first)
                     v[e] = (gi < g.n) ? R::load(c, gi) : R::pad(c);
+                else if (SORT && is_global)
+                    v[e] = (gi < Np) ? R::load(c, gi) : R::pad(c);
                 else
                     v[e] = R::load(c, gi);
             }
@@ -491,7 +579,9 @@ struct Net {
             if (PK != PK_GLOBAL && PK != PK_MERGE && p.kind == P_SORT_TILE) {
                 for (int K = 1; K <= p.K; K++) {
                     const bool dconst = K >= LT;
-                    const bool asc_c = ((cta_bits >> K) & 1) == 0;
+                    const bool asc_c = (((cta_bits ^ g.dirx) >> K) & 1) == 0;
+                    if constexpr (FLIP)
+                        flip_phase(v, s, K, asc_c ? 0u : 1u, false);
                     int b = K - 1;
                     while (b >= 0) {
                         if (b < s || b >= s + LOG_E) {
@@ -499,15 +589,19 @@ struct Net {
                             transpose<CT, BOFF>(v, s, ns, sm);
                             s = ns;
                         }
-                        bitonic_window(v, c, s, b, s, K, dconst, asc_c);
+                        bitonic_window(v, c, s, b, s, K, FLIP || dconst, FLIP || asc_c);
                         b = s - 1;
                     }
                 }
+                if constexpr (FLIP)
+                    flip_phase(v, s, p.K + 1, (uint32_t)((cta_bits ^ g.dirx) >> LT) & 1u, true);
             } else {
                 // MERGE: bits LT-1..0; GLOBAL: local bits C+L-1..C (the L fused
                 // global levels); the direction is fixed for the tile
                 const bool merge = PK == PK_MERGE || (PK != PK_GLOBAL && p.kind == P_SORT_MERGE);
-                const bool asc_c = (((merge ? cta_bits : gidx(0)) >> p.K) & 1) == 0;
+                const bool asc_c = ((((merge ? cta_bits : gidx(0)) ^ g.dirx) >> p.K) & 1) == 0;
+                if constexpr (FLIP)
+                    flip_all(v, asc_c);
                 const int top = merge ? LT - 1 : C + p.L - 1;
                 const int bottom = merge ? 0 : C;
                 int b = top;
@@ -519,9 +613,11 @@ struct Net {
                         s = ns;
                     }
                     const int lo = s > bottom ? s : bottom;
-                    bitonic_window(v, c, s, b, lo, p.K, true, asc_c);
+                    bitonic_window(v, c, s, b, lo, p.K, true, FLIP || asc_c);
                     b = lo - 1;
                 }
+                if constexpr (FLIP)
+                    flip_all(v, asc_c);
             }
         } else {
             if (PK == PK_LOCAL || (PK != PK_GLOBAL && p.kind == P_COMPACT_TILE)) {
