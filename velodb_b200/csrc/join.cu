@@ -4,25 +4,29 @@
 // 63-199, src/operator/sort_merge_join_operator.cpp:27-257: per-block
 // sequential merge, atomics, output sized by the true join cardinality) with
 // the oblivious union-sort formulation:
-//   1. pack     dimension rows (key, tag 0, date filter) and fact rows
-//               (fk, tag 1, price filter, price) into one record array,
-//               padded to a power of two
-//   2. sort     bitonic network on (key, tag): each dimension row heads the
-//               run of fact rows that reference it
-//   3. fill     forward fill of the last dimension row (segmented scan): a
-//               fact row joins iff its key's dimension row exists and passes
-//   4. compact  ORCompact of joined fact rows to the front (order kept)
-//   5. group    segmented sums of price per fk over the joined prefix: the
-//               last row of each fk run carries the group's (sum, count)
-//   6. top-k    groups ordered on (sum desc, fk asc) by a bitonic top-k
-//               network (topk.cuh): each 1024-row tile of the group-by keeps
-//               its best c = max(16, next_pow2(k)) rows in shared memory,
-//               then rounds over blocks of 4096 candidates keep their best
-//               c, until one sorted run of c is left; first k
-// Record layout of the union (2 u64 words):
+//   1. pack     dimension rows and fact rows into one array of 12-byte rows
+//               (RowKP: key, then a 64-bit order word u; join.cuh)
+//   2. sort     bitonic network on the whole row, the rows past the union left
+//               out (NetGeom::trimmed): each key's passing dimension rows, then
+//               the rows that fail their filter, then its passing fact rows
+//   3. group    segmented sums over the runs of equal keys (price, fact rows,
+//               passing dimension rows): a key is a group iff it has a passing
+//               dimension row and a passing fact row, and all its passing fact
+//               rows join then, so no fill, joined flag or compaction is needed
+//               to find them; the last row of the run carries the group
+//   4. top-k    groups ordered on (sum desc, fk asc) by a bitonic top-k
+//               network (topk.cuh): each 2048-row tile of the group-by keeps
+//               its best c = max(16, next_pow2(k)) rows, then rounds over
+//               blocks of 4096 candidates keep their best c, until one sorted
+//               run of c is left; first k
+// A predicate with price_hi = INT64_MAX leaves no order word free for a row
+// that fails, so it takes the record form: 16-byte records of next_pow2 rows,
+// sort on (key, tag), forward fill of the last dimension row, segmented sums,
+// top-k.  (1.5 M x 6 M rows: JOIN_FILL)
+// Record layout of that form (2 u64 words):
 //   w0 = [63:32] key ^ 0x80000000 | [31] tag (0 dim, 1 fact) | [30] row passes
 //        its side's filter | [29] joined (set by fill) ; w1 = price (fact rows)
-#include "net_impl.cuh"
+#include "net_host.cuh"
 #include "join.cuh"
 
 namespace velo {
@@ -97,6 +101,54 @@ __global__ void __launch_bounds__(SEG_THREADS, 5) k_jseg_emit_topk(JRec::Cols c,
     jseg_emit_topk_tile(c, ntiles, aggs, carry_in, cand, out0, out1, blockIdx.x, sm);
 }
 
+// ---- the 12-byte form --------------------------------------------------------
+
+__global__ void __launch_bounds__(256) k_jk_pack(const int32_t* dk, const int32_t* dd, size_t nd, const int32_t* ff,
+                                                 const int64_t* fp, size_t nf, int32_t date_hi, int64_t price_hi,
+                                                 uint64_t* k, uint32_t* p, uint64_t* n_groups, uint64_t* n_joined)
+{
+    VELO_TRACE_KERNEL(velo_site_hash("k_jk_pack"));
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        *n_groups = 0;
+        *n_joined = 0;
+    }
+    const size_t n = nd + nf;
+    for (size_t g = blockIdx.x * (size_t)blockDim.x + threadIdx.x; VELO_GRID_COND(g, n);
+         g += (size_t)gridDim.x * blockDim.x) {
+        uint32_t key;
+        uint64_t u;
+        if (g < nd) {
+            key = (uint32_t)dk[g];
+            u = dd[g] < date_hi ? JK_DIM : JK_DEAD;
+        } else {
+            const size_t j = g - nd;
+            const int64_t pr = fp[j];
+            key = (uint32_t)ff[j];
+            u = pr < price_hi ? ~((uint64_t)pr ^ SIGN64) : JK_DEAD;
+        }
+        VELO_TRACE_AT(TS_ROW_STORE, k + g);
+        k[g] = ((uint64_t)(key ^ 0x80000000u) << 32) | (u >> 32);
+        p[g] = (uint32_t)u;
+    }
+}
+
+__global__ void __launch_bounds__(JK_THREADS) k_jk_summary(const uint64_t* k, const uint32_t* p, size_t n,
+                                                           SegTileAgg* aggs, int64_t* runs)
+{
+    VELO_TRACE_KERNEL(velo_site_hash("k_jk_summary"));
+    jk_summary_tile(k, p, n, blockIdx.x, aggs, runs);
+}
+
+__global__ void __launch_bounds__(JK_THREADS, 4) k_jk_emit_topk(const uint64_t* k, const uint32_t* p, size_t n,
+                                                                int ntiles, const SegTileAgg* aggs,
+                                                                const int64_t* carry_in, int cand, uint64_t* out0,
+                                                                uint64_t* out1, uint64_t* n_groups, uint64_t* n_joined)
+{
+    VELO_TRACE_KERNEL(velo_site_hash("k_jk_emit_topk"));
+    extern __shared__ __align__(16) char sm[];
+    jk_emit_topk_tile(k, p, n, ntiles, aggs, carry_in, cand, out0, out1, n_groups, n_joined, blockIdx.x, sm);
+}
+
 static velo_status join_attrs()
 {
     static int done[64] = {};
@@ -109,11 +161,105 @@ static velo_status join_attrs()
     VELO_CUDA_TRY(cudaFuncSetAttribute(k_jseg_emit_topk, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)JSEG_TOPK_SMEM),
                   "cudaFuncSetAttribute");
+    VELO_CUDA_TRY(cudaFuncSetAttribute(k_jk_emit_topk, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)JK_EMIT_SMEM),
+                  "cudaFuncSetAttribute");
     VELO_CUDA_TRY(cudaFuncSetAttribute(k_topk_reduce, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)(2 * TK_RED_ROWS * 8)),
                   "cudaFuncSetAttribute");
     if (dev >= 0 && dev < 64)
         done[dev] = 1;
+    return VELO_OK;
+}
+
+// The record form up to the candidates of the group-by tiles.
+static velo_status join_records(const JoinScratch& s, const velo_join_tables* t, const velo_join_pred* pred, int cand,
+                                StageTimer& tm, size_t* n_cand, cudaStream_t st)
+{
+    const int logR = ilog2_floor(s.n_rec);
+    const size_t n_union = t->n_dim + t->n_fact;
+    const int logU = ilog2_floor(next_pow2(n_union));
+    // 1. pack
+    const unsigned blocks = 148 * 8;
+    k_join_pack<<<blocks, 256, 0, st>>>(t->dim_key, t->dim_date, t->n_dim, t->fact_fk, t->fact_price, t->n_fact,
+                                        pred->date_hi, pred->price_hi, s.n_rec, s.u[0], s.u[1]);
+    VELO_CUDA_TRY(cudaGetLastError(), "join pack launch");
+    tm.mark();
+    JRec::Cols uc;
+    uc.w[0] = s.u[0];
+    uc.w[1] = s.u[1];
+    uc.mask[0] = J_KEYTAG;
+    uc.pad[0] = uc.pad[1] = ~0ull;
+    uc.mark_bit = 29;
+    uc.mark_inv = 0;
+    uc.mark_word = 0;
+    // 2. sort the union on (key, tag)
+    velo_status rc = launch_sort_records<JRec>(uc, logU, st);
+    if (rc != VELO_OK)
+        return rc;
+    tm.mark();
+    // 3. forward fill of the dimension side -> joined flag
+    const int ntf = (int)(s.n_rec / FILL_TS);
+    k_fill_summary<<<ntf, FILL_THREADS, 0, st>>>(s.u[0], s.tile_last);
+    k_fill_carries<<<1, 1024, 0, st>>>(s.tile_last, ntf, s.fcarry);
+    k_fill_apply<<<ntf, FILL_THREADS, 0, st>>>(s.u[0], s.fcarry);
+    VELO_CUDA_TRY(cudaGetLastError(), "join fill launch");
+    tm.mark();
+    // 4. the number of joined fact rows.  They need no compaction: the joined
+    // rows of a key are neighbours (all its passing fact rows or none), so each
+    // key's are one run of (key, joined)
+    rc = launch_count_scan<JRec>(uc, s.n_rec, logR, J_LT, s.counts, s.prefix, s.n_joined, st);
+    if (rc != VELO_OK)
+        return rc;
+    tm.mark();
+    // 5. group-by fk over the sorted union, fused with the first top-k round:
+    // the best `cand` groups of every tile
+    const int nts = (int)(s.n_rec / SEG_TS);
+    k_jseg_summary<<<nts, SEG_THREADS, JSeg::SMEM_IN, st>>>(uc, s.aggs, s.runs);
+    k_jseg_carries<<<1, 1024, JoinAgg::V * 1024 * 8 + 2 * 1024 * 4, st>>>(s.aggs, s.runs, nts, s.carry,
+                                                                            s.tail_prefix, s.n_groups);
+    const size_t topk_smem = cand == 16 ? JSEG_TOPK16_SMEM : JSEG_TOPK_SMEM;
+    k_jseg_emit_topk<<<nts, SEG_THREADS, topk_smem, st>>>(uc, nts, s.aggs, s.carry, cand, s.cand[0], s.cand[1]);
+    VELO_CUDA_TRY(cudaGetLastError(), "join group-by launch");
+    tm.mark();
+    *n_cand = (size_t)nts * cand;
+    return VELO_OK;
+}
+
+// The 12-byte form up to the candidates of the group-by tiles.
+static velo_status join_rows(const JoinScratch& s, const velo_join_tables* t, const velo_join_pred* pred, int cand,
+                             StageTimer& tm, size_t* n_cand, cudaStream_t st)
+{
+    const size_t n = t->n_dim + t->n_fact;
+    const int logU = ilog2_floor(next_pow2(n));
+    uint64_t* k = s.u[0];
+    uint32_t* p = reinterpret_cast<uint32_t*>(s.u[1]);
+    // 1. pack
+    const size_t want = (n + 255) / 256;
+    k_jk_pack<<<(unsigned)(want < 148 * 8 ? want : 148 * 8), 256, 0, st>>>(t->dim_key, t->dim_date, t->n_dim, t->fact_fk,
+                                                                           t->fact_price, t->n_fact, pred->date_hi,
+                                                                           pred->price_hi, k, p, s.n_groups, s.n_joined);
+    VELO_CUDA_TRY(cudaGetLastError(), "join pack launch");
+    tm.mark();
+    // 2. sort
+    if (n > 1) {
+        const velo_status rc = sort_kp_rows(RowKP::Cols { k, p }, n, logU, 0, st);
+        if (rc != VELO_OK)
+            return rc;
+    }
+    tm.mark();
+    // 3. segmented sums; the emit pass runs a power of two of tiles, the ones
+    // past the rows writing empty candidates
+    const int nt = (int)((n + JK_TS - 1) / JK_TS);
+    const int nts = (int)next_pow2((size_t)nt);
+    k_jk_summary<<<nt, JK_THREADS, 0, st>>>(k, p, n, s.aggs, s.runs);
+    k_jseg_carries<<<1, 1024, JoinAgg::V * 1024 * 8 + 2 * 1024 * 4, st>>>(s.aggs, s.runs, nt, s.carry, s.tail_prefix,
+                                                                            s.unused);
+    k_jk_emit_topk<<<nts, JK_THREADS, cand == 16 ? JK_EMIT16_SMEM : JK_EMIT_SMEM, st>>>(
+        k, p, n, nt, s.aggs, s.carry, cand, s.cand[0], s.cand[1], s.n_groups, s.n_joined);
+    VELO_CUDA_TRY(cudaGetLastError(), "join group-by launch");
+    tm.mark();
+    *n_cand = (size_t)nts * cand;
     return VELO_OK;
 }
 
@@ -147,65 +293,17 @@ extern "C" velo_status velo_join_groupby_topk(const velo_join_tables* t, const v
     velo_status rc = join_attrs();
     if (rc != VELO_OK)
         return rc;
-    const int logR = ilog2_floor(s.n_rec);
-    const size_t n_union = t->n_dim + t->n_fact;
-    const int logU = ilog2_floor(next_pow2(n_union));
+    const int cand = k <= (uint32_t)J_TOPK_MIN ? J_TOPK_MIN : (int)next_pow2(k);
     StageTimer tm(st);
-
-    // 1. pack
-    const unsigned blocks = 148 * 8;
-    k_join_pack<<<blocks, 256, 0, st>>>(t->dim_key, t->dim_date, t->n_dim, t->fact_fk, t->fact_price, t->n_fact,
-                                        pred->date_hi, pred->price_hi, s.n_rec, s.u[0], s.u[1]);
-    VELO_CUDA_TRY(cudaGetLastError(), "join pack launch");
-    tm.mark();
-    JRec::Cols uc;
-    uc.w[0] = s.u[0];
-    uc.w[1] = s.u[1];
-    uc.mask[0] = J_KEYTAG;
-    uc.pad[0] = uc.pad[1] = ~0ull;
-    uc.mark_bit = 29;
-    uc.mark_inv = 0;
-    uc.mark_word = 0;
-    // 2. sort the union on (key, tag)
-    rc = launch_sort_records<JRec>(uc, logU, st);
+    size_t n_c = 0;
+    // the 12-byte form needs two prices that no passing fact row has
+    rc = pred->price_hi < INT64_MAX ? join_rows(s, t, pred, cand, tm, &n_c, st)
+                                    : join_records(s, t, pred, cand, tm, &n_c, st);
     if (rc != VELO_OK)
         return rc;
-    tm.mark();
-    // 3. forward fill of the dimension side -> joined flag
-    const int ntf = (int)(s.n_rec / FILL_TS);
-    k_fill_summary<<<ntf, FILL_THREADS, 0, st>>>(s.u[0], s.tile_last);
-    k_fill_carries<<<1, 1024, 0, st>>>(s.tile_last, ntf, s.fcarry);
-    k_fill_apply<<<ntf, FILL_THREADS, 0, st>>>(s.u[0], s.fcarry);
-    VELO_CUDA_TRY(cudaGetLastError(), "join fill launch");
-    tm.mark();
-    // 4. ORCompact of the joined fact rows
-    {
-        const int ntc = logR > J_LT ? 1 << (logR - J_LT) : 1;
-        k_count_marks<JRec><<<ntc, 256, 0, st>>>(uc, s.n_rec, J_LT, s.counts);
-        k_scan_tiles<<<1, 1024, 0, st>>>(s.counts, ntc, s.prefix, s.n_joined);
-        std::vector<NetPass> passes;
-        plan_compact(logR, J_LT, J_LMAX, passes);
-        rc = launch_net12<JRec>(uc, NetGeom { s.n_rec, logR, 0 }, passes, s.prefix, st);
-        if (rc != VELO_OK)
-            return rc;
-    }
-    tm.mark();
-    // 5. group-by fk over the joined prefix (already in fk order: the
-    // compaction keeps the sorted order of the joined rows), fused with the
-    // first top-k round: the best `cand` groups of every tile
-    const int nts = (int)(s.n_rec / SEG_TS);
-    const int cand = k <= (uint32_t)J_TOPK_MIN ? J_TOPK_MIN : (int)next_pow2(k);
-    k_jseg_summary<<<nts, SEG_THREADS, JSeg::SMEM_IN, st>>>(uc, s.aggs, s.runs);
-    k_jseg_carries<<<1, 1024, JoinAgg::V * 1024 * 8 + 2 * 1024 * 4, st>>>(s.aggs, s.runs, nts, s.carry,
-                                                                            s.tail_prefix, s.n_groups);
-    const size_t topk_smem = cand == 16 ? JSEG_TOPK16_SMEM : JSEG_TOPK_SMEM;
-    k_jseg_emit_topk<<<nts, SEG_THREADS, topk_smem, st>>>(uc, nts, s.aggs, s.carry, cand, s.cand[0], s.cand[1]);
-    VELO_CUDA_TRY(cudaGetLastError(), "join group-by launch");
-    tm.mark();
-    // 6. top-k rounds over blocks of candidates (the union area is free now)
+    // top-k rounds over blocks of candidates (the union area is free now)
     uint64_t* cur[2] = { s.cand[0], s.cand[1] };
     uint64_t* nxt[2] = { s.u[0], s.u[1] };
-    size_t n_c = (size_t)nts * cand;
     while (n_c > (size_t)cand) {
         const int rn = n_c < (size_t)TK_RED_ROWS ? (int)n_c : TK_RED_ROWS;
         const size_t blocks = n_c / rn;

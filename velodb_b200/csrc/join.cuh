@@ -358,6 +358,230 @@ __device__ __forceinline__ void jseg_emit_topk_tile(const JRec::Cols& c, int nti
 }
 
 
+// ---- the 12-byte form ----------------------------------------------------------
+// A union row as RowKP (key word, payload), ordered on all 96 bits:
+//   k = (key ^ 2^31) << 32 | u >> 32, p = low half of u, with the order word
+//   u = JK_DIM   a dimension row that passes the date filter
+//       JK_DEAD  a row of either side that fails its filter
+//       ~(price ^ 2^63)  a passing fact row; its price is below price_hi <
+//                INT64_MAX, so its u is at least 2
+constexpr uint64_t JK_DIM = 0, JK_DEAD = 1;
+// 2048-row tiles, 8 consecutive rows a thread: a group has at least two rows
+// (a dimension row and a fact row), so a pair of neighbouring rows holds at most
+// one group's last row and the top-k sees half as many rows
+constexpr int JK_THREADS = 256, JK_RPT = 8, JK_TS = JK_THREADS * JK_RPT;
+constexpr uint64_t JK_NOKEY = 1ull << 32; // key of a row past the union
+
+// slot of tile row i: one pad word after every 8 rows, so that the 8 rows of
+// neighbouring threads fall in different banks
+__device__ __forceinline__ int jk_slot(int i) { return i + (i >> 3); }
+constexpr int JK_TS_PAD = JK_TS + JK_TS / 8;
+
+// (sum of price, fact rows | passing dimension rows << 32) of one row; values
+// a and b add up over the rows of a key, each half below 2^31
+__device__ __forceinline__ void jk_values(uint64_t u, int64_t& a, int64_t& b)
+{
+    const bool fact = u > JK_DEAD;
+    a = fact ? (int64_t)(~u ^ SIGN64) : 0;
+    b = fact ? 1 : u == JK_DIM ? (int64_t)1 << 32 : 0;
+}
+
+// tile `blk`: first and last key, the last key's sums inside the tile
+__device__ __forceinline__ void jk_summary_tile(const uint64_t* k, const uint32_t* p, size_t n, size_t blk,
+                                                SegTileAgg* aggs, int64_t* runs)
+{
+    __shared__ int64_t red[2][JK_THREADS / 32];
+    const size_t base = blk * JK_TS;
+    const size_t last = base + JK_TS - 1;
+    VELO_TRACE_AT(TS_SEG_LOAD, k + base);
+    const uint64_t head = k[base] >> 32; // base < n
+    const uint64_t tail = last < n ? k[last] >> 32 : JK_NOKEY;
+    int64_t a = 0, b = 0;
+#pragma unroll
+    for (int r = 0; r < JK_RPT; r++) {
+        const size_t g = base + (size_t)r * JK_THREADS + threadIdx.x;
+        uint64_t kk = ~0ull;
+        uint32_t pp = 0;
+        if (g < n) {
+            VELO_TRACE_AT(TS_SEG_LOAD, k + g);
+            kk = k[g];
+            pp = p[g];
+        }
+        int64_t va, vb;
+        jk_values((kk << 32) | pp, va, vb);
+        const bool in = (g < n) & ((kk >> 32) == tail);
+        a += in ? va : 0;
+        b += in ? vb : 0;
+    }
+    a = warp_sum_i64(a);
+    b = warp_sum_i64(b);
+    if ((threadIdx.x & 31) == 0) {
+        red[0][threadIdx.x >> 5] = a;
+        red[1][threadIdx.x >> 5] = b;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < JK_THREADS / 32; w++) {
+            a += red[0][w];
+            b += red[1][w];
+        }
+        VELO_TRACE_AT(TS_SEG_META, aggs + blk);
+        aggs[blk] = SegTileAgg { head, tail, head == tail ? 1u : 0u, 0u, 0u, 0u };
+        runs[blk * 2] = a;
+        runs[blk * 2 + 1] = b;
+    }
+}
+
+// group sums of tile `blk` and its best `cand` groups; tiles past the rows
+// write empty candidates.  sm: JK_EMIT_SMEM bytes (JK_EMIT16_SMEM for 16)
+constexpr size_t JK_VALS_OFF = (size_t)JK_TS_PAD * 12;
+constexpr size_t JK_KEYS_OFF = (JK_VALS_OFF + (size_t)(2 * JK_THREADS + 64) * 8 + JK_THREADS * 4 + 256 + 15) & ~(size_t)15;
+constexpr int JK_CROWS = JK_TS / 2; // candidate rows of a tile
+constexpr size_t JK_EMIT_SMEM = JK_KEYS_OFF + (size_t)2 * JK_CROWS * 8;
+constexpr size_t JK_EMIT16_SMEM = JK_KEYS_OFF + (size_t)2 * 128 * 8;
+
+__device__ __forceinline__ void jk_emit_topk_tile(const uint64_t* k, const uint32_t* p, size_t n, int ntiles,
+                                                  const SegTileAgg* aggs, const int64_t* carry_in, int cand,
+                                                  uint64_t* out0, uint64_t* out1, uint64_t* n_groups,
+                                                  uint64_t* n_joined, size_t blk, char* sm)
+{
+    if (blk >= (size_t)ntiles) {
+        for (int j = threadIdx.x; j < cand; j += JK_THREADS) {
+            VELO_TRACE_AT(TS_TOPK, out0 + blk * cand + j);
+            out0[blk * cand + j] = ~0ull;
+            out1[blk * cand + j] = ~0ull;
+        }
+        return;
+    }
+    uint64_t* sk = reinterpret_cast<uint64_t*>(sm);
+    uint32_t* sp = reinterpret_cast<uint32_t*>(sm + (size_t)JK_TS_PAD * 8);
+    int64_t* svals = reinterpret_cast<int64_t*>(sm + JK_VALS_OFF);
+    uint32_t* sflags = reinterpret_cast<uint32_t*>(svals + 2 * JK_THREADS + 64);
+    uint64_t* k0 = reinterpret_cast<uint64_t*>(sm + JK_KEYS_OFF);
+    const size_t base = blk * JK_TS;
+#pragma unroll
+    for (int r = 0; r < JK_RPT; r++) {
+        const int i = r * JK_THREADS + (int)threadIdx.x;
+        const size_t g = base + i;
+        uint64_t kk = ~0ull;
+        uint32_t pp = ~0u;
+        if (g < n) {
+            VELO_TRACE_AT(TS_SEG_LOAD, k + g);
+            kk = k[g];
+            pp = p[g];
+        }
+        sk[jk_slot(i)] = kk;
+        sp[jk_slot(i)] = pp;
+    }
+    __syncthreads();
+    const bool more = (int)blk + 1 < ntiles;
+    const uint64_t next_head = more ? aggs[blk + 1].head_key : JK_NOKEY << 1;
+    const uint64_t head_key = aggs[blk].head_key;
+    const int r0 = threadIdx.x * JK_RPT;
+    // key of tile row i (a row past the union has a key of its own)
+    auto key_at = [&](int i) -> uint64_t { return base + i < n ? sk[jk_slot(i)] >> 32 : JK_NOKEY; };
+    const uint64_t prev_key = r0 > 0 ? key_at(r0 - 1) : 0;
+    int64_t pa[JK_RPT], pb[JK_RPT];
+    uint64_t keys[JK_RPT];
+    bool start = false;
+    {
+        int64_t a = 0, b = 0;
+        uint64_t kp = prev_key;
+#pragma unroll
+        for (int r = 0; r < JK_RPT; r++) {
+            const int sl = threadIdx.x * (JK_RPT + 1) + r;
+            const uint64_t kk = sk[sl];
+            const bool in = base + r0 + r < n;
+            keys[r] = in ? kk >> 32 : JK_NOKEY;
+            int64_t va, vb;
+            jk_values((kk << 32) | sp[sl], va, vb);
+            const bool starts = (r0 + r == 0) | (keys[r] != kp);
+            start = start | starts;
+            a = (starts ? 0 : a) + (in ? va : 0);
+            b = (starts ? 0 : b) + (in ? vb : 0);
+            pa[r] = a;
+            pb[r] = b;
+            kp = keys[r];
+        }
+    }
+    const uint64_t after = r0 + JK_RPT < JK_TS ? key_at(r0 + JK_RPT) : next_head;
+    int64_t agg[2] = { pa[JK_RPT - 1], pb[JK_RPT - 1] };
+    bool fl = start;
+    block_seg_scan<2>(fl, agg, svals, sflags);
+    svals[threadIdx.x] = agg[0];
+    svals[JK_THREADS + threadIdx.x] = agg[1];
+    __syncthreads();
+    const int64_t ca = threadIdx.x > 0 ? svals[threadIdx.x - 1] : 0;
+    const int64_t cb = threadIdx.x > 0 ? svals[JK_THREADS + threadIdx.x - 1] : 0;
+    const int64_t ta = carry_in[blk * 2], tb = carry_in[blk * 2 + 1];
+    bool lead = r0 > 0 && prev_key == keys[0];
+    uint64_t x0[JK_RPT / 2], x1[JK_RPT / 2];
+    uint32_t groups = 0;
+    uint64_t joined = 0;
+#pragma unroll
+    for (int r = 0; r < JK_RPT; r++) {
+        if (r > 0)
+            lead = lead & (keys[r] == keys[r - 1]);
+        const bool first = keys[r] == head_key; // the tile's first run goes on from earlier tiles
+        const int64_t sum = pa[r] + (lead ? ca : 0) + (first ? ta : 0);
+        const uint64_t cnt = (uint64_t)(pb[r] + (lead ? cb : 0) + (first ? tb : 0));
+        const bool ends = keys[r] != (r + 1 < JK_RPT ? keys[r + 1 < JK_RPT ? r + 1 : r] : after);
+        const bool grp = ends & ((cnt >> 32) != 0) & ((uint32_t)cnt != 0);
+        groups += grp ? 1u : 0u;
+        joined += grp ? (uint64_t)(uint32_t)cnt : 0ull;
+        uint64_t y0, y1;
+        topk_key((grp ? 0ull : SIGN64) | (keys[r] & 0xFFFFFFFFull), (uint64_t)sum, (uint32_t)cnt, y0, y1);
+        if ((r & 1) == 0) {
+            x0[r / 2] = grp ? y0 : ~0ull;
+            x1[r / 2] = grp ? y1 : ~0ull;
+        } else {
+            x0[r / 2] = grp ? y0 : x0[r / 2];
+            x1[r / 2] = grp ? y1 : x1[r / 2];
+        }
+    }
+    // the tile's groups and joined rows: one update each at a fixed address
+    {
+        const int64_t g = warp_sum_i64((int64_t)groups), j = warp_sum_i64((int64_t)joined);
+        __syncthreads();
+        if ((threadIdx.x & 31) == 0) {
+            svals[threadIdx.x >> 5] = g;
+            svals[32 + (threadIdx.x >> 5)] = j;
+        }
+        __syncthreads();
+        if (threadIdx.x < 2) {
+            int64_t s = 0;
+            for (int w = 0; w < JK_THREADS / 32; w++)
+                s += svals[32 * threadIdx.x + w];
+            atomicAdd(reinterpret_cast<unsigned long long*>(threadIdx.x ? n_joined : n_groups), (unsigned long long)s);
+        }
+    }
+    if (cand == 16) {
+        static_assert(JK_RPT / 2 == 4 && JK_THREADS == 256, "4 candidate rows a thread, 8 warps");
+        uint64_t y0, y1;
+        topk16_block(x0, x1, k0, TK_M1, y0, y1);
+        if (threadIdx.x < 16) {
+            const size_t o = blk * 16 + tk_row16(threadIdx.x);
+            VELO_TRACE_AT(TS_TOPK, out0 + o);
+            out0[o] = y0;
+            out1[o] = y1;
+        }
+        return;
+    }
+    uint64_t* k1 = k0 + JK_CROWS;
+#pragma unroll
+    for (int e = 0; e < JK_RPT / 2; e++) {
+        k0[threadIdx.x * (JK_RPT / 2) + e] = x0[e];
+        k1[threadIdx.x * (JK_RPT / 2) + e] = x1[e];
+    }
+    topk_net<JK_CROWS / 2 / JK_THREADS>(k0, k1, JK_CROWS, cand, TK_M1, false);
+    for (int j = threadIdx.x; j < cand; j += JK_THREADS) {
+        VELO_TRACE_AT(TS_TOPK, out0 + blk * cand + j);
+        out0[blk * cand + j] = k0[j];
+        out1[blk * cand + j] = k1[j];
+    }
+}
+
+
 struct JoinScratch {
     uint64_t* u[2];      // union records
     uint64_t* cand[2];   // top-k candidates of the group-by tiles (later rounds reuse u)
@@ -371,6 +595,7 @@ struct JoinScratch {
     int64_t* carry;
     uint32_t* tail_prefix;
     uint64_t* n_groups;
+    uint64_t* unused; // the group count of the carry scan, which the 12-byte form does not use
     size_t bytes, n_rec;
 };
 
@@ -404,6 +629,7 @@ inline JoinScratch join_layout(char* base, size_t nd, size_t nf)
     s.carry = reinterpret_cast<int64_t*>(take(nts * JoinAgg::V * 8));
     s.tail_prefix = reinterpret_cast<uint32_t*>(take(nts * 4));
     s.n_groups = reinterpret_cast<uint64_t*>(take(8));
+    s.unused = base ? s.n_groups + 1 : nullptr; // in the 256 bytes of n_groups
     s.bytes = off;
     return s;
 }
