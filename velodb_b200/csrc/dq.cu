@@ -85,9 +85,8 @@ public:
         a.g = g;
         a.prefix = prefix;
         const uint32_t off = arg(a);
-        const uint64_t nt = g.logN > lt ? 1ull << (g.logN - lt) : 1ull;
         for (const NetPass& p : passes)
-            step(kind, nt, off, p);
+            step(kind, net_pass_tiles(g, p, lt), off, p);
     }
     template <class R>
     void count(uint32_t kind, const typename R::Cols& c, size_t n, int lt, uint32_t* counts, uint64_t ntiles)
@@ -240,8 +239,8 @@ static velo_status plan_osort_kp(B& b, uint64_t* k, uint32_t* pay, size_t n, siz
     if (np == 1)
         return VELO_OK;
     std::vector<NetPass> passes;
-    plan_sort(logN, DQ_LT, DQ_LT - 5, passes);
-    b.net<RowKP>(DQ_K_SORT_KP, RowKP::Cols { k, pay }, NetGeom { n, logN, 0 }, nullptr, passes, DQ_LT);
+    plan_sort(logN, DQ_LT, DQ_LT - 4, passes);
+    b.net<RowKP>(DQ_K_SORT_KP, RowKP::Cols { k, pay }, NetGeom::trimmed(n, logN, DQ_LT, 1), nullptr, passes, DQ_LT);
     return VELO_OK;
 }
 
@@ -319,11 +318,11 @@ velo_status dq_plan_filter_groupby(DqPlan& p, const velo_lineitem* cols, size_t 
     b.step(W == 2 ? DQ_K_LI_PACK2 : DQ_K_LI_PACK3, s.n_rec >> lt, b.arg(pk));
     const uint64_t ntiles_np = logN > lt ? 1ull << (logN - lt) : 1;
     b.scan(s.counts, ntiles_np, s.prefix, s.d_rows);
-    // 2. ORCompact and 3. sort of the next_pow2(n) records
-    std::vector<NetPass> cp, sp;
-    plan_compact(logN, lt, lmax, cp);
+    // 2. sort the n records, passing ones first (the count of passing rows is
+    // the scan's total, so nothing has to be compacted before the sort)
+    std::vector<NetPass> sp;
     plan_sort(logN, lt, lmax, sp);
-    const NetGeom g { np, logN, 0 };
+    const NetGeom g = NetGeom::trimmed(n, logN, lt, 0);
     if (W == 2) {
         using R = LiTypes<2>::Rec;
         R::Cols rc;
@@ -336,7 +335,6 @@ velo_status dq_plan_filter_groupby(DqPlan& p, const velo_lineitem* cols, size_t 
         rc.mark_bit = 63;
         rc.mark_inv = 1;
         rc.mark_word = 0;
-        b.net<R>(DQ_K_COMPACT_LI2, rc, g, s.prefix, cp, lt);
         if (logN > 0)
             b.net<R>(DQ_K_SORT_LI2, rc, g, nullptr, sp, lt);
     } else {
@@ -351,11 +349,10 @@ velo_status dq_plan_filter_groupby(DqPlan& p, const velo_lineitem* cols, size_t 
         rc.mark_bit = 63;
         rc.mark_inv = 1;
         rc.mark_word = 0;
-        b.net<R>(DQ_K_COMPACT_LI3, rc, g, s.prefix, cp, lt);
         if (logN > 0)
             b.net<R>(DQ_K_SORT_LI3, rc, g, nullptr, sp, lt);
     }
-    // 4. segmented sums with the public output bound
+    // 3. segmented sums with the public output bound
     size_t nseg = np < (size_t)SEG_TS ? (size_t)SEG_TS : np;
     DqSegArgs sg;
     std::memset(&sg, 0, sizeof(sg));
@@ -427,7 +424,7 @@ velo_status dq_plan_join_topk(DqPlan& p, const velo_join_tables* t, const velo_j
     if (logU > 0) {
         std::vector<NetPass> sp;
         plan_sort(logU, DQ_LT, J_LMAX, sp);
-        b.net<JRec>(DQ_K_SORT_JREC, uc, NetGeom { (size_t)1 << logU, logU, 0 }, nullptr, sp, DQ_LT);
+        b.net<JRec>(DQ_K_SORT_JREC, uc, NetGeom::trimmed(t->n_dim + t->n_fact, logU, DQ_LT, 0), nullptr, sp, DQ_LT);
     }
     // 3. forward fill of the dimension side
     DqJFillArgs fa {};
@@ -439,13 +436,12 @@ velo_status dq_plan_join_topk(DqPlan& p, const velo_join_tables* t, const velo_j
     b.step(DQ_K_JFILL_SUMMARY, (uint64_t)fa.ntiles, fo);
     b.step(DQ_K_JFILL_CARRIES, 1, fo);
     b.step(DQ_K_JFILL_APPLY, (uint64_t)fa.ntiles, fo);
-    // 4. ORCompact of the joined fact rows
+    // 4. the number of joined fact rows.  They need no compaction: the joined
+    // rows of a key are neighbours (all its passing fact rows or none), so each
+    // is one run of (key, joined) for the segmented sums
     const uint64_t ntc = logR > DQ_LT ? 1ull << (logR - DQ_LT) : 1;
     b.count<JRec>(DQ_K_COUNT_JREC, uc, s.n_rec, DQ_LT, s.counts, ntc);
     b.scan(s.counts, ntc, s.prefix, s.n_joined);
-    std::vector<NetPass> cp;
-    plan_compact(logR, DQ_LT, J_LMAX, cp);
-    b.net<JRec>(DQ_K_COMPACT_JREC, uc, NetGeom { s.n_rec, logR, 0 }, s.prefix, cp, DQ_LT);
     // 5. group-by fk fused with the first top-k round
     const int nts = (int)(s.n_rec / SEG_TS);
     const int cand = k <= (uint32_t)J_TOPK_MIN ? J_TOPK_MIN : (int)next_pow2(k);

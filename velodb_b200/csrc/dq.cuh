@@ -43,11 +43,8 @@ enum DqKind : uint32_t {
     DQ_K_SORT_KP,
     DQ_K_COMPACT_KPM,
     DQ_K_SORT_LI2,
-    DQ_K_COMPACT_LI2,
     DQ_K_SORT_LI3,
-    DQ_K_COMPACT_LI3,
     DQ_K_SORT_JREC,
-    DQ_K_COMPACT_JREC,
     DQ_K_SORT_REC3,
     DQ_K_SORT_REC3K2,
     DQ_K_COMPACT_REC3K2,

@@ -38,8 +38,8 @@ constexpr size_t dq_max(size_t a, size_t b) { return a > b ? a : b; }
 // dynamic shared memory of the consumer: the largest step
 constexpr size_t DQ_SMEM = dq_max(
     dq_max(dq_max(NetKP::smem_bytes_sort(), NetKPM::smem_bytes_compact()),
-           dq_max(NetLI2::smem_bytes_compact(), NetLI3::smem_bytes_compact())),
-    dq_max(dq_max(NetJ::smem_bytes_compact(), dq_max(NetR3::smem_bytes_sort(), NetR3K2::smem_bytes_compact())),
+           dq_max(NetLI2::smem_bytes_sort(), NetLI3::smem_bytes_sort())),
+    dq_max(dq_max(NetJ::smem_bytes_sort(), dq_max(NetR3::smem_bytes_sort(), NetR3K2::smem_bytes_compact())),
            dq_max(dq_max(LiTypes<3>::Seg::SMEM, JSEG_TOPK_SMEM),
                   dq_max((size_t)2 * TK_RED_ROWS * 8, (size_t)FILL_TS_PAD * 8))));
 static_assert(DQ_SMEM <= 110 * 1024, "two consumer CTAs fit on an SM");
@@ -135,29 +135,14 @@ __device__ void dq_run(const DqStep& step, const unsigned char* s_args, uint32_t
         NetLI2::run<true>(A.c, A.g, step.pass, nullptr, (int)tile, sm);
         break;
     }
-    case DQ_K_COMPACT_LI2: {
-        const auto& A = dq_arg<DqNetArgs<DqLI2>>(s_args);
-        NetLI2::run<false>(A.c, A.g, step.pass, A.prefix, (int)tile, sm);
-        break;
-    }
     case DQ_K_SORT_LI3: {
         const auto& A = dq_arg<DqNetArgs<DqLI3>>(s_args);
         NetLI3::run<true>(A.c, A.g, step.pass, nullptr, (int)tile, sm);
         break;
     }
-    case DQ_K_COMPACT_LI3: {
-        const auto& A = dq_arg<DqNetArgs<DqLI3>>(s_args);
-        NetLI3::run<false>(A.c, A.g, step.pass, A.prefix, (int)tile, sm);
-        break;
-    }
     case DQ_K_SORT_JREC: {
         const auto& A = dq_arg<DqNetArgs<JRec>>(s_args);
         NetJ::run<true>(A.c, A.g, step.pass, nullptr, (int)tile, sm);
-        break;
-    }
-    case DQ_K_COMPACT_JREC: {
-        const auto& A = dq_arg<DqNetArgs<JRec>>(s_args);
-        NetJ::run<false>(A.c, A.g, step.pass, A.prefix, (int)tile, sm);
         break;
     }
     case DQ_K_SORT_REC3: {

@@ -50,6 +50,7 @@ static velo_status batch_plan(velo_batch* b, const velo_batch_item* items, size_
 {
     const int lt = b->log_nt + b->log_e;
     const int lmax = lt - 5 < 8 ? lt - 5 : 8;
+    const int lmax_sort = lt - 4 < 8 ? lt - 4 : 8; // as velo_osort_kp
     std::vector<std::vector<std::pair<uint32_t, NetPass>>> per(n_items); // (kind, pass) per instance
     std::vector<std::vector<uint32_t>> tiles(n_items);
     size_t scratch_u32 = 0;
@@ -81,10 +82,11 @@ static velo_status batch_plan(velo_batch* b, const velo_batch_item* items, size_
         std::vector<NetPass> passes;
         if (it.kind == VELO_ITEM_SORT_KP) {
             if (np > 1)
-                plan_sort(in.logN, lt, lmax, passes);
+                plan_sort(in.logN, lt, lmax_sort, passes);
+            const NetGeom g = NetGeom::trimmed(it.n, in.logN, lt, 1);
             for (auto& p : passes) {
                 per[i].push_back({ STEP_SORT_PASS, p });
-                tiles[i].push_back((uint32_t)ntiles);
+                tiles[i].push_back((uint32_t)net_pass_tiles(g, p, lt));
             }
         } else {
             per[i].push_back({ STEP_COMPACT_COUNT, NetPass {} });

@@ -127,7 +127,7 @@ struct Sched {
             switch (st.kind) {
             case STEP_SORT_PASS: {
                 RowKP::Cols c { in.k, in.p };
-                NS::template run<true>(c, g, st.pass, nullptr, tile, sm);
+                NS::template run<true>(c, NetGeom::trimmed(in.n, in.logN, LT, 1), st.pass, nullptr, tile, sm);
                 break;
             }
             case STEP_COMPACT_COUNT: {
