@@ -139,8 +139,16 @@ __device__ __forceinline__ void store_raw(const ColSpec& s, int c, size_t g, uin
     }
 }
 
+// How the row index rides along (row indices are below 2^31):
+//   FORM_WORD  a word of its own after the KW key words
+//   FORM_LOW   the low half of the last key word, where the key leaves it free
+//   FORM_K12   the 32-bit payload of 12-byte rows, KW = 1
+// 1.5 M rows by (DOUBLE, DATE), 96 key bits: 24-byte records in 8192-row tiles
+// 816 us, 16-byte ones 436 us.
+enum SortForm : int { FORM_WORD = 0, FORM_LOW = 1, FORM_K12 = 2 };
+
 // key bits are laid out MSB-first across KW words
-template <int KW>
+template <int KW, int FORM>
 __global__ void k_pack_cols(ColSpec s, size_t n, size_t np, uint64_t* words)
 {
     VELO_TRACE_KERNEL(velo_site_hash("k_pack_cols"));
@@ -165,14 +173,20 @@ __global__ void k_pack_cols(ColSpec s, size_t n, size_t np, uint64_t* words)
             }
             pos += bits;
         }
+        // row index rides along
+        if constexpr (FORM == FORM_LOW)
+            w[KW - 1] |= g;
 #pragma unroll
         for (int i = 0; i < KW; i++)
             words[(size_t)i * np + g] = w[i];
-        words[(size_t)KW * np + g] = g; // row index rides along
+        if constexpr (FORM == FORM_WORD)
+            words[(size_t)KW * np + g] = g;
+        if constexpr (FORM == FORM_K12)
+            reinterpret_cast<uint32_t*>(words + np)[g] = (uint32_t)g;
     }
 }
 
-template <int KW>
+template <int KW, int FORM>
 __global__ void k_unpack_cols(ColSpec s, size_t np, const uint64_t* words, int64_t* indices)
 {
     VELO_TRACE_KERNEL(velo_site_hash("k_unpack_cols"));
@@ -197,43 +211,67 @@ __global__ void k_unpack_cols(ColSpec s, size_t np, const uint64_t* words, int64
             store_raw(s, c, g, decode(s.type[c], s.asc[c] != 0, u & mask));
             pos += bits;
         }
-        indices[g] = (int64_t)words[(size_t)KW * np + g];
+        if constexpr (FORM == FORM_LOW)
+            indices[g] = (int64_t)(uint32_t)w[KW - 1];
+        else if constexpr (FORM == FORM_K12)
+            indices[g] = (int64_t) reinterpret_cast<const uint32_t*>(words + np)[g];
+        else
+            indices[g] = (int64_t)words[(size_t)KW * np + g];
     }
 }
 
-template <int KW, int LOG_NT, int LOG_E>
-static velo_status sort_cols_kw(const ColSpec& s, size_t n, int logN, uint64_t* words, int64_t* indices,
-                                cudaStream_t st)
+// columns of a row type over the packed words (array i at words + i * np)
+template <int W, int KW, int KM>
+static typename RowRec<W, KW, true, KM>::Cols sort_cols_of(RowRec<W, KW, true, KM>*, uint64_t* words, size_t np)
 {
-    using R = RowRec<KW + 1, KW>;
-    const size_t np = (size_t)1 << logN;
-    const int threads = 256;
-    const unsigned blocks = (unsigned)((np + threads - 1) / threads < 148 * 16 ? (np + threads - 1) / threads : 148 * 16);
-    k_pack_cols<KW><<<blocks, threads, 0, st>>>(s, n, np, words);
-    VELO_CUDA_TRY(cudaGetLastError(), "pack launch");
-    typename R::Cols c;
-    for (int i = 0; i <= KW; i++)
+    typename RowRec<W, KW, true, KM>::Cols c;
+    for (int i = 0; i < W; i++) {
         c.w[i] = words + (size_t)i * np;
+        c.pad[i] = ~0ull; // unused: every row (real or pad) is packed explicitly
+    }
     for (int i = 0; i < KW; i++)
         c.mask[i] = ~0ull;
-    for (int i = 0; i <= KW; i++)
-        c.pad[i] = ~0ull; // unused: every row (real or pad) is packed explicitly
     c.mark_bit = 0;
     c.mark_inv = 0;
     c.mark_word = 0;
+    return c;
+}
+static RowK12<K12_KEY>::Cols sort_cols_of(RowK12<K12_KEY>*, uint64_t* words, size_t np)
+{
+    return { words, reinterpret_cast<uint32_t*>(words + np) };
+}
+
+template <class R, int KW, int FORM, int LOG_NT, int LOG_E>
+static velo_status sort_cols(const ColSpec& s, size_t n, int logN, uint64_t* words, int64_t* indices, cudaStream_t st)
+{
+    const size_t np = (size_t)1 << logN;
+    const int threads = 256;
+    const unsigned blocks = (unsigned)((np + threads - 1) / threads < 148 * 16 ? (np + threads - 1) / threads : 148 * 16);
+    k_pack_cols<KW, FORM><<<blocks, threads, 0, st>>>(s, n, np, words);
+    VELO_CUDA_TRY(cudaGetLastError(), "pack launch");
     if (np > 1) {
         std::vector<NetPass> passes;
         const int lt = LOG_NT + LOG_E;
-        plan_sort(logN, lt, lt - 5 < 8 ? lt - 5 : 8, passes);
-        // every row is materialised by the pack kernel, so n = np here
+        plan_sort(logN, lt, FORM == FORM_WORD ? (lt - 5 < 8 ? lt - 5 : 8) : 8, passes);
+        // every row is materialised by the pack kernel, so n = np here; the
+        // order of equal keys is seen, so the padding stays in the network
         NetGeom g { np, logN, 0 };
-        velo_status rc = launch_net<R, LOG_NT, LOG_E>(c, g, passes, nullptr, st);
+        velo_status rc =
+            launch_net<R, LOG_NT, LOG_E>(sort_cols_of((R*)nullptr, words, np), g, passes, nullptr, st);
         if (rc != VELO_OK)
             return rc;
     }
-    k_unpack_cols<KW><<<blocks, threads, 0, st>>>(s, np, words, indices);
+    k_unpack_cols<KW, FORM><<<blocks, threads, 0, st>>>(s, np, words, indices);
     VELO_CUDA_TRY(cudaGetLastError(), "unpack launch");
     return VELO_OK;
+}
+
+static int key_bits(const uint32_t* types, uint32_t n_cols)
+{
+    int bits = 0;
+    for (uint32_t c = 0; c < n_cols; c++)
+        bits += type_bits(types[c]);
+    return bits;
 }
 
 static int key_words(const uint32_t* types, uint32_t n_cols)
@@ -298,18 +336,23 @@ extern "C" velo_status velo_sort_columns(void* const* d_cols, const uint32_t* ty
     }
     uint64_t* words = static_cast<uint64_t*>(d_scratch);
     cudaStream_t st = (cudaStream_t)stream;
+    const int bits = key_bits(types, n_cols);
+    if (bits <= 32)
+        return sort_cols<RowRec<1, 1, true, KEY_HI32>, 1, FORM_LOW, 8, 4>(s, n, logN, words, d_indices, st);
+    if (bits <= 64)
+        return sort_cols<RowK12<K12_KEY>, 1, FORM_K12, 8, 4>(s, n, logN, words, d_indices, st);
+    if (bits <= 96)
+        return sort_cols<RowRec<2, 2, true, KEY_HI96>, 2, FORM_LOW, 8, 4>(s, n, logN, words, d_indices, st);
     switch (kw) {
-    case 1:
-        return sort_cols_kw<1, 9, 4>(s, n, logN, words, d_indices, st);
     case 2:
-        return sort_cols_kw<2, 9, 4>(s, n, logN, words, d_indices, st);
+        return sort_cols<RowRec<3, 2>, 2, FORM_WORD, 8, 4>(s, n, logN, words, d_indices, st);
     // wider records take fewer rows a thread, so the row words stay in
     // registers (W x E words under the 128-register cap)
     case 3:
-        return sort_cols_kw<3, 9, 3>(s, n, logN, words, d_indices, st);
+        return sort_cols<RowRec<4, 3>, 3, FORM_WORD, 9, 3>(s, n, logN, words, d_indices, st);
     case 4:
-        return sort_cols_kw<4, 9, 2>(s, n, logN, words, d_indices, st);
+        return sort_cols<RowRec<5, 4>, 4, FORM_WORD, 9, 2>(s, n, logN, words, d_indices, st);
     default:
-        return sort_cols_kw<8, 9, 2>(s, n, logN, words, d_indices, st);
+        return sort_cols<RowRec<9, 8>, 8, FORM_WORD, 9, 2>(s, n, logN, words, d_indices, st);
     }
 }
