@@ -6,9 +6,17 @@
 //   oblivious:   position-map shuffle (device PRF + bitonic network),
 //                oblivious gather (union sort + fill + sort back),
 //                PK-FK equi-join producing (build rowid, probe rowid) pairs
+#include "k12.cuh"
 #include "ops.cuh"
 
 namespace velo {
+
+// instantiated in net_inst_kp_b.cu and net_inst_pipe.cu
+extern template velo_status launch_net<RowKP, 8, 4>(const RowKP::Cols&, const NetGeom&, const std::vector<NetPass>&,
+                                                    const uint32_t*, cudaStream_t);
+using Pair = RowRec<1, 1, false, KEY_FULL>;
+extern template velo_status launch_net<Pair, 8, 4>(const Pair::Cols&, const NetGeom&, const std::vector<NetPass>&,
+                                                   const uint32_t*, cudaStream_t);
 
 static unsigned grid_for(size_t n)
 {
@@ -83,29 +91,81 @@ __global__ void __launch_bounds__(1024) k_fill_scan(const FillCarry* tile_last, 
     fill_scan_body(tile_last, ntiles, carry, wsm);
 }
 
-__global__ void k_ogather_pack(const uint64_t* table, size_t tn, const uint32_t* rids, size_t rn, size_t rows,
-                               uint64_t* w0, uint64_t* w1, uint64_t* w2)
+__global__ void k_ogather_pack(const uint64_t* table, size_t tn, const uint32_t* rids, size_t rn, uint64_t* k,
+                               uint32_t* p)
 {
     VELO_TRACE_KERNEL(velo_site_hash("k_ogather_pack"));
-    ogather_pack_body(table, tn, rids, rn, rows, w0, w1, w2, blockIdx.x, gridDim.x);
+    VELO_BLK_STRIDE(g, tn + rn, blockIdx.x, gridDim.x)
+    {
+        uint64_t x;
+        uint32_t id, req;
+        if (g < tn) {
+            x = table[g];
+            id = (uint32_t)g;
+            req = 0;
+        } else {
+            const uint32_t r = rids[g - tn];
+            x = g - tn;
+            id = r < tn ? r : OG_NONE;
+            req = 1;
+        }
+        k[g] = ((uint64_t)id << 33) | ((uint64_t)req << 32) | (x >> 32);
+        p[g] = (uint32_t)x;
+    }
 }
 
-__global__ void k_ogather_out(const uint64_t* w1, size_t rn, uint64_t* out)
+__global__ void k_ogather_out(const uint64_t* k, const uint32_t* p, size_t rn, uint64_t* out)
 {
     VELO_TRACE_KERNEL(velo_site_hash("k_ogather_out"));
-    ogather_out_body(w1, rn, out, blockIdx.x, gridDim.x);
+    VELO_BLK_STRIDE(j, rn, blockIdx.x, gridDim.x)
+    out[j] = (k[j] << 32) | p[j];
 }
 
 __global__ void k_ojoin_pack(const void* bk, const uint8_t* bm, size_t bn, const void* pk, const uint8_t* pm, size_t pn,
-                             int key64, size_t rows, uint64_t* w0, uint64_t* w1, uint64_t* w2)
+                             int key64, uint64_t* k, uint32_t* p, unsigned long long* stat)
 {
     VELO_TRACE_KERNEL(velo_site_hash("k_ojoin_pack"));
+    if (blockIdx.x == 0 && threadIdx.x == 0)
+        *stat = 0;
+    VELO_BLK_STRIDE(g, bn + pn, blockIdx.x, gridDim.x)
+    {
+        const bool build = g < bn;
+        const size_t j = build ? g : g - bn;
+        const void* keys = build ? bk : pk;
+        const uint8_t* mask = build ? bm : pm;
+        const uint64_t key = key64 ? ((uint64_t) static_cast<const int64_t*>(keys)[j] ^ 0x8000000000000000ull)
+                                   : (uint64_t)((uint32_t) static_cast<const int32_t*>(keys)[j] ^ 0x80000000u);
+        const bool valid = mask == nullptr || mask[j] != 0;
+        k[g] = key;
+        p[g] = (build ? 0u : OJ12_TAG) | (valid ? OJ12_VALID : 0u) | (uint32_t)j;
+    }
+}
+
+__global__ void k_ojoin_out(const uint64_t* w, size_t pn, int64_t* ob, int64_t* op, const uint64_t* n_joined,
+                            const unsigned long long* dups, uint64_t* d_counts)
+{
+    VELO_TRACE_KERNEL(velo_site_hash("k_ojoin_out"));
+    VELO_BLK_STRIDE(i, pn, blockIdx.x, gridDim.x)
+    {
+        const uint64_t x = w[i];
+        const bool j = x != ~0ull;
+        ob[i] = j ? (int64_t)(x >> 30) : -1;
+        op[i] = j ? (int64_t)(x & OJ12_ROWID) : -1;
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0)
+        join_counts_body(n_joined, dups, d_counts);
+}
+
+__global__ void k_ojoin_pack_rec(const void* bk, const uint8_t* bm, size_t bn, const void* pk, const uint8_t* pm, size_t pn,
+                             int key64, size_t rows, uint64_t* w0, uint64_t* w1, uint64_t* w2)
+{
+    VELO_TRACE_KERNEL(velo_site_hash("k_ojoin_pack_rec"));
     ojoin_pack_body(bk, bm, bn, pk, pm, pn, key64, rows, w0, w1, w2, blockIdx.x, gridDim.x);
 }
 
-__global__ void k_ojoin_out(const uint64_t* w1, const uint64_t* w2, size_t pn, int64_t* ob, int64_t* op)
+__global__ void k_ojoin_out_rec(const uint64_t* w1, const uint64_t* w2, size_t pn, int64_t* ob, int64_t* op)
 {
-    VELO_TRACE_KERNEL(velo_site_hash("k_ojoin_out"));
+    VELO_TRACE_KERNEL(velo_site_hash("k_ojoin_out_rec"));
     ojoin_out_body(w1, w2, pn, ob, op, blockIdx.x, gridDim.x);
 }
 
@@ -120,6 +180,50 @@ __global__ void k_join_counts(const uint64_t* n_joined, const unsigned long long
 {
     VELO_TRACE_KERNEL(velo_site_hash("k_join_counts"));
     join_counts_body(n_joined, dups, d_counts);
+}
+
+// The join over more than 2^30 rows, whose row ids do not fit beside the tag in
+// 32 bits: 24-byte records, the same network and results.
+static velo_status ojoin_records(const UnionScratch& s, size_t rows, int logR, const void* d_build_keys,
+                                 const uint8_t* d_build_mask, size_t build_n, const void* d_probe_keys,
+                                 const uint8_t* d_probe_mask, size_t probe_n, uint32_t key_type,
+                                 int64_t* d_out_build_rowid, int64_t* d_out_probe_rowid, uint64_t* d_counts,
+                                 cudaStream_t st)
+{
+    k_zero_u64<<<1, 32, 0, st>>>(s.stat, 1);
+    k_ojoin_pack_rec<<<grid_for(rows), 256, 0, st>>>(d_build_keys, d_build_mask, build_n, d_probe_keys, d_probe_mask,
+                                                 probe_n, key_type == VELO_BIGINT, rows, s.w[0], s.w[1], s.w[2]);
+    VELO_CUDA_TRY(cudaGetLastError(), "ojoin pack launch");
+    Rec3K2::Cols c;
+    for (int i = 0; i < 3; i++) {
+        c.w[i] = s.w[i];
+        c.pad[i] = ~0ull;
+    }
+    c.mask[0] = ~0ull;
+    c.mask[1] = OJ_TAG;
+    c.mark_word = 1;
+    c.mark_bit = 61;
+    c.mark_inv = 0;
+    std::vector<NetPass> passes;
+    plan_sort(logR, OP_LT, OP_LMAX, passes);
+    velo_status rc = launch_net12<Rec3K2>(c, NetGeom { rows, logR, 0 }, passes, nullptr, st);
+    if (rc != VELO_OK)
+        return rc;
+    rc = run_fill<JoinFill>(s.w[0], s.w[1], s.w[2], rows, s.tl, s.carry, s.stat, st);
+    if (rc != VELO_OK)
+        return rc;
+    const int nct = (int)(rows >> OP_LT);
+    k_count_marks<Rec3K2><<<nct, 256, 0, st>>>(c, rows, OP_LT, s.counts);
+    k_scan_tiles<<<1, 1024, 0, st>>>(s.counts, nct, s.prefix, s.n_marked);
+    std::vector<NetPass> cp;
+    plan_compact(logR, OP_LT, OP_LMAX, cp);
+    rc = launch_net12<Rec3K2>(c, NetGeom { rows, logR, 0 }, cp, s.prefix, st);
+    if (rc != VELO_OK)
+        return rc;
+    k_ojoin_out_rec<<<grid_for(probe_n), 256, 0, st>>>(s.w[1], s.w[2], probe_n, d_out_build_rowid, d_out_probe_rowid);
+    k_join_counts<<<1, 1, 0, st>>>(s.n_marked, s.stat, d_counts);
+    VELO_CUDA_TRY(cudaGetLastError(), "ojoin out launch");
+    return VELO_OK;
 }
 
 } // namespace velo
@@ -304,9 +408,9 @@ extern "C" velo_status velo_oshuffle_position_map(uint32_t* d_map, size_t n, uin
     }
     uint64_t* k = static_cast<uint64_t*>(d_scratch);
     uint32_t* p = reinterpret_cast<uint32_t*>(static_cast<char*>(d_scratch) + align_up(np * 8, 256));
-    k_shuffle_pack<<<grid_for(np), 256, 0, st>>>(d_map, n, np, counter, key, k, p);
+    k_shuffle_pack<<<grid_for(n), 256, 0, st>>>(d_map, n, n, counter, key, k, p);
     VELO_CUDA_TRY(cudaGetLastError(), "shuffle pack launch");
-    velo_status rc = velo_osort_kp(k, p, np, np, nullptr, stream);
+    velo_status rc = velo_osort_kp(k, p, n, np, nullptr, stream); // pads rows n .. np - 1
     if (rc != VELO_OK)
         return rc;
     k_copy_u32<<<grid_for(n), 256, 0, st>>>(d_map, p, n);
@@ -340,30 +444,38 @@ extern "C" velo_status velo_ogather_u64(const uint64_t* d_table, size_t table_n,
         set_error("velo_ogather_u64: scratch must hold velo_ogather_scratch_bytes() bytes");
         return VELO_ENOMEM;
     }
-    k_ogather_pack<<<grid_for(rows), 256, 0, st>>>(d_table, table_n, d_rids, n_req, rows, s.w[0], s.w[1], s.w[2]);
+    const size_t n = table_n + n_req;
+    uint64_t* k = s.w[0];
+    uint32_t* p = reinterpret_cast<uint32_t*>(s.w[1]);
+    k_ogather_pack<<<grid_for(n), 256, 0, st>>>(d_table, table_n, d_rids, n_req, k, p);
     VELO_CUDA_TRY(cudaGetLastError(), "ogather pack launch");
-    Rec3::Cols c;
-    for (int i = 0; i < 3; i++) {
-        c.w[i] = s.w[i];
-        c.pad[i] = ~0ull;
+    // each table row, then the requests for it
+    const RowKP::Cols c { k, p };
+    velo_status rc = sort_kp_rows(c, n, ilog2_floor(next_pow2(n)), 0, st);
+    if (rc != VELO_OK)
+        return rc;
+    rc = run_fill_k12<GatherK12>(k, p, n, GatherK12::Out { k, p }, s.tl, s.carry, nullptr, st);
+    if (rc != VELO_OK)
+        return rc;
+    // back to request order.  When at most half the rows are requests they are
+    // compacted first (three passes), so that only they are sorted; above, the
+    // passes would cost more than the rows they keep out of the sort
+    size_t m = n;
+    if (n_req <= n / 2) {
+        rc = launch_count_scan<RowKP>(c, n, logR, OP_LT, s.counts, s.prefix, nullptr, st);
+        if (rc != VELO_OK)
+            return rc;
+        std::vector<NetPass> cp;
+        plan_compact(logR, OP_LT, OP_LMAX_COMPACT, cp);
+        rc = launch_net<RowKP, 8, 4>(c, NetGeom(n, logR), cp, s.prefix, st);
+        if (rc != VELO_OK)
+            return rc;
+        m = n_req;
     }
-    c.mask[0] = 0xFFFFFFFF80000000ull;
-    c.mark_bit = 0;
-    c.mark_inv = 0;
-    c.mark_word = 0;
-    std::vector<NetPass> passes;
-    plan_sort(logR, OP_LT, OP_LMAX, passes);
-    velo_status rc = launch_net12<Rec3>(c, NetGeom { rows, logR, 0 }, passes, nullptr, st);
+    rc = sort_kp_rows(c, m, ilog2_floor(next_pow2(m)), 0, st);
     if (rc != VELO_OK)
         return rc;
-    rc = run_fill<GatherFill>(s.w[0], s.w[1], s.w[2], rows, s.tl, s.carry, nullptr, st);
-    if (rc != VELO_OK)
-        return rc;
-    c.mask[0] = ~0ull;
-    rc = launch_net12<Rec3>(c, NetGeom { rows, logR, 0 }, passes, nullptr, st);
-    if (rc != VELO_OK)
-        return rc;
-    k_ogather_out<<<grid_for(n_req), 256, 0, st>>>(s.w[1], n_req, d_out);
+    k_ogather_out<<<grid_for(n_req), 256, 0, st>>>(k, p, n_req, d_out);
     VELO_CUDA_TRY(cudaGetLastError(), "ogather out launch");
     return VELO_OK;
 }
@@ -404,38 +516,43 @@ extern "C" velo_status velo_ojoin_pkfk(const void* d_build_keys, const uint8_t* 
         set_error("velo_ojoin_pkfk: scratch must hold velo_ojoin_scratch_bytes() bytes");
         return VELO_ENOMEM;
     }
-    k_zero_u64<<<1, 32, 0, st>>>(s.stat, 1);
-    k_ojoin_pack<<<grid_for(rows), 256, 0, st>>>(d_build_keys, d_build_mask, build_n, d_probe_keys, d_probe_mask,
-                                                 probe_n, key_type == VELO_BIGINT, rows, s.w[0], s.w[1], s.w[2]);
+    const size_t n = build_n + probe_n;
+    if (n > (size_t)1 << 30)
+        return ojoin_records(s, rows, logR, d_build_keys, d_build_mask, build_n, d_probe_keys, d_probe_mask, probe_n,
+                             key_type, d_out_build_rowid, d_out_probe_rowid, d_counts, st);
+    uint64_t* k = s.w[0];
+    uint32_t* p = reinterpret_cast<uint32_t*>(s.w[1]);
+    k_ojoin_pack<<<grid_for(n), 256, 0, st>>>(d_build_keys, d_build_mask, build_n, d_probe_keys, d_probe_mask, probe_n,
+                                              key_type == VELO_BIGINT, k, p, s.stat);
     VELO_CUDA_TRY(cudaGetLastError(), "ojoin pack launch");
-    Rec3K2::Cols c;
-    for (int i = 0; i < 3; i++) {
-        c.w[i] = s.w[i];
-        c.pad[i] = ~0ull;
-    }
-    c.mask[0] = ~0ull;
-    c.mask[1] = OJ_TAG;
-    c.mark_word = 1;
-    c.mark_bit = 61;
-    c.mark_inv = 0;
+    // sort on (key, tag); the probe rows of a key are seen in the padded
+    // network's order, so the padding stays in it
     std::vector<NetPass> passes;
     plan_sort(logR, OP_LT, OP_LMAX, passes);
-    velo_status rc = launch_net12<Rec3K2>(c, NetGeom { rows, logR, 0 }, passes, nullptr, st);
+    velo_status rc = launch_net<RowK12<K12_KEY_TAG>, 8, 4>({ k, p }, NetGeom(n, logR), passes, nullptr, st);
     if (rc != VELO_OK)
         return rc;
-    rc = run_fill<JoinFill>(s.w[0], s.w[1], s.w[2], rows, s.tl, s.carry, s.stat, st);
+    // pairs, one word each, compacted to the front
+    rc = run_fill_k12<JoinK12>(k, p, rows, JoinK12::Out { s.w[2] }, s.tl, s.carry, s.stat, st);
     if (rc != VELO_OK)
         return rc;
-    const int nct = (int)(rows >> OP_LT);
-    k_count_marks<Rec3K2><<<nct, 256, 0, st>>>(c, rows, OP_LT, s.counts);
-    k_scan_tiles<<<1, 1024, 0, st>>>(s.counts, nct, s.prefix, s.n_marked);
+    Pair::Cols c;
+    c.w[0] = s.w[2];
+    c.mask[0] = ~0ull;
+    c.pad[0] = ~0ull;
+    c.mark_word = 0;
+    c.mark_bit = 63;
+    c.mark_inv = 1;
+    rc = launch_count_scan<Pair>(c, rows, logR, OP_LT, s.counts, s.prefix, s.n_marked, st);
+    if (rc != VELO_OK)
+        return rc;
     std::vector<NetPass> cp;
-    plan_compact(logR, OP_LT, OP_LMAX, cp);
-    rc = launch_net12<Rec3K2>(c, NetGeom { rows, logR, 0 }, cp, s.prefix, st);
+    plan_compact(logR, OP_LT, OP_LMAX_COMPACT, cp);
+    rc = launch_net<Pair, 8, 4>(c, NetGeom(rows, logR), cp, s.prefix, st);
     if (rc != VELO_OK)
         return rc;
-    k_ojoin_out<<<grid_for(probe_n), 256, 0, st>>>(s.w[1], s.w[2], probe_n, d_out_build_rowid, d_out_probe_rowid);
-    k_join_counts<<<1, 1, 0, st>>>(s.n_marked, s.stat, d_counts);
+    k_ojoin_out<<<grid_for(probe_n), 256, 0, st>>>(s.w[2], probe_n, d_out_build_rowid, d_out_probe_rowid, s.n_marked,
+                                                   s.stat, d_counts);
     VELO_CUDA_TRY(cudaGetLastError(), "ojoin out launch");
     return VELO_OK;
 }

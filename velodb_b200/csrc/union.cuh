@@ -236,6 +236,9 @@ constexpr int OP_LT = 12; // 4096-row tiles (CTA shape per record width: Tile12)
 // up to 8 fused global levels: the 16 contiguous rows a segment keeps of
 // each 8-byte word array fill a 128-byte line
 constexpr int OP_LMAX = OP_LT - 4 < 8 ? OP_LT - 4 : 8;
+// the compactions up to 10 (4-row segments, a 32-byte sector of a word array):
+// 9 levels of 2^21 24-byte rows in one pass 40 us, in two passes of 8 and 1 59
+constexpr int OP_LMAX_COMPACT = OP_LT - 2;
 
 // scratch of the union-sort operators: 3 words x rows + fill carries + compaction
 inline size_t union_rows(size_t n)
