@@ -16,10 +16,13 @@
 //               number of groups)
 // Every address depends only on n, group_bound and the key type.  INTEGER
 // keys share word 0 with the exclusion bit.  BIGINT keys use all 64 bits of
-// word 0 (key ^ 2^63), so their records carry the row's validity in a word of
-// its own, sorted after the key: within a key the rows left out come first,
-// so a key run ends on a valid row exactly when it holds one; their group
-// records carry the group flag in a word of its own too (segagg FLAG_WORD).
+// word 0 (key ^ 2^63).  A row left out becomes the largest word, ~0, which is
+// also the key 2^63 - 1: the rows that really have that key are summed while
+// they are packed and packed as rows left out, and their group, the last in
+// key order, is added at the output.  So these records need no word for the
+// row's validity: (key, sum) 16 bytes where (key, validity, sum, sum) took 32,
+// and 24-byte group records (key, flag | count, sum) where they took 40;
+// 2 M rows, SUM and COUNT: 1,145 -> 530 us.
 #include "net_impl.cuh"
 #include "segagg.cuh"
 
@@ -28,6 +31,8 @@ namespace velo {
 constexpr int GB_LT = 12; // 4096-row tiles (CTA shape per record width: Tile12)
 // up to 8 fused global levels: 16 contiguous rows of 8-byte words fill a line
 constexpr int GB_LMAX = GB_LT - 4 < 8 ? GB_LT - 4 : 8;
+// compactions: up to 10 (4-row segments of a 32-byte sector)
+constexpr int GB_LMAX_COMPACT = GB_LT - 2;
 constexpr uint64_t GB_EXCL = 1ull << 63;
 constexpr int64_t GB_BIG = (int64_t)1 << 62;
 
@@ -53,35 +58,38 @@ struct GbAgg {
     __device__ __forceinline__ static uint64_t out_bits(uint64_t key) { return key & ~GB_EXCL; }
 };
 
-// BIGINT keys: records (key ^ 2^63, validity, sum 0, sum 1); aggregates
-// (count, sum 0, sum 1) -- the ones not asked for are computed on zeros and
-// dropped at the output
+// BIGINT keys: records (key ^ 2^63, NS sums), ~0 a row left out; the count is
+// always the first aggregate (it carries the group flag) and dropped at the
+// output when it is not asked for
+template <int NS>
 struct GbAggWide {
-    static constexpr int W = 4;
-    static constexpr int V = 3;
-    static constexpr bool FLAG_WORD = true;
+    static constexpr int W = 1 + NS;
+    static constexpr int V = 1 + NS;
+    static constexpr bool FLAG_IN_COUNT = true;
     struct Params { };
     __device__ __forceinline__ static uint64_t key(const uint64_t* w) { return w[0]; }
-    __device__ __forceinline__ static bool valid(const uint64_t* w) { return (w[1] & 1ull) != 0; }
+    __device__ __forceinline__ static bool valid(const uint64_t* w) { return w[0] != ~0ull; }
     __device__ __forceinline__ static void values(const uint64_t* w, int64_t (&v)[V], const Params&)
     {
         const bool ok = valid(w);
         v[0] = ok ? 1 : 0;
-        v[1] = ok ? (int64_t)w[2] : 0;
-        v[2] = ok ? (int64_t)w[3] : 0;
+#pragma unroll
+        for (int s = 0; s < NS; s++)
+            v[1 + s] = ok ? (int64_t)w[1 + s] : 0;
     }
     __device__ __forceinline__ static int64_t out_key_from(uint64_t key) { return (int64_t)(key ^ (1ull << 63)); }
     __device__ __forceinline__ static uint64_t out_bits(uint64_t key) { return key; }
 };
 
 // the per-tile run and carry arrays of the scratch hold 3 values a tile
-static_assert(GbAggWide::V <= 3 && GbAgg<2, 0>::V <= 3 && GbAgg<1, 1>::V <= 3, "aggregates a tile in scratch");
+static_assert(GbAggWide<2>::V <= 3 && GbAgg<2, 0>::V <= 3 && GbAgg<1, 1>::V <= 3, "aggregates a tile in scratch");
 
+template <int NS>
 struct GbTypesWide {
-    using Agg = GbAggWide;
+    using Agg = GbAggWide<NS>;
     using Seg = SegAgg<Agg>;
-    using Rec = RowRec<4, 2, false, KEY_FULL>; // sorted on (key, validity)
-    using Grp = RowRec<5, 1, false>;           // key, flag, count, sum 0, sum 1
+    using Rec = RowRec<1 + NS, 1, false, KEY_FULL>; // sorted on the key word
+    using Grp = RowRec<2 + NS, 1, false, KEY_FULL>; // group records, compaction only
 };
 
 template <int NS, int CNT>
@@ -89,7 +97,7 @@ struct GbTypes {
     using Agg = GbAgg<NS, CNT>;
     using Seg = SegAgg<Agg>;
     using Rec = RowRec<1 + NS, 1, false, KEY_FULL>;  // sorted on the whole of word 0
-    using Grp = RowRec<1 + NS + CNT, 1, false>;      // group records, compaction only
+    using Grp = RowRec<1 + NS + CNT, 1, false, KEY_FULL>; // group records, compaction only
 };
 
 struct GbIn {
@@ -151,49 +159,74 @@ __global__ void __launch_bounds__(256) k_gb_pack(GbIn in, size_t n, size_t np, u
         atomicAdd(d_rejected, (unsigned long long)total);
 }
 
-__global__ void __launch_bounds__(256) k_gb_pack_wide(GbIn in, int n_sums, size_t n, size_t np, uint64_t* w0,
-                                                      uint64_t* w1, uint64_t* w2, uint64_t* w3)
+// extra: (count, sums) of the rows with the key 2^63 - 1
+template <int NS>
+__global__ void __launch_bounds__(256) k_gb_pack_wide(GbIn in, size_t n, uint64_t* w0, uint64_t* w1, uint64_t* w2,
+                                                      unsigned long long* extra)
 {
     VELO_TRACE_KERNEL(velo_site_hash("k_gb_pack_wide"));
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; VELO_GRID_COND(i, np);
+    __shared__ int64_t red[8][1 + NS];
+    int64_t top[1 + NS];
+#pragma unroll
+    for (int s = 0; s <= NS; s++)
+        top[s] = 0;
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; VELO_GRID_COND(i, n);
          i += (size_t)gridDim.x * blockDim.x) {
-        uint64_t k = ~0ull, f = 0, s0 = 0, s1 = 0;
-        if (i < n) {
-            k = (uint64_t) static_cast<const int64_t*>(in.keys)[i] ^ (1ull << 63);
-            f = (in.mask ? in.mask[i] != 0 : true) ? 1ull : 0ull;
-            s0 = n_sums >= 1 ? (uint64_t)in.sums[0][i] : 0ull;
-            s1 = n_sums >= 2 ? (uint64_t)in.sums[1][i] : 0ull;
-        }
+        const uint64_t k = (uint64_t) static_cast<const int64_t*>(in.keys)[i] ^ (1ull << 63);
+        const bool take = in.mask ? in.mask[i] != 0 : true;
+        const bool last = take & (k == ~0ull);
+        top[0] += last ? 1 : 0;
         VELO_TRACE_AT(TS_ROW_STORE, w0 + i);
-        w0[i] = k;
-        w1[i] = f;
-        w2[i] = s0;
-        w3[i] = s1;
+        w0[i] = take ? k : ~0ull;
+#pragma unroll
+        for (int s = 0; s < NS; s++) {
+            const int64_t x = in.sums[s][i];
+            top[1 + s] += last ? x : 0;
+            (s == 0 ? w1 : w2)[i] = (uint64_t)x;
+        }
+    }
+    // one update per CTA at fixed addresses
+#pragma unroll
+    for (int s = 0; s <= NS; s++) {
+        top[s] = warp_sum_i64(top[s]);
+        if ((threadIdx.x & 31) == 0)
+            red[threadIdx.x >> 5][s] = top[s];
+    }
+    __syncthreads();
+    if (threadIdx.x <= NS) {
+        int64_t t = 0;
+        for (int w = 0; w < 8; w++)
+            t += red[w][threadIdx.x];
+        atomicAdd(extra + threadIdx.x, (unsigned long long)t);
     }
 }
 
-__global__ void __launch_bounds__(SEG_THREADS) k_gbw_summary(GbTypesWide::Rec::Cols c, SegTileAgg* aggs, int64_t* runs)
+template <int NS>
+__global__ void __launch_bounds__(SEG_THREADS) k_gbw_summary(typename GbTypesWide<NS>::Rec::Cols c, SegTileAgg* aggs,
+                                                             int64_t* runs)
 {
     VELO_TRACE_KERNEL(velo_site_hash("k_gbw_summary"));
     extern __shared__ __align__(16) char sm[];
-    GbTypesWide::Seg::tile_summary(c.w, blockIdx.x, aggs, runs, {}, sm);
+    GbTypesWide<NS>::Seg::tile_summary(c.w, blockIdx.x, aggs, runs, {}, sm);
 }
 
+template <int NS>
 __global__ void __launch_bounds__(1024) k_gbw_carries(const SegTileAgg* aggs, const int64_t* runs, int ntiles,
                                                       int64_t* carry_in, uint32_t* tail_prefix, uint64_t* n_groups)
 {
     VELO_TRACE_KERNEL(velo_site_hash("k_gbw_carries"));
     extern __shared__ __align__(16) char sm[];
-    GbTypesWide::Seg::carries(aggs, runs, ntiles, carry_in, tail_prefix, n_groups, sm);
+    GbTypesWide<NS>::Seg::carries(aggs, runs, ntiles, carry_in, tail_prefix, n_groups, sm);
 }
 
-__global__ void __launch_bounds__(SEG_THREADS) k_gbw_emit_rows(GbTypesWide::Rec::Cols c, int ntiles,
+template <int NS>
+__global__ void __launch_bounds__(SEG_THREADS) k_gbw_emit_rows(typename GbTypesWide<NS>::Rec::Cols c, int ntiles,
                                                                const SegTileAgg* aggs, const int64_t* carry_in,
-                                                               GbTypesWide::Grp::Cols g)
+                                                               typename GbTypesWide<NS>::Grp::Cols g)
 {
     VELO_TRACE_KERNEL(velo_site_hash("k_gbw_emit_rows"));
     extern __shared__ __align__(16) char sm[];
-    GbTypesWide::Seg::emit_rows(c.w, blockIdx.x, ntiles, aggs, carry_in, g.w, {}, sm);
+    GbTypesWide<NS>::Seg::emit_rows(c.w, blockIdx.x, ntiles, aggs, carry_in, g.w, {}, sm);
 }
 
 template <int NS, int CNT>
@@ -259,28 +292,31 @@ __global__ void k_gb_out(const uint64_t* g0, const uint64_t* g1, const uint64_t*
     }
 }
 
-// wide group records: g[0] = key ^ 2^63, g[1] = flag, g[2] count, g[3..4] sums
+// wide group records: g[0] = key ^ 2^63, g[1] = flag | count, g[2..3] sums; the
+// group of the key 2^63 - 1 follows the others
 struct GbwWords {
-    const uint64_t* g[5];
+    const uint64_t* g[4];
 };
 
-__global__ void k_gbw_out(GbwWords g, size_t bound, int n_sums, int with_count, GbOut out,
-                          const uint64_t* n_groups, uint64_t* d_counts)
+__global__ void k_gbw_out(GbwWords g, size_t bound, int n_sums, int with_count, GbOut out, const uint64_t* n_groups,
+                          const unsigned long long* extra, uint64_t* d_counts)
 {
     VELO_TRACE_KERNEL(velo_site_hash("k_gbw_out"));
     const uint64_t ng = *n_groups;
+    const bool top = extra[0] != 0;
     for (size_t j = blockIdx.x * (size_t)blockDim.x + threadIdx.x; VELO_GRID_COND(j, bound);
          j += (size_t)gridDim.x * blockDim.x) {
         const bool ok = j < ng;
+        const bool lst = top & (j == ng);
         VELO_TRACE_AT(TS_ROW_LOAD, g.g[0] + j);
-        out.keys[j] = ok ? (int64_t)(g.g[0][j] ^ (1ull << 63)) : 0;
+        out.keys[j] = lst ? (int64_t)~(1ull << 63) : ok ? (int64_t)(g.g[0][j] ^ (1ull << 63)) : 0;
         if (with_count)
-            out.counts[j] = ok ? (int64_t)g.g[2][j] : 0;
+            out.counts[j] = lst ? (int64_t)extra[0] : ok ? (int64_t)g.g[1][j] : 0;
         for (int s = 0; s < n_sums; s++)
-            out.sums[s][j] = ok ? (int64_t)g.g[3 + s][j] : 0;
+            out.sums[s][j] = lst ? (int64_t)extra[1 + s] : ok ? (int64_t)g.g[2 + s][j] : 0;
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
-        d_counts[0] = ng;
+        d_counts[0] = ng + (top ? 1 : 0);
         d_counts[1] = 0;
     }
 }
@@ -359,10 +395,12 @@ static velo_status gb_run(const GbScratch& s, const GbIn& in, size_t n, size_t b
         if (dev >= 0 && dev < 64)
             done[dev] = 1;
     }
-    const size_t np = s.n_rec;
-    const int logN = ilog2_floor(np);
+    const int logN = ilog2_floor(s.n_rec);
+    // the sort leaves out the padding past the last tile; so do the later steps
+    const NetGeom geom = NetGeom::trimmed(n, logN, GB_LT, 0);
+    const size_t m = geom.m;
     VELO_CUDA_TRY(cudaMemsetAsync(s.rejected, 0, 8, st), "cudaMemsetAsync");
-    k_gb_pack<NS><<<gb_grid(np), 256, 0, st>>>(in, n, np, s.r[0], s.r[1], s.r[2], s.rejected);
+    k_gb_pack<NS><<<gb_grid(n), 256, 0, st>>>(in, n, n, s.r[0], s.r[1], s.r[2], s.rejected);
     VELO_CUDA_TRY(cudaGetLastError(), "group-by pack launch");
 
     typename T::Rec::Cols rc;
@@ -376,11 +414,11 @@ static velo_status gb_run(const GbScratch& s, const GbIn& in, size_t n, size_t b
     rc.mark_word = 0;
     std::vector<NetPass> passes;
     plan_sort(logN, GB_LT, GB_LMAX, passes);
-    velo_status rc2 = launch_net12<typename T::Rec>(rc, NetGeom { np, logN, 0 }, passes, nullptr, st);
+    velo_status rc2 = launch_net12<typename T::Rec>(rc, geom, passes, nullptr, st);
     if (rc2 != VELO_OK)
         return rc2;
 
-    const int nts = (int)(np / SEG_TS);
+    const int nts = (int)(m / SEG_TS);
     typename T::Grp::Cols gc;
     for (int i = 0; i < 1 + NS + CNT; i++) {
         gc.w[i] = s.g[i];
@@ -396,12 +434,12 @@ static velo_status gb_run(const GbScratch& s, const GbIn& in, size_t n, size_t b
     k_gb_emit_rows<NS, CNT><<<nts, SEG_THREADS, Seg::SMEM, st>>>(rc, nts, s.aggs, s.carry, gc);
     VELO_CUDA_TRY(cudaGetLastError(), "group-by aggregation launch");
 
-    const int ntc = (int)(np >> GB_LT);
-    k_count_marks<typename T::Grp><<<ntc, 256, 0, st>>>(gc, np, GB_LT, s.counts);
-    k_scan_tiles<<<1, 1024, 0, st>>>(s.counts, ntc, s.prefix, s.n_grp_rows);
+    rc2 = launch_count_scan<typename T::Grp>(gc, m, logN, GB_LT, s.counts, s.prefix, s.n_grp_rows, st);
+    if (rc2 != VELO_OK)
+        return rc2;
     passes.clear();
-    plan_compact(logN, GB_LT, GB_LMAX, passes);
-    rc2 = launch_net12<typename T::Grp>(gc, NetGeom { np, logN, 0 }, passes, s.prefix, st);
+    plan_compact(logN, GB_LT, GB_LMAX_COMPACT, passes);
+    rc2 = launch_net12<typename T::Grp>(gc, NetGeom(m, logN), passes, s.prefix, st);
     if (rc2 != VELO_OK)
         return rc2;
     k_gb_out<NS, CNT><<<gb_grid(bound), 256, 0, st>>>(s.g[0], s.g[1], s.g[2], bound, in.key_type, out, s.n_groups,
@@ -410,48 +448,50 @@ static velo_status gb_run(const GbScratch& s, const GbIn& in, size_t n, size_t b
     return VELO_OK;
 }
 
-// BIGINT keys over their whole range: the same steps on wide records
-static velo_status gb_run_wide(const GbScratch& s, const GbIn& in, int n_sums, int with_count, size_t n, size_t bound,
-                               GbOut out, uint64_t* d_counts, cudaStream_t st)
+// BIGINT keys over their whole range: the same steps on their records
+template <int NS>
+static velo_status gb_run_wide(const GbScratch& s, const GbIn& in, int with_count, size_t n, size_t bound, GbOut out,
+                               uint64_t* d_counts, cudaStream_t st)
 {
-    using T = GbTypesWide;
-    using Seg = T::Seg;
+    using T = GbTypesWide<NS>;
+    using Seg = typename T::Seg;
     static int done[64] = {};
     int dev = 0;
     VELO_CUDA_TRY(cudaGetDevice(&dev), "cudaGetDevice");
     if (dev < 0 || dev >= 64 || !done[dev]) {
-        VELO_CUDA_TRY(cudaFuncSetAttribute(k_gbw_summary, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        VELO_CUDA_TRY(cudaFuncSetAttribute(k_gbw_summary<NS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            (int)Seg::SMEM_IN),
                       "cudaFuncSetAttribute");
-        VELO_CUDA_TRY(cudaFuncSetAttribute(k_gbw_emit_rows, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        VELO_CUDA_TRY(cudaFuncSetAttribute(k_gbw_emit_rows<NS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            (int)Seg::SMEM),
                       "cudaFuncSetAttribute");
         if (dev >= 0 && dev < 64)
             done[dev] = 1;
     }
-    const size_t np = s.n_rec;
-    const int logN = ilog2_floor(np);
-    k_gb_pack_wide<<<gb_grid(np), 256, 0, st>>>(in, n_sums, n, np, s.r[0], s.r[1], s.r[2], s.r[3]);
+    const int logN = ilog2_floor(s.n_rec);
+    const NetGeom geom = NetGeom::trimmed(n, logN, GB_LT, 0);
+    const size_t m = geom.m;
+    unsigned long long* extra = s.rejected; // 3 words of its 256 bytes
+    VELO_CUDA_TRY(cudaMemsetAsync(extra, 0, 24, st), "cudaMemsetAsync");
+    k_gb_pack_wide<NS><<<gb_grid(n), 256, 0, st>>>(in, n, s.r[0], s.r[1], s.r[2], extra);
     VELO_CUDA_TRY(cudaGetLastError(), "group-by pack launch");
-    T::Rec::Cols rc;
-    for (int i = 0; i < 4; i++) {
+    typename T::Rec::Cols rc;
+    for (int i = 0; i < 1 + NS; i++) {
         rc.w[i] = s.r[i];
         rc.pad[i] = ~0ull;
     }
-    rc.pad[1] = 0; // network pads, if any, are rows left out
     rc.mask[0] = ~0ull;
-    rc.mask[1] = ~0ull;
     rc.mark_bit = 0;
     rc.mark_inv = 0;
-    rc.mark_word = 1;
+    rc.mark_word = 0;
     std::vector<NetPass> passes;
     plan_sort(logN, GB_LT, GB_LMAX, passes);
-    velo_status rc2 = launch_net12<T::Rec>(rc, NetGeom { np, logN, 0 }, passes, nullptr, st);
+    velo_status rc2 = launch_net12<typename T::Rec>(rc, geom, passes, nullptr, st);
     if (rc2 != VELO_OK)
         return rc2;
-    const int nts = (int)(np / SEG_TS);
-    T::Grp::Cols gc;
-    for (int i = 0; i < 5; i++) {
+    const int nts = (int)(m / SEG_TS);
+    typename T::Grp::Cols gc;
+    for (int i = 0; i < 2 + NS; i++) {
         gc.w[i] = s.g[i];
         gc.pad[i] = ~0ull;
     }
@@ -459,23 +499,23 @@ static velo_status gb_run_wide(const GbScratch& s, const GbIn& in, int n_sums, i
     gc.mark_bit = 63;
     gc.mark_inv = 1;
     gc.mark_word = 1;
-    k_gbw_summary<<<nts, SEG_THREADS, Seg::SMEM_IN, st>>>(rc, s.aggs, s.runs);
-    k_gbw_carries<<<1, 1024, 3 * 1024 * 8 + 2 * 1024 * 4, st>>>(s.aggs, s.runs, nts, s.carry, s.tail_prefix,
-                                                                s.n_groups);
-    k_gbw_emit_rows<<<nts, SEG_THREADS, Seg::SMEM, st>>>(rc, nts, s.aggs, s.carry, gc);
+    k_gbw_summary<NS><<<nts, SEG_THREADS, Seg::SMEM_IN, st>>>(rc, s.aggs, s.runs);
+    k_gbw_carries<NS><<<1, 1024, (1 + NS) * 1024 * 8 + 2 * 1024 * 4, st>>>(s.aggs, s.runs, nts, s.carry,
+                                                                           s.tail_prefix, s.n_groups);
+    k_gbw_emit_rows<NS><<<nts, SEG_THREADS, Seg::SMEM, st>>>(rc, nts, s.aggs, s.carry, gc);
     VELO_CUDA_TRY(cudaGetLastError(), "group-by aggregation launch");
-    const int ntc = (int)(np >> GB_LT);
-    k_count_marks<T::Grp><<<ntc, 256, 0, st>>>(gc, np, GB_LT, s.counts);
-    k_scan_tiles<<<1, 1024, 0, st>>>(s.counts, ntc, s.prefix, s.n_grp_rows);
+    rc2 = launch_count_scan<typename T::Grp>(gc, m, logN, GB_LT, s.counts, s.prefix, s.n_grp_rows, st);
+    if (rc2 != VELO_OK)
+        return rc2;
     passes.clear();
-    plan_compact(logN, GB_LT, GB_LMAX, passes);
-    rc2 = launch_net12<T::Grp>(gc, NetGeom { np, logN, 0 }, passes, s.prefix, st);
+    plan_compact(logN, GB_LT, GB_LMAX_COMPACT, passes);
+    rc2 = launch_net12<typename T::Grp>(gc, NetGeom(m, logN), passes, s.prefix, st);
     if (rc2 != VELO_OK)
         return rc2;
     GbwWords gw;
-    for (int i = 0; i < 5; i++)
+    for (int i = 0; i < 4; i++)
         gw.g[i] = s.g[i];
-    k_gbw_out<<<gb_grid(bound), 256, 0, st>>>(gw, bound, n_sums, with_count, out, s.n_groups, d_counts);
+    k_gbw_out<<<gb_grid(bound), 256, 0, st>>>(gw, bound, NS, with_count, out, s.n_groups, extra, d_counts);
     VELO_CUDA_TRY(cudaGetLastError(), "group-by output launch");
     return VELO_OK;
 }
@@ -523,8 +563,12 @@ extern "C" velo_status velo_ogroupby(const void* d_keys, uint32_t key_type, cons
         out.sums[i] = d_out_sums[i];
     }
     cudaStream_t st = (cudaStream_t)stream;
-    if (key_type == VELO_BIGINT)
-        return gb_run_wide(s, in, (int)n_sums, with_count ? 1 : 0, n, group_bound, out, d_counts, st);
+    if (key_type == VELO_BIGINT) {
+        const int cnt = with_count ? 1 : 0;
+        return n_sums == 0 ? gb_run_wide<0>(s, in, cnt, n, group_bound, out, d_counts, st)
+            : n_sums == 1  ? gb_run_wide<1>(s, in, cnt, n, group_bound, out, d_counts, st)
+                           : gb_run_wide<2>(s, in, cnt, n, group_bound, out, d_counts, st);
+    }
     if (with_count && n_sums == 0)
         return gb_run<0, 1>(s, in, n, group_bound, out, d_counts, st);
     if (with_count && n_sums == 1)

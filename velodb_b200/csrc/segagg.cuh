@@ -142,16 +142,16 @@ __device__ __forceinline__ void warp_reduce_scatter16(int64_t (&a)[16], int lane
     a[0] += __shfl_xor_sync(0xffffffffu, a[0], 1);
 }
 
-// Group records with a separate flag word (Agg::FLAG_WORD = true): o0 = the
-// whole 64-bit out_bits(key), o1 = [63] not the last row of a valid group,
-// then the sums; otherwise the flag shares word 0 with a key of at most 63 bits.
+// Group records of a 64-bit key (Agg::FLAG_IN_COUNT = true): o0 = the whole
+// out_bits(key), o1 = [63] not the last row of a valid group | the first value,
+// a count; otherwise the flag shares word 0 with a key of at most 63 bits.
 template <class A, class = void>
-struct SegFlagWord {
+struct SegFlagInCount {
     static constexpr bool value = false;
 };
 template <class A>
-struct SegFlagWord<A, std::void_t<decltype(A::FLAG_WORD)>> {
-    static constexpr bool value = A::FLAG_WORD;
+struct SegFlagInCount<A, std::void_t<decltype(A::FLAG_IN_COUNT)>> {
+    static constexpr bool value = A::FLAG_IN_COUNT;
 };
 
 // Agg: static constexpr int W (record words), V (values); struct Params
@@ -164,9 +164,10 @@ template <class Agg>
 struct SegAgg {
     static constexpr int W = Agg::W;
     static constexpr int V = Agg::V;
-    // group record words of emit_rows: key (and flag), then the V sums
-    static constexpr int FW = SegFlagWord<Agg>::value ? 1 : 0;
-    static constexpr int OW = 1 + FW + V;
+    // group record words of emit_rows: key, then the V sums; the flag in word
+    // 1 (FC) or word 0
+    static constexpr bool FC = SegFlagInCount<Agg>::value;
+    static constexpr int OW = 1 + V;
     // the tile area holds the W input words, later the OW output words
     static constexpr int TW = W > OW ? W : OW;
     using Params = typename Agg::Params;
@@ -668,15 +669,12 @@ struct SegAgg {
                 if (r > 0)
                     lead = lead & (keys[r] == keys[r - 1]);
                 const bool first_run_of_tile = (keys[r] == head_key);
-                if constexpr (FW == 1) {
-                    regs[r][0] = Agg::out_bits(keys[r]);
-                    regs[r][1] = (uint64_t)(!tail[r]) << 63;
-                } else {
-                    regs[r][0] = ((uint64_t)(!tail[r]) << 63) | Agg::out_bits(keys[r]);
-                }
+                const uint64_t flag = (uint64_t)(!tail[r]) << 63;
+                regs[r][0] = (FC ? 0ull : flag) | Agg::out_bits(keys[r]);
 #pragma unroll
                 for (int i = 0; i < V; i++)
-                    regs[r][1 + FW + i] = (uint64_t)(pref[r][i] + (lead ? cin[i] : 0) + (first_run_of_tile ? tc[i] : 0));
+                    regs[r][1 + i] = (uint64_t)(pref[r][i] + (lead ? cin[i] : 0) + (first_run_of_tile ? tc[i] : 0))
+                        | (FC && i == 0 ? flag : 0ull);
             }
             return;
         }
@@ -688,16 +686,13 @@ struct SegAgg {
             if (r > 0)
                 lead = lead & (keys[r] == keys[r - 1]);
             const bool first_run_of_tile = (keys[r] == head_key);
-            if constexpr (FW == 1) {
-                so[seg_slot(r0 + r)] = Agg::out_bits(keys[r]);
-                so[(size_t)SEG_TS_PAD + seg_slot(r0 + r)] = (uint64_t)(!tail[r]) << 63;
-            } else {
-                so[seg_slot(r0 + r)] = ((uint64_t)(!tail[r]) << 63) | Agg::out_bits(keys[r]);
-            }
+            const uint64_t flag = (uint64_t)(!tail[r]) << 63;
+            so[seg_slot(r0 + r)] = (FC ? 0ull : flag) | Agg::out_bits(keys[r]);
 #pragma unroll
             for (int i = 0; i < V; i++)
-                so[(size_t)(1 + FW + i) * SEG_TS_PAD + seg_slot(r0 + r)] =
-                    (uint64_t)(pref[r][i] + (lead ? cin[i] : 0) + (first_run_of_tile ? tc[i] : 0));
+                so[(size_t)(1 + i) * SEG_TS_PAD + seg_slot(r0 + r)] =
+                    (uint64_t)(pref[r][i] + (lead ? cin[i] : 0) + (first_run_of_tile ? tc[i] : 0))
+                    | (FC && i == 0 ? flag : 0ull);
         }
         __syncthreads();
     }
