@@ -78,8 +78,10 @@ const char* velo_last_error_text(void);
  * after each stage and synchronize that stream before returning; the stage
  * durations of the calling thread's last such call are then read with
  * velo_last_stage_times (ms, in stage order; returns how many were written).
- *   velo_filter_groupby:    pack, compact, sort, aggregate
- *   velo_join_groupby_topk: pack, sort, fill, compact, aggregate, top-k
+ *   velo_filter_groupby:    keys, sort, groups, sums
+ *   velo_join_groupby_topk: pack, sort, aggregate, top-k (with price_hi =
+ *                           INT64_MAX: pack, sort, fill, count, aggregate,
+ *                           top-k)
  * No reference counterpart: a measurement hook of this implementation.
  */
 void velo_set_stage_timing(int on);
@@ -135,8 +137,9 @@ int velo_last_pass_times(velo_pass_time* out, int capacity);
  * (key, payload).  Replaces OP_SORT / executeBitonicSort
  * (include/cuda/sort.cuh:70-118, include/cuda/commands.hpp:68-76) for two
  * sort columns: same network (k ascending, j descending, partner i^j,
- * direction (i&k)==0), same exchange rule (swap iff strictly out of order),
- * so the output is identical to the reference network's.  Buffers hold
+ * direction (i&k)==0; when n is not a power of two the directions count from
+ * the last block and the exchanges with padding are left out).  Every field
+ * is compared, so the output is identical to the reference network's.  Buffers hold
  * capacity >= velo_next_pow2(n) rows; rows [n, next_pow2(n)) are filled with
  * the sentinel (UINT64_MAX, UINT32_MAX) and sort last. */
 velo_status velo_osort_kp(uint64_t* d_keys, uint32_t* d_payload, size_t n, size_t capacity, const velo_tune* tune,
@@ -473,18 +476,20 @@ typedef struct velo_lineitem_pred {
     int32_t qty_lo, qty_hi;
 } velo_lineitem_pred;
 
-/* flags: sort only next_pow2(filtered count) rows after compaction, reading
- * the count back to the host first (the reference FilterCompactionOperator
- * reveals it, src/operator/filter_compaction_operator.cpp:171-178).  Without
- * this flag the whole pipeline is oblivious and never synchronises. */
+/* flags: the caller does not mind the filtered count being revealed (the
+ * reference FilterCompactionOperator reads it back to the host,
+ * src/operator/filter_compaction_operator.cpp:171-178).  Accepted and without
+ * effect: no step needs the count on the host, with or without the flag the
+ * whole pipeline is oblivious and never synchronises. */
 #define VELO_REVEAL_COUNT 1u
 
 /* Oblivious filter + GROUP BY (flag1, flag2) with exact int64 sums:
- * predicate and record packing on the GPU (replacing the CPU predicate of
- * src/operator/seq_scan_operator.cpp:38-45), ORCompact of passing rows
- * (replacing src/operator/filter_compaction_operator.cpp:65-184), bitonic
- * sort on the group key, segmented sums
- * (obliviator/operator_2/enclave/scalable_oblivious_join.c:221-262, int64
+ * predicate on the GPU (replacing the CPU predicate of
+ * src/operator/seq_scan_operator.cpp:38-45 and the compaction of
+ * src/operator/filter_compaction_operator.cpp:65-184), bitonic sort of the
+ * passing rows' 16-bit group keys, the first group_bound distinct keys, and one
+ * pass that adds every row to every group's slot with masks (the sums of
+ * obliviator/operator_2/enclave/scalable_oblivious_join.c:221-262, int64
  * instead of float), output padded to the public bound group_bound (1..16).
  * d_out: group_bound rows x 6 int64 = (flag1 << 8 | flag2, count, sum qty,
  * sum price, sum price*(100-disc), sum price*(100-disc)*(100+tax)) in key
@@ -520,8 +525,9 @@ typedef struct velo_join_pred {
  * reference's sort-merge join kernels and operator
  * (include/cuda/sort_merge_join.cuh:63-199,
  * src/operator/sort_merge_join_operator.cpp:27-257) with union -> bitonic
- * sort on (key, tag) -> forward fill -> ORCompact -> segmented sums ->
- * bitonic top-k network on (sum desc, fk asc) (each group-by tile keeps its
+ * sort on (key, side) -> segmented sums per key, kept where the key has a
+ * passing dimension row -> bitonic top-k network on (sum desc, fk asc) (each
+ * group-by tile keeps its
  * best max(16, next_pow2(k)) groups, then rounds over candidate blocks).
  * k is 1..1024.  d_out: k rows x 3 int64 = (fk, sum price, count), unused
  * rows zero.  d_counts: 2 u64 = (joined fact rows, groups). */
