@@ -296,105 +296,40 @@ velo_status dq_plan_filter_groupby(DqPlan& p, const velo_lineitem* cols, size_t 
         return VELO_ENOMEM;
     }
     const LiCols c { cols->qty, cols->price, cols->disc, cols->tax, cols->shipdate, cols->flag1, cols->flag2 };
-    const LiParams prm { pred->qty_lo, pred->disc_lo, band_bits(pred->qty_lo, pred->qty_hi), 0 };
-    const int W = prm.qbits + band_bits(pred->disc_lo, pred->disc_hi) <= (uint32_t)LI_FIELD_BITS ? 2 : 3;
-    // two-word records in 4096-row tiles, three-word records in 2048-row tiles
-    const int lt = W == 2 ? DQ_LT : DQ_LT3;
-    const int lmax = lt - 4 < 8 ? lt - 4 : 8;
-    const size_t np = next_pow2(n);
-    const int logN = ilog2_floor(np);
-    // 1. predicate + pack, per-tile pass counts, their scan
-    DqLiPackArgs pk;
-    std::memset(&pk, 0, sizeof(pk));
-    pk.c = c;
-    pk.p = *pred;
-    pk.prm = prm;
-    pk.n = n;
-    pk.n_rec = s.n_rec;
-    pk.lt = lt;
-    for (int i = 0; i < 3; i++)
-        pk.w[i] = s.w[i];
-    pk.counts = s.counts;
-    b.step(W == 2 ? DQ_K_LI_PACK2 : DQ_K_LI_PACK3, s.n_rec >> lt, b.arg(pk));
-    const uint64_t ntiles_np = logN > lt ? 1ull << (logN - lt) : 1;
-    b.scan(s.counts, ntiles_np, s.prefix, s.d_rows);
-    // 2. sort the n records, passing ones first (the count of passing rows is
-    // the scan's total, so nothing has to be compacted before the sort)
-    std::vector<NetPass> sp;
-    plan_sort(logN, lt, lmax, sp);
-    const NetGeom g = NetGeom::trimmed(n, logN, lt, 0);
-    if (W == 2) {
-        using R = LiTypes<2>::Rec;
-        R::Cols rc;
-        std::memset(&rc, 0, sizeof(rc));
-        for (int i = 0; i < 2; i++) {
-            rc.w[i] = s.w[i];
-            rc.pad[i] = ~0ull;
-        }
-        rc.mask[0] = LI_KEYMASK;
-        rc.mark_bit = 63;
-        rc.mark_inv = 1;
-        rc.mark_word = 0;
-        if (logN > 0)
-            b.net<R>(DQ_K_SORT_LI2, rc, g, nullptr, sp, lt);
-    } else {
-        using R = LiTypes<3>::Rec;
-        R::Cols rc;
-        std::memset(&rc, 0, sizeof(rc));
-        for (int i = 0; i < 3; i++) {
-            rc.w[i] = s.w[i];
-            rc.pad[i] = ~0ull;
-        }
-        rc.mask[0] = LI_KEYMASK;
-        rc.mark_bit = 63;
-        rc.mark_inv = 1;
-        rc.mark_word = 0;
-        if (logN > 0)
-            b.net<R>(DQ_K_SORT_LI3, rc, g, nullptr, sp, lt);
+    // the steps of run_groupby (groupby.cu)
+    DqLiArgs a;
+    std::memset(&a, 0, sizeof(a));
+    a.c = c;
+    a.p = *pred;
+    a.n = n;
+    a.q = lk_plan(s, n, DQ_LK_LT, 0xFFFFFFFFu);
+    a.out = d_out;
+    a.d_counts = d_counts;
+    a.G = (int)group_bound;
+    a.chunks = (a.G + DQ_LK_SLOTS - 1) / DQ_LK_SLOTS;
+    const uint32_t ao = b.arg(a);
+    const LkPlan& q = a.q;
+    b.step(DQ_K_LI_KEYS, q.nblk, ao);
+    if (q.h > 1) {
+        std::vector<NetPass> sp;
+        plan_sort(q.logH, DQ_LK_LT, LK_LMAX, sp);
+        b.net<RowU2>(DQ_K_SORT_U2, RowU2::Cols { q.ka }, NetGeom::trimmed(q.h, q.logH, DQ_LK_LT, 0), nullptr, sp,
+                     DQ_LK_LT);
     }
-    // 3. segmented sums with the public output bound
-    size_t nseg = np < (size_t)SEG_TS ? (size_t)SEG_TS : np;
-    DqSegArgs sg;
-    std::memset(&sg, 0, sizeof(sg));
-    for (int i = 0; i < 3; i++)
-        sg.w[i] = s.w[i];
-    sg.aggs = s.aggs;
-    sg.runs = s.runs;
-    sg.carry = s.carry;
-    sg.tail_prefix = s.tail_prefix;
-    sg.n_groups = s.n_groups;
-    sg.tile_out = s.tile_out;
-    sg.out = d_out;
-    sg.d_rows = s.d_rows;
-    sg.d_counts = d_counts;
-    sg.prm = prm;
-    sg.ntiles = (int)(nseg / SEG_TS);
-    sg.G = (int)group_bound;
-    const uint32_t sa = b.arg(sg);
-    b.step(W == 2 ? DQ_K_SEG_SUMMARY2 : DQ_K_SEG_SUMMARY3, (uint64_t)sg.ntiles, sa);
-    b.step(W == 2 ? DQ_K_SEG_CARRIES2 : DQ_K_SEG_CARRIES3, 1, sa);
-    b.step(W == 2 ? DQ_K_SEG_EMIT2 : DQ_K_SEG_EMIT3, (uint64_t)sg.ntiles, sa);
-    b.step(DQ_K_SEG_FINISH, (uint64_t)group_bound * (1 + LI_V), sa);
+    b.step(DQ_K_LI_FOLD, (q.N + DQ_ELEM_ITEM - 1) / DQ_ELEM_ITEM, ao);
+    std::vector<NetPass> mp;
+    plan_merge(q.logN, DQ_LK_LT, LK_LMAX, q.logN, mp);
+    b.net<RowU2>(DQ_K_SORT_U2, RowU2::Cols { q.kb }, NetGeom(q.N, q.logN), nullptr, mp, DQ_LK_LT);
+    b.step(DQ_K_LI_DISTINCT, (uint64_t)q.ntiles, ao);
+    b.step(DQ_K_LI_SLOTS, (uint64_t)q.ntiles, ao);
+    b.step(DQ_K_LI_SUMS, (n + DQ_ELEM_ITEM - 1) / DQ_ELEM_ITEM * (uint64_t)a.chunks, ao);
     return VELO_OK;
 }
 
-velo_status dq_plan_join_topk(DqPlan& p, const velo_join_tables* t, const velo_join_pred* pred, uint32_t k,
-                              int64_t* d_out, uint64_t* d_counts, void* d_scratch, size_t scratch_bytes)
+// the record form (join_records, join.cu) up to its candidates
+static size_t plan_join_records(B& b, const JoinScratch& s, const velo_join_tables* t, const velo_join_pred* pred,
+                                int cand)
 {
-    B b(p);
-    if (!t || !pred || !d_out || !d_counts)
-        return einval("velo_join_groupby_topk: null argument");
-    if (!t->dim_key || !t->dim_date || !t->fact_fk || !t->fact_price || t->n_dim == 0)
-        return einval("velo_join_groupby_topk: null column or empty dimension table");
-    if (k == 0 || k > 1024)
-        return einval("velo_join_groupby_topk: k must be 1..1024");
-    if (t->n_dim + t->n_fact > ((size_t)1 << MAX_LOGN))
-        return einval("velo_join_groupby_topk: tables too large");
-    const JoinScratch s = join_layout(static_cast<char*>(d_scratch), t->n_dim, t->n_fact);
-    if (!d_scratch || scratch_bytes < s.bytes) {
-        set_error("velo_join_groupby_topk: scratch must hold velo_join_groupby_topk_scratch_bytes() bytes");
-        return VELO_ENOMEM;
-    }
     const int logR = ilog2_floor(s.n_rec);
     const int logU = ilog2_floor(next_pow2(t->n_dim + t->n_fact));
     // 1. pack
@@ -444,7 +379,6 @@ velo_status dq_plan_join_topk(DqPlan& p, const velo_join_tables* t, const velo_j
     b.scan(s.counts, ntc, s.prefix, s.n_joined);
     // 5. group-by fk fused with the first top-k round
     const int nts = (int)(s.n_rec / SEG_TS);
-    const int cand = k <= (uint32_t)J_TOPK_MIN ? J_TOPK_MIN : (int)next_pow2(k);
     DqJSegArgs ja;
     std::memset(&ja, 0, sizeof(ja));
     ja.c = uc;
@@ -461,10 +395,79 @@ velo_status dq_plan_join_topk(DqPlan& p, const velo_join_tables* t, const velo_j
     b.step(DQ_K_JSEG_SUMMARY, (uint64_t)nts, jo);
     b.step(DQ_K_JSEG_CARRIES, 1, jo);
     b.step(DQ_K_JSEG_EMIT_TOPK, (uint64_t)nts, jo);
-    // 6. top-k rounds over blocks of candidates (the union area is free now)
+    return (size_t)nts * cand;
+}
+
+// the 12-byte form (join_rows, join.cu) up to its candidates
+static size_t plan_join_rows(B& b, const JoinScratch& s, const velo_join_tables* t, const velo_join_pred* pred, int cand)
+{
+    const size_t n = t->n_dim + t->n_fact;
+    const int logU = ilog2_floor(next_pow2(n));
+    const int nt = (int)((n + JK_TS - 1) / JK_TS);
+    const int nts = (int)next_pow2((size_t)nt);
+    DqJkArgs a {};
+    a.dk = t->dim_key;
+    a.dd = t->dim_date;
+    a.ff = t->fact_fk;
+    a.fp = t->fact_price;
+    a.nd = t->n_dim;
+    a.nf = t->n_fact;
+    a.date_hi = pred->date_hi;
+    a.price_hi = pred->price_hi;
+    a.k = s.u[0];
+    a.p = reinterpret_cast<uint32_t*>(s.u[1]);
+    a.aggs = s.aggs;
+    a.runs = s.runs;
+    a.carry = s.carry;
+    a.n_groups = s.n_groups;
+    a.n_joined = s.n_joined;
+    a.out0 = s.cand[0];
+    a.out1 = s.cand[1];
+    a.ntiles = nt;
+    a.cand = cand;
+    const uint32_t ao = b.arg(a);
+    b.step(DQ_K_JK_PACK, (n + DQ_ELEM_ITEM - 1) / DQ_ELEM_ITEM, ao);
+    if (n > 1) {
+        std::vector<NetPass> sp;
+        plan_sort(logU, DQ_LT, DQ_LT - 4, sp);
+        b.net<RowKP>(DQ_K_SORT_KP, RowKP::Cols { a.k, a.p }, NetGeom::trimmed(n, logU, DQ_LT, 0), nullptr, sp, DQ_LT);
+    }
+    DqJSegArgs ja;
+    std::memset(&ja, 0, sizeof(ja));
+    ja.aggs = s.aggs;
+    ja.runs = s.runs;
+    ja.carry = s.carry;
+    ja.tail_prefix = s.tail_prefix;
+    ja.n_groups = s.unused;
+    ja.ntiles = nt;
+    b.step(DQ_K_JK_SUMMARY, (uint64_t)nt, ao);
+    b.step(DQ_K_JSEG_CARRIES, 1, b.arg(ja));
+    b.step(DQ_K_JK_EMIT_TOPK, (uint64_t)nts, ao);
+    return (size_t)nts * cand;
+}
+
+velo_status dq_plan_join_topk(DqPlan& p, const velo_join_tables* t, const velo_join_pred* pred, uint32_t k,
+                              int64_t* d_out, uint64_t* d_counts, void* d_scratch, size_t scratch_bytes)
+{
+    B b(p);
+    if (!t || !pred || !d_out || !d_counts)
+        return einval("velo_join_groupby_topk: null argument");
+    if (!t->dim_key || !t->dim_date || !t->fact_fk || !t->fact_price || t->n_dim == 0)
+        return einval("velo_join_groupby_topk: null column or empty dimension table");
+    if (k == 0 || k > 1024)
+        return einval("velo_join_groupby_topk: k must be 1..1024");
+    if (t->n_dim + t->n_fact > ((size_t)1 << MAX_LOGN))
+        return einval("velo_join_groupby_topk: tables too large");
+    const JoinScratch s = join_layout(static_cast<char*>(d_scratch), t->n_dim, t->n_fact);
+    if (!d_scratch || scratch_bytes < s.bytes) {
+        set_error("velo_join_groupby_topk: scratch must hold velo_join_groupby_topk_scratch_bytes() bytes");
+        return VELO_ENOMEM;
+    }
+    const int cand = k <= (uint32_t)J_TOPK_MIN ? J_TOPK_MIN : (int)next_pow2(k);
+    size_t n_c = pred->price_hi < INT64_MAX ? plan_join_rows(b, s, t, pred, cand) : plan_join_records(b, s, t, pred, cand);
+    // top-k rounds over blocks of candidates (the union area is free now)
     uint64_t* cur[2] = { s.cand[0], s.cand[1] };
     uint64_t* nxt[2] = { s.u[0], s.u[1] };
-    size_t n_c = (size_t)nts * cand;
     while (n_c > (size_t)cand) {
         const int rn = n_c < (size_t)TK_RED_ROWS ? (int)n_c : TK_RED_ROWS;
         const size_t blocks = n_c / rn;

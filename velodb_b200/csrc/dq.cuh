@@ -42,8 +42,6 @@ enum DqKind : uint32_t {
     // network passes (tile = item)
     DQ_K_SORT_KP,
     DQ_K_COMPACT_KPM,
-    DQ_K_SORT_LI2,
-    DQ_K_SORT_LI3,
     DQ_K_SORT_JREC,
     DQ_K_SORT_REC3,
     DQ_K_SORT_REC3K2,
@@ -54,16 +52,16 @@ enum DqKind : uint32_t {
     DQ_K_COUNT_REC3K2,
     DQ_K_SCAN_TILES,
     // filter + group-by
-    DQ_K_LI_PACK2,
-    DQ_K_LI_PACK3,
-    DQ_K_SEG_SUMMARY2,
-    DQ_K_SEG_SUMMARY3,
-    DQ_K_SEG_CARRIES2,
-    DQ_K_SEG_CARRIES3,
-    DQ_K_SEG_EMIT2,
-    DQ_K_SEG_EMIT3,
-    DQ_K_SEG_FINISH,
+    DQ_K_SORT_U2,
+    DQ_K_LI_KEYS,
+    DQ_K_LI_FOLD,
+    DQ_K_LI_DISTINCT,
+    DQ_K_LI_SLOTS,
+    DQ_K_LI_SUMS,
     // join + group-by + top-k
+    DQ_K_JK_PACK,
+    DQ_K_JK_SUMMARY,
+    DQ_K_JK_EMIT_TOPK,
     DQ_K_JOIN_PACK,
     DQ_K_JFILL_SUMMARY,
     DQ_K_JFILL_CARRIES,
@@ -158,30 +156,36 @@ struct DqScanArgs {
     int ntiles;
 };
 
-struct DqLiPackArgs {
+struct DqLiArgs {
     LiCols c;
     velo_lineitem_pred p;
-    LiParams prm;
-    size_t n, n_rec;
-    int lt;
-    uint64_t* w[3];
-    uint32_t* counts;
+    size_t n;
+    LkPlan q;
+    int64_t* out;
+    uint64_t* d_counts;
+    int G;
+    int chunks; // chunks of DQ_LK_SLOTS slots: the sums' item i is block i / chunks
 };
+// slots of one sums item (20 sums a thread under the consumer's 128 registers)
+constexpr int DQ_LK_SLOTS = 4;
+// 8192-word key tiles (256 threads x 32 words)
+constexpr int DQ_LK_LT = 13;
 
-struct DqSegArgs {
-    uint64_t* w[3];
+struct DqJkArgs {
+    const int32_t *dk, *dd, *ff;
+    const int64_t* fp;
+    size_t nd, nf;
+    int32_t date_hi;
+    int64_t price_hi;
+    uint64_t* k;
+    uint32_t* p;
     SegTileAgg* aggs;
     int64_t* runs;
     int64_t* carry;
-    uint32_t* tail_prefix;
-    uint64_t* n_groups;
-    int64_t* tile_out;
-    int64_t* out;
-    const uint64_t* d_rows;
-    uint64_t* d_counts;
-    LiParams prm;
+    uint64_t *n_groups, *n_joined;
+    uint64_t *out0, *out1;
     int ntiles;
-    int G;
+    int cand;
 };
 
 struct DqJoinPackArgs {

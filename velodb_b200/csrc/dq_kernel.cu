@@ -24,12 +24,10 @@
 
 namespace velo {
 
-using DqLI2 = LiTypes<2>::Rec;
-using DqLI3 = LiTypes<3>::Rec;
 using NetKP = Net<RowKP, 8, 4>;
 using NetKPM = Net<RowKPM, 8, 4>;
-using NetLI2 = Net<DqLI2, 8, 4>;
-using NetLI3 = Net<DqLI3, 8, 3>;
+using NetU2 = Net<RowU2, 8, 5>;
+static_assert(NetU2::LT == DQ_LK_LT, "the planned key tile");
 using NetJ = Net<JRec, 8, 4>;
 using NetR3 = Net<Rec3, 8, 3>;
 using NetR3K2 = Net<Rec3K2, 8, 3>;
@@ -38,9 +36,9 @@ constexpr size_t dq_max(size_t a, size_t b) { return a > b ? a : b; }
 // dynamic shared memory of the consumer: the largest step
 constexpr size_t DQ_SMEM = dq_max(
     dq_max(dq_max(NetKP::smem_bytes_sort(), NetKPM::smem_bytes_compact()),
-           dq_max(NetLI2::smem_bytes_sort(), NetLI3::smem_bytes_sort())),
+           dq_max(NetU2::smem_bytes_sort(), dq_max((size_t)LK_SM * 4, JK_EMIT_SMEM))),
     dq_max(dq_max(NetJ::smem_bytes_sort(), dq_max(NetR3::smem_bytes_sort(), NetR3K2::smem_bytes_compact())),
-           dq_max(dq_max(LiTypes<3>::Seg::SMEM, JSEG_TOPK_SMEM),
+           dq_max(JSEG_TOPK_SMEM,
                   dq_max((size_t)2 * TK_RED_ROWS * 8, (size_t)FILL_TS_PAD * 8))));
 static_assert(DQ_SMEM <= 110 * 1024, "two consumer CTAs fit on an SM");
 static_assert(TK_RED_ROWS / 2 % DQ_THREADS == 0, "top-k rounds: whole compare-exchanges a thread");
@@ -130,16 +128,6 @@ __device__ void dq_run(const DqStep& step, const unsigned char* s_args, uint32_t
         NetKPM::run<false>(A.c, A.g, step.pass, A.prefix, (int)tile, sm);
         break;
     }
-    case DQ_K_SORT_LI2: {
-        const auto& A = dq_arg<DqNetArgs<DqLI2>>(s_args);
-        NetLI2::run<true>(A.c, A.g, step.pass, nullptr, (int)tile, sm);
-        break;
-    }
-    case DQ_K_SORT_LI3: {
-        const auto& A = dq_arg<DqNetArgs<DqLI3>>(s_args);
-        NetLI3::run<true>(A.c, A.g, step.pass, nullptr, (int)tile, sm);
-        break;
-    }
     case DQ_K_SORT_JREC: {
         const auto& A = dq_arg<DqNetArgs<JRec>>(s_args);
         NetJ::run<true>(A.c, A.g, step.pass, nullptr, (int)tile, sm);
@@ -182,55 +170,59 @@ __device__ void dq_run(const DqStep& step, const unsigned char* s_args, uint32_t
         break;
     }
     // ---- filter + group-by
-    case DQ_K_LI_PACK2:
-    case DQ_K_LI_PACK3: {
-        const auto& A = dq_arg<DqLiPackArgs>(s_args);
-        if (step.kind == DQ_K_LI_PACK2)
-            li_pack_tile<2>(A.c, A.p, A.prm, A.n, A.n_rec, A.lt, A.w[0], A.w[1], A.w[2], A.counts, tile, tmp);
-        else
-            li_pack_tile<3>(A.c, A.p, A.prm, A.n, A.n_rec, A.lt, A.w[0], A.w[1], A.w[2], A.counts, tile, tmp);
+    case DQ_K_SORT_U2: {
+        const auto& A = dq_arg<DqNetArgs<RowU2>>(s_args);
+        NetU2::run<true>(A.c, A.g, step.pass, nullptr, (int)tile, sm);
         break;
     }
-    case DQ_K_SEG_SUMMARY2: {
-        const auto& A = dq_arg<DqSegArgs>(s_args);
-        LiTypes<2>::Seg::tile_summary(A.w, (int)tile, A.aggs, A.runs, A.prm, sm);
+    case DQ_K_LI_KEYS: {
+        const auto& A = dq_arg<DqLiArgs>(s_args);
+        li_keys_body(A.c, A.p, A.n, A.q.h, A.q.ka, A.q.n_pass, A.q.n_ffff, A.out, A.G * (1 + LI_V), A.q.meta, tile, nt,
+                     tmp);
         break;
     }
-    case DQ_K_SEG_SUMMARY3: {
-        const auto& A = dq_arg<DqSegArgs>(s_args);
-        LiTypes<3>::Seg::tile_summary(A.w, (int)tile, A.aggs, A.runs, A.prm, sm);
+    case DQ_K_LI_FOLD: {
+        const auto& A = dq_arg<DqLiArgs>(s_args);
+        li_fold_body(A.q.ka, A.q.h, A.q.N, A.q.kb, tile, nt);
         break;
     }
-    case DQ_K_SEG_CARRIES2: {
-        const auto& A = dq_arg<DqSegArgs>(s_args);
-        LiTypes<2>::Seg::carries(A.aggs, A.runs, A.ntiles, A.carry, A.tail_prefix, A.n_groups, sm);
+    case DQ_K_LI_DISTINCT: {
+        const auto& A = dq_arg<DqLiArgs>(s_args);
+        li_distinct_tile(A.q.kb, A.q.N, A.q.cnt0, A.q.cnt1, tile, reinterpret_cast<uint32_t*>(sm), tmp);
         break;
     }
-    case DQ_K_SEG_CARRIES3: {
-        const auto& A = dq_arg<DqSegArgs>(s_args);
-        LiTypes<3>::Seg::carries(A.aggs, A.runs, A.ntiles, A.carry, A.tail_prefix, A.n_groups, sm);
+    case DQ_K_LI_SLOTS: {
+        const auto& A = dq_arg<DqLiArgs>(s_args);
+        li_slots_tile(A.q.kb, A.q.N, A.q.ntiles, A.q.cnt0, A.q.cnt1, A.q.n_pass, A.q.n_ffff, (int)A.q.nblk, A.G,
+                      A.q.meta, (int)tile, reinterpret_cast<uint32_t*>(sm), *reinterpret_cast<LkSlotShared*>(sx.b));
         break;
     }
-    case DQ_K_SEG_EMIT2: {
-        const auto& A = dq_arg<DqSegArgs>(s_args);
-        LiTypes<2>::Seg::emit(A.w, (int)tile, A.ntiles, A.aggs, A.carry, A.tail_prefix, A.G, A.tile_out, A.prm, sm);
-        break;
-    }
-    case DQ_K_SEG_EMIT3: {
-        const auto& A = dq_arg<DqSegArgs>(s_args);
-        LiTypes<3>::Seg::emit(A.w, (int)tile, A.ntiles, A.aggs, A.carry, A.tail_prefix, A.G, A.tile_out, A.prm, sm);
-        break;
-    }
-    case DQ_K_SEG_FINISH: {
-        const auto& A = dq_arg<DqSegArgs>(s_args);
-        LiTypes<3>::Seg::finish(A.tile_out, A.ntiles, A.G, A.out, (int)tile);
-        if (tile == 0 && threadIdx.x == 0) {
-            A.d_counts[0] = *A.d_rows;
-            A.d_counts[1] = *A.n_groups;
-        }
+    case DQ_K_LI_SUMS: {
+        const auto& A = dq_arg<DqLiArgs>(s_args);
+        const uint32_t blk = tile / (uint32_t)A.chunks;
+        li_sums_body<DQ_LK_SLOTS, DQ_THREADS>(A.c, A.p, A.n, A.G, A.q.meta, A.out, A.d_counts,
+                                              (int)(tile - blk * (uint32_t)A.chunks), blk, nt / (uint32_t)A.chunks,
+                                              reinterpret_cast<int64_t*>(sm));
         break;
     }
     // ---- join + group-by + top-k
+    case DQ_K_JK_PACK: {
+        const auto& A = dq_arg<DqJkArgs>(s_args);
+        jk_pack_body(A.dk, A.dd, A.nd, A.ff, A.fp, A.nf, A.date_hi, A.price_hi, A.k, A.p, A.n_groups, A.n_joined, tile,
+                     nt);
+        break;
+    }
+    case DQ_K_JK_SUMMARY: {
+        const auto& A = dq_arg<DqJkArgs>(s_args);
+        jk_summary_tile(A.k, A.p, A.nd + A.nf, tile, A.aggs, A.runs);
+        break;
+    }
+    case DQ_K_JK_EMIT_TOPK: {
+        const auto& A = dq_arg<DqJkArgs>(s_args);
+        jk_emit_topk_tile(A.k, A.p, A.nd + A.nf, A.ntiles, A.aggs, A.carry, A.cand, A.out0, A.out1, A.n_groups,
+                          A.n_joined, tile, sm);
+        break;
+    }
     case DQ_K_JOIN_PACK: {
         const auto& A = dq_arg<DqJoinPackArgs>(s_args);
         join_pack_body(A.dk, A.dd, A.nd, A.ff, A.fp, A.nf, A.date_hi, A.price_hi, A.n_rec, A.w0, A.w1, tile, nt);

@@ -108,28 +108,7 @@ __global__ void __launch_bounds__(256) k_jk_pack(const int32_t* dk, const int32_
                                                  uint64_t* k, uint32_t* p, uint64_t* n_groups, uint64_t* n_joined)
 {
     VELO_TRACE_KERNEL(velo_site_hash("k_jk_pack"));
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        *n_groups = 0;
-        *n_joined = 0;
-    }
-    const size_t n = nd + nf;
-    for (size_t g = blockIdx.x * (size_t)blockDim.x + threadIdx.x; VELO_GRID_COND(g, n);
-         g += (size_t)gridDim.x * blockDim.x) {
-        uint32_t key;
-        uint64_t u;
-        if (g < nd) {
-            key = (uint32_t)dk[g];
-            u = dd[g] < date_hi ? JK_DIM : JK_DEAD;
-        } else {
-            const size_t j = g - nd;
-            const int64_t pr = fp[j];
-            key = (uint32_t)ff[j];
-            u = pr < price_hi ? ~((uint64_t)pr ^ SIGN64) : JK_DEAD;
-        }
-        VELO_TRACE_AT(TS_ROW_STORE, k + g);
-        k[g] = ((uint64_t)(key ^ 0x80000000u) << 32) | (u >> 32);
-        p[g] = (uint32_t)u;
-    }
+    jk_pack_body(dk, dd, nd, ff, fp, nf, date_hi, price_hi, k, p, n_groups, n_joined, blockIdx.x, gridDim.x);
 }
 
 __global__ void __launch_bounds__(JK_THREADS) k_jk_summary(const uint64_t* k, const uint32_t* p, size_t n,

@@ -386,6 +386,37 @@ __device__ __forceinline__ void jk_values(uint64_t u, int64_t& a, int64_t& b)
     b = fact ? 1 : u == JK_DIM ? (int64_t)1 << 32 : 0;
 }
 
+// pack of the union rows handled by block `blk` of `nblk` (grid stride); clears
+// the counts that the group-by adds to
+__device__ __forceinline__ void jk_pack_body(const int32_t* dk, const int32_t* dd, size_t nd, const int32_t* ff,
+                                             const int64_t* fp, size_t nf, int32_t date_hi, int64_t price_hi,
+                                             uint64_t* k, uint32_t* p, uint64_t* n_groups, uint64_t* n_joined,
+                                             size_t blk, size_t nblk)
+{
+    if (blk == 0 && threadIdx.x == 0) {
+        *n_groups = 0;
+        *n_joined = 0;
+    }
+    const size_t n = nd + nf;
+    for (size_t g = blk * (size_t)blockDim.x + threadIdx.x; VELO_GRID_COND(g, n);
+         g += nblk * blockDim.x) {
+        uint32_t key;
+        uint64_t u;
+        if (g < nd) {
+            key = (uint32_t)dk[g];
+            u = dd[g] < date_hi ? JK_DIM : JK_DEAD;
+        } else {
+            const size_t j = g - nd;
+            const int64_t pr = fp[j];
+            key = (uint32_t)ff[j];
+            u = pr < price_hi ? ~((uint64_t)pr ^ SIGN64) : JK_DEAD;
+        }
+        VELO_TRACE_AT(TS_ROW_STORE, k + g);
+        k[g] = ((uint64_t)(key ^ 0x80000000u) << 32) | (u >> 32);
+        p[g] = (uint32_t)u;
+    }
+}
+
 // tile `blk`: first and last key, the last key's sums inside the tile
 __device__ __forceinline__ void jk_summary_tile(const uint64_t* k, const uint32_t* p, size_t n, size_t blk,
                                                 SegTileAgg* aggs, int64_t* runs)

@@ -6,7 +6,7 @@
 using JoinRec = velo::RowRec<2, 1, false, velo::KEY_FULL>;
 VELO_INSTANTIATE_NET(JoinRec, 8, 4)
 
-VELO_INSTANTIATE_NET(velo::RowU2, 9, 5)
+VELO_INSTANTIATE_NET(velo::RowU2, 8, 5)
 
 // generic group-by records (velo_ogroupby): key word plus 0 or 2 sum words
 using GbRec1 = velo::RowRec<1, 1, false, velo::KEY_FULL>;

@@ -1,5 +1,5 @@
-// Oblivious segmented aggregation over key-sorted records with a small public
-// output bound G (group-by tail of the filter + group-by pipeline).
+// Oblivious segmented aggregation over key-sorted records (the group-by steps of
+// the generic GROUP BY and of the join's record form).
 //
 // The algorithm is the segmented-sum group-by of the reference's oblivious
 // aggregation (obliviator/operator_2/enclave/scalable_oblivious_join.c:221-262:
@@ -9,12 +9,8 @@
 //      complete groups ending inside the tile
 //   B  one CTA: carries between tiles (segmented scan over tiles) and the
 //      exclusive group-count prefix
-//   C  per tile: in-tile segmented scan + carry; the last row of each valid
-//      group carries the group total; the group with rank r (its position in
-//      key order) is accumulated into output slot r by masked sums over all
-//      G slots -- every row touches every slot, so addresses never depend on
-//      the data
-//   D  one CTA: slot-wise sum of the per-tile slot vectors.
+//   C  per tile: in-tile segmented scan + carry; every row writes a group
+//      record, valid on the last row of each valid group
 // Rows whose "valid" flag is clear form their own key runs (the flag is part
 // of the key) and never produce output.
 #pragma once
@@ -121,27 +117,6 @@ __device__ __forceinline__ int64_t warp_sum_i64(int64_t x)
     return x;
 }
 
-// Warp reduce-scatter of 16 int64 values a lane: four halving steps over
-// lane bits 4..1 (each lane keeps the half its lane bit selects and adds the
-// partner's copy of it) and one add across lane bit 0; afterwards a[0] of
-// lane L is the warp sum of value L >> 1.
-__device__ __forceinline__ void warp_reduce_scatter16(int64_t (&a)[16], int lane)
-{
-#pragma unroll
-    for (int step = 0; step < 4; step++) {
-        const int o = 16 >> step;
-        const int h = 8 >> step; // current length / 2
-        const bool up = (lane & o) != 0;
-#pragma unroll
-        for (int k = 0; k < h; k++) {
-            const int64_t keep = up ? a[h + k] : a[k];
-            const int64_t send = up ? a[k] : a[h + k];
-            a[k] = keep + __shfl_xor_sync(0xffffffffu, send, o);
-        }
-    }
-    a[0] += __shfl_xor_sync(0xffffffffu, a[0], 1);
-}
-
 // Group records of a 64-bit key (Agg::FLAG_IN_COUNT = true): o0 = the whole
 // out_bits(key), o1 = [63] not the last row of a valid group | the first value,
 // a count; otherwise the flag shares word 0 with a key of at most 63 bits.
@@ -175,7 +150,6 @@ struct SegAgg {
     // only the W input words (smaller footprint, more CTAs per SM)
     static constexpr size_t SMEM = (size_t)SEG_TS_PAD * TW * 8 + (size_t)V * SEG_THREADS * 8 + SEG_THREADS * 4 + 256;
     static constexpr size_t SMEM_IN = (size_t)SEG_TS_PAD * W * 8 + (size_t)V * SEG_THREADS * 8 + SEG_THREADS * 4 + 256;
-    static_assert((size_t)SEG_MAX_G * (1 + V) * 8 * 8 <= (size_t)SEG_TS_PAD * W * 8, "emit reduction fits the tile area");
 
     // stage the tile's records in smem (coalesced), then thread t owns rows
     // [t*RPT, t*RPT + RPT)
@@ -411,161 +385,7 @@ struct SegAgg {
             *n_groups = cnt_prev;
     }
 
-    // pass C
-    __device__ static void emit(uint64_t* const* words, int tile, int ntiles, const SegTileAgg* aggs,
-                                const int64_t* carry_in, const uint32_t* tail_prefix, int G, int64_t* tile_out,
-                                const Params& prm, char* smem)
-    {
-        uint64_t* sw = reinterpret_cast<uint64_t*>(smem);
-        int64_t* svals = reinterpret_cast<int64_t*>(smem + (size_t)SEG_TS_PAD * W * 8);
-        uint32_t* sflags = reinterpret_cast<uint32_t*>(smem + (size_t)SEG_TS_PAD * W * 8 + (size_t)V * SEG_THREADS * 8);
-        const size_t base = (size_t)tile * SEG_TS;
-        load_tile(words, base, sw);
-        const uint64_t next_head = (tile + 1 < ntiles) ? aggs[tile + 1].head_key : ~0ull;
-        const bool last_tile = (tile + 1 >= ntiles);
-        const uint64_t head_key = aggs[tile].head_key;
-        const int r0 = threadIdx.x * SEG_RPT;
-
-        // thread-local inclusive segmented scan of my rows
-        int64_t pref[SEG_RPT][V];
-        uint64_t keys[SEG_RPT];
-        bool tail[SEG_RPT];
-        bool start_flag = false; // a run starts inside my rows (at row r0 or later)
-        {
-            uint64_t wprev[W];
-            row(sw, r0 > 0 ? r0 - 1 : 0, wprev);
-            uint64_t prev_key = Agg::key(wprev);
-            int64_t run[V];
-#pragma unroll
-            for (int i = 0; i < V; i++)
-                run[i] = 0;
-#pragma unroll
-            for (int r = 0; r < SEG_RPT; r++) {
-                uint64_t w[W];
-                row(sw, r0 + r, w);
-                const uint64_t k = Agg::key(w);
-                int64_t v[V];
-                Agg::values(w, v, prm);
-                const bool starts = (r0 + r == 0) ? true : (k != prev_key);
-                start_flag = start_flag | starts;
-#pragma unroll
-                for (int i = 0; i < V; i++)
-                    run[i] = (starts ? 0 : run[i]) + v[i];
-#pragma unroll
-                for (int i = 0; i < V; i++)
-                    pref[r][i] = run[i];
-                keys[r] = k;
-                prev_key = k;
-                uint64_t wn[W];
-                const int nxt = r0 + r + 1 < SEG_TS ? r0 + r + 1 : SEG_TS - 1;
-                row(sw, nxt, wn);
-                const uint64_t kn = (r0 + r + 1 < SEG_TS) ? Agg::key(wn) : next_head;
-                const bool ends = (r0 + r + 1 < SEG_TS || !last_tile) ? (k != kn) : true;
-                tail[r] = ends & Agg::valid(w);
-            }
-        }
-        // exclusive block segmented scan of thread aggregates: my carry-in is
-        // the inclusive result of thread-1 unless a run starts at my row r0
-        int64_t agg[V];
-#pragma unroll
-        for (int i = 0; i < V; i++)
-            agg[i] = pref[SEG_RPT - 1][i];
-        bool fl = start_flag;
-        block_seg_scan<V>(fl, agg, svals, sflags);
-#pragma unroll
-        for (int i = 0; i < V; i++)
-            svals[i * SEG_THREADS + threadIdx.x] = agg[i];
-        __syncthreads();
-        int64_t cin[V];
-#pragma unroll
-        for (int i = 0; i < V; i++)
-            cin[i] = (threadIdx.x > 0) ? svals[i * SEG_THREADS + threadIdx.x - 1] : 0;
-        // the tile-level carry applies to rows of the tile's first run
-        int64_t tc[V];
-#pragma unroll
-        for (int i = 0; i < V; i++)
-            tc[i] = carry_in[(size_t)tile * V + i];
-        // rank of my first tail: tail prefix of the tile + tails of threads before me
-        uint32_t my_tails = 0;
-#pragma unroll
-        for (int r = 0; r < SEG_RPT; r++)
-            my_tails += tail[r] ? 1u : 0u;
-        uint32_t tails_total;
-        const uint32_t before = block_exclusive_scan(my_tails, reinterpret_cast<uint32_t*>(svals), &tails_total);
-        const uint32_t rank0 = tail_prefix[tile] + before;
-
-        // my leading rows continue the run open at the end of thread t-1
-        // unless a new run starts exactly at my first row
-        bool lead = (r0 > 0);
-        if (r0 > 0) {
-            uint64_t wp[W];
-            row(sw, r0 - 1, wp);
-            lead = (Agg::key(wp) == keys[0]);
-        }
-        // segment totals up to each row: my prefix, the in-tile carry of the
-        // preceding threads, and the cross-tile carry of the tile's first run
-#pragma unroll
-        for (int r = 0; r < SEG_RPT; r++) {
-            if (r > 0)
-                lead = lead & (keys[r] == keys[r - 1]);
-            const bool first_run_of_tile = (keys[r] == head_key);
-#pragma unroll
-            for (int i = 0; i < V; i++)
-                pref[r][i] += (lead ? cin[i] : 0) + (first_run_of_tile ? tc[i] : 0);
-        }
-        // output slot j receives (key, totals) of the tail whose rank is j;
-        // every row is folded into every slot with a mask
-        __syncthreads();
-        int64_t* red = reinterpret_cast<int64_t*>(smem); // reuse the tile area
-        // slots in chunks of 2: every lane folds its rows into 2 x 8 values
-        // (slot, value; values past 1+V stay zero), then a warp reduce-scatter
-        // leaves lanes 2L and 2L + 1 with the warp sum of value L (chunks of
-        // 4 slots kept 32 sums a lane live: 102 registers, two CTAs an SM)
-        static_assert(1 + V <= 8, "a slot's key and values fit 8 words");
-        constexpr int SLOTS = 2;
-        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-        for (int j0 = 0; j0 < G; j0 += SLOTS) {
-            int64_t acc[8 * SLOTS];
-#pragma unroll
-            for (int q = 0; q < 8 * SLOTS; q++)
-                acc[q] = 0;
-            // the ranks of a thread's tails are distinct, so each slot takes
-            // at most one of its rows: a select, not an add (the block sum
-            // below adds the threads' slots, all but one zero)
-            uint32_t rank = rank0;
-#pragma unroll
-            for (int r = 0; r < SEG_RPT; r++) {
-                const int64_t kv = Agg::out_key_from(keys[r]);
-#pragma unroll
-                for (int jj = 0; jj < SLOTS; jj++) {
-                    const bool hit = tail[r] & (rank == (uint32_t)(j0 + jj));
-                    acc[jj * 8] = hit ? kv : acc[jj * 8];
-#pragma unroll
-                    for (int i = 0; i < V; i++)
-                        acc[jj * 8 + 1 + i] = hit ? pref[r][i] : acc[jj * 8 + 1 + i];
-                }
-                rank += tail[r] ? 1u : 0u;
-            }
-            warp_reduce_scatter16(acc, lane);
-            if ((lane & 1) == 0)
-                red[(lane >> 1) * 8 + warp] = acc[0];
-            __syncthreads();
-            const int gn = G - j0 < SLOTS ? G - j0 : SLOTS;
-            for (int q = threadIdx.x; q < gn * (1 + V); q += SEG_THREADS) {
-                const int jj = q / (1 + V), i = q - jj * (1 + V);
-                const size_t o = (size_t)tile * G * (1 + V) + (size_t)(j0 + jj) * (1 + V) + i;
-                VELO_TRACE_AT(TS_SEG_OUT, tile_out + o);
-                int64_t sum = 0;
-#pragma unroll
-                for (int w = 0; w < SEG_THREADS / 32; w++)
-                    sum += red[(jj * 8 + i) * 8 + w];
-                tile_out[o] = sum;
-            }
-            __syncthreads();
-        }
-    }
-
-    // pass C for a large output bound: every row writes a group record
+    // pass C: every row writes a group record
     // (o0 = [63] not the last row of a valid group | [31:0] Agg::out_bits,
     // o1.. = the group's sums, valid only on the group's last row); an
     // ORCompact of the records then yields the groups in key order.
@@ -695,29 +515,6 @@ struct SegAgg {
                     | (FC && i == 0 ? flag : 0ull);
         }
         __syncthreads();
-    }
-
-    // pass D: out[q] = sum over tiles of tile_out[tile][q]; one CTA of
-    // SEG_THREADS threads per output word q (0 .. G*(1+V)-1)
-    __device__ static void finish(const int64_t* tile_out, int ntiles, int G, int64_t* out, int q)
-    {
-        __shared__ int64_t part[SEG_THREADS / 32];
-        const int QN = G * (1 + V);
-        int64_t sum = 0;
-        for (int t = threadIdx.x; t < ntiles; t += SEG_THREADS) {
-            VELO_TRACE_AT(TS_SEG_OUT, tile_out + (size_t)t * QN + q);
-            sum += tile_out[(size_t)t * QN + q];
-        }
-        sum = warp_sum_i64(sum);
-        if ((threadIdx.x & 31) == 0)
-            part[threadIdx.x >> 5] = sum;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            int64_t s = 0;
-            for (int w = 0; w < SEG_THREADS / 32; w++)
-                s += part[w];
-            out[q] = s;
-        }
     }
 };
 
