@@ -60,7 +60,7 @@ METRIC = "obliv sort & join Mrows/s (frac of HBM peak); p50/p99 latency served v
 # DRAM bytes (read + write) per launch of the dominant kernel from one ncu
 # capture of the same pipeline (the mean over its sort passes), or None when
 # no capture of that launch exists.
-TRAFFIC = {"groupby": 210.1e6, "sort": 12.65e6, "join": 210.6e6, "batch": None}
+TRAFFIC = {"groupby": None, "sort": 12.65e6, "join": None, "batch": None}
 
 # warm-up runs at least this long (seconds) so that the clock samples taken
 # from the end of the warm-up through the timed steps show the GPU under load
@@ -79,9 +79,15 @@ def hbm_peak():
 # pass-count models
 # --------------------------------------------------------------------------
 
-# levels fused per global pass: plain (u64, u32) sorts keep 32 contiguous rows
-# per warp (lmax = lt - 5); the pipelines' 8-byte records use 16 (lt - 4)
+# levels fused per global pass: 16 contiguous rows a segment (lmax = lt - 4)
 PIPE_LMAX = 8
+
+
+def sorted_rows(n: int) -> dict:
+    """Rows the passes of a sort of n rows work on, by log2 of the padded size:
+    whole 4096-row tiles, the padding past the last one left out."""
+    return {max(0, (n - 1).bit_length()): -(-n // 4096) * 4096}
+
 
 
 def sort_passes(logn: int, lt: int, lmax: int) -> int:
@@ -187,10 +193,11 @@ class JoinTopK:
         self.counts_host = torch.empty(2, dtype=torch.int64).pin_memory()
         self.in_bytes = sum(v.numel() * v.element_size() for v in self.pinned.values())
         self.np_rows = 1 << int(np.ceil(np.log2(self.n)))
-        self.rec_bytes = 16
-        self.flush_l2 = False  # inputs (60 MB) plus union records (268 MB) exceed the 126 MB L2
-        self.kernel = ("k_sort_pass<RowRec<2,1,false,KEY_FULL>,8,4,PK,2> (union sort: 2^23 two-word records, "
-                       "4096-row tiles, two CTAs per SM)")
+        self.rec_bytes = 12
+        self.pass_rows = sorted_rows(self.n)
+        self.flush_l2 = False  # inputs (84 MB) plus union rows (90 MB) exceed the 126 MB L2
+        self.kernel = ("k_sort_pass<RowKP,8,4,PK,3> (union sort: 7.5 M 12-byte rows, 4096-row tiles, three CTAs "
+                       "per SM)")
 
     def step(self):
         self.capi.join_groupby_topk(self.dev, self.pred, self.k, scratch=self.scratch, out=self.out,
@@ -227,14 +234,13 @@ class JoinTopK:
         return self.out.numel() * 8 + self.counts.numel() * 8
 
     def launches(self):
-        u = int(np.log2(self.np_rows))
-        top = int(np.log2(1 << int(np.ceil(np.log2(self.nd)))))
-        # pack, union sort, fill, count+scan, compaction, aggregation, count+scan,
-        # group compaction, top-k pack, tile pass, candidates, candidate sort, out
-        cand = int(np.log2((1 << max(0, top - 12)) * 16)) if top > 12 else 0
-        topk = (1 + 1 + sort_passes(cand, 12, PIPE_LMAX)) if top > 12 else sort_passes(top, 12, PIPE_LMAX)
-        return (1 + sort_passes(u, 12, PIPE_LMAX) + 3 + 2 + compact_passes(u, 12, PIPE_LMAX) + 3 + 2
-                + compact_passes(u, 12, PIPE_LMAX) + 1 + topk + 1)
+        # pack, union sort, summary, carries, emit + first top-k round, rounds, out
+        tiles = 1 << max(0, (-(-self.n // 2048) - 1).bit_length())
+        rounds, c = 0, tiles * 16
+        while c > 16:
+            c = c // min(c, 4096) * 16
+            rounds += 1
+        return 1 + sort_passes(int(np.log2(self.np_rows)), 12, PIPE_LMAX) + 3 + rounds + 1
 
     def rdm_bytes(self):
         """The algorithmic-bytes model of the join pipeline: union sort
@@ -303,10 +309,10 @@ class GroupBy:
         self.counts_host = torch.empty(2, dtype=torch.int64).pin_memory()
         self.in_bytes = sum(v.numel() * v.element_size() for v in self.pinned.values())
         self.np_rows = 1 << int(np.ceil(np.log2(self.n)))
-        self.rec_bytes = 16  # 2-word records (the predicate's bands fit the packed layout)
-        self.flush_l2 = False  # inputs (156 MB) and records (134 MB) exceed the 126 MB L2
-        self.kernel = ("k_sort_pass<RowRec<2,1,false,KEY_HI32>,8,4,PK,3> (sort stage: 2^23 two-word records, "
-                       "4096-row tiles, three CTAs per SM)")
+        self.rec_bytes = 4  # a pair of 16-bit group keys
+        self.pass_rows = sorted_rows((self.n + 1) // 2)
+        self.flush_l2 = False  # inputs (156 MB) exceed the 126 MB L2
+        self.kernel = "k_sort_pass<RowU2,8,5,PK> (sort stage: 3 M pairs of 16-bit keys, 8192-word tiles)"
 
     def step(self):
         self.capi.filter_groupby(self.dev, self.n, self.pred, self.G, scratch=self.scratch, out=self.out,
@@ -342,8 +348,10 @@ class GroupBy:
         return self.out.numel() * 8 + self.counts.numel() * 8
 
     def launches(self):
-        logn = int(np.log2(self.np_rows))
-        return 2 + compact_passes(logn, 12, PIPE_LMAX) + sort_passes(logn, 12, PIPE_LMAX) + 4
+        # keys, sort, fold, the last merge, distinct, slots, sums
+        logn = int(np.log2(self.np_rows)) - 1
+        merge = -(-(logn - 13) // 9) + 1
+        return 1 + sort_passes(logn, 13, 9) + 1 + merge + 2 + 1
 
     def rdm_bytes(self):
         npr = self.np_rows
@@ -422,7 +430,7 @@ class SortKP:
         return self.n * 12
 
     def launches(self):
-        return sort_passes(int(np.log2(self.n)), 12, 7)
+        return sort_passes(int(np.log2(self.n)), 12, 8)
 
     def rdm_bytes(self):
         return 2 * self.n * 12 * rdm_psort(self.n)
@@ -512,7 +520,12 @@ class Batched:
         return 8 * sum(1 for it in self.items if "count" in it)
 
     def launches(self):
-        return 1  # one persistent kernel per step (plus one counter memset)
+        # one persistent kernel per step (plus one counter memset); with the
+        # default tile the sorts of more than 2^20 rows run their own passes
+        big = [it["n"] for it in self.items if it["kind"] == "sort" and it["n"] > 1 << 20]
+        if tuple(self.tune) != (12, 256):
+            big = []
+        return 1 + sum(sort_passes(int(np.ceil(np.log2(n))), 12, 8) for n in big)
 
     def rdm_bytes(self):
         tot = 0
@@ -533,7 +546,8 @@ class Batched:
             lt = self.tune[0]
             lmax = min(8, lt - 5)
             if it["kind"] == "sort":
-                tot += 2 * npr * 12 * sort_passes(int(np.log2(npr)), lt, lmax)
+                rows = min(npr, -(-it["n"] // (1 << lt)) * (1 << lt))
+                tot += 2 * rows * 12 * sort_passes(int(np.log2(npr)), lt, min(8, lt - 4))
             else:
                 tot += 2 * npr * 13 * compact_passes(int(np.log2(npr)), lt, lmax) + npr * 5
         return tot
@@ -592,11 +606,16 @@ def warm(torch, fn, warmup, min_s=SOAK_S):
 PASS_KINDS = ("tile_sort", "merge", "global", "compact_tile", "compact_global")
 
 
-def pass_roofline(torch, capi, run, peak, reps=3, reset=None):
+def pass_roofline(torch, capi, run, peak, reps=3, reset=None, pass_rows=None):
     """Every network pass of `run` timed on its own (the library's pass timer:
     CUDA events around each pass, on the pass's stream) and grouped by pass
-    kind.  Algorithmic bytes of a pass: every row read and written once,
-    2 x rows x row bytes."""
+    kind.  Algorithmic bytes of a pass: every row it works on read and written
+    once, 2 x rows x row bytes (pass_rows: rows by log2 of the padded size where
+    the sorts leave padding out)."""
+    def bytes_of(kind, lg, rb):
+        trimmed = (pass_rows or {}).get(lg) if kind in ("tile_sort", "merge", "global") else None
+        return 2 * (trimmed or 1 << lg) * rb
+
     rows = []
     for _ in range(reps):
         if reset is not None:
@@ -611,7 +630,7 @@ def pass_roofline(torch, capi, run, peak, reps=3, reset=None):
             capi.set_pass_timing(False)
     out = {}
     for kind in PASS_KINDS:
-        xs = [(2 * (1 << lg) * rb, ms) for (k, lg, rb, ms) in rows if k == kind and ms > 0]
+        xs = [(bytes_of(k, lg, rb), ms) for (k, lg, rb, ms) in rows if k == kind and ms > 0]
         if not xs:
             continue
         byt = sum(b for b, _ in xs)
@@ -625,7 +644,7 @@ def pass_roofline(torch, capi, run, peak, reps=3, reset=None):
     dom = None
     if sorts:
         lg_max = max(lg for lg, _, _ in sorts)
-        xs = [(2 * (1 << lg) * rb, ms) for lg, rb, ms in sorts if lg == lg_max]
+        xs = [(bytes_of("merge", lg, rb), ms) for lg, rb, ms in sorts if lg == lg_max]
         dom = {"launches_per_step": len(xs) // reps, "avg_launch_us": sum(m for _, m in xs) / len(xs) * 1e3,
                "algorithmic_bytes_per_launch": xs[0][0], "log2_rows": lg_max}
     return out, dom
@@ -763,7 +782,7 @@ def roofline_of(torch, capi, wl, peak, peak_kind):
 
         def run():
             wl.capi.osort_kp(wl.k, wl.p, wl.n)
-    kinds, dom = pass_roofline(torch, capi, run, peak, reset=reset)
+    kinds, dom = pass_roofline(torch, capi, run, peak, reset=reset, pass_rows=getattr(wl, "pass_rows", None))
     if dom is None:
         return None
     achieved = dom["algorithmic_bytes_per_launch"] / (dom["avg_launch_us"] / 1e6) / 1e9

@@ -430,8 +430,10 @@ typedef struct velo_batch velo_batch;
  * Allocates the batch's device plan (cudaMalloc) here, never at launch. */
 velo_status velo_batch_create(const velo_batch_item* items, size_t n_items, const velo_tune* tune,
                               velo_batch** out);
-/* Enqueues the whole batch on `stream`: a counter reset and ONE kernel
- * launch, so the call can be captured into a CUDA graph and replayed. */
+/* Enqueues the whole batch on `stream`: a counter reset and ONE persistent
+ * kernel launch, then -- with the default tile -- the passes of the sorts of
+ * more than 2^20 rows, which fill the GPU by themselves; the call can be
+ * captured into a CUDA graph and replayed. */
 velo_status velo_batch_launch(velo_batch* batch, void* stream);
 /* Synchronises `stream` and returns VELO_ETIMEDOUT if a device-side wait of
  * the last launch ran out of time (the kernel never spins unbounded). */

@@ -20,6 +20,22 @@ namespace velo {
     X(9, 4)                                                                                                            \
     X(10, 3)
 
+// Sorts of 2^21 padded rows and more (n above 2^20) run as the passes of
+// velo_osort_kp after the persistent launch, when the batch has the default
+// tile: they fill the GPU by themselves, and the pass kernels (compile-time
+// layouts, three CTAs an SM) are faster there than the scheduler's one kernel.
+// The sorts of the 512-instance mix, ms by the scheduler / by pass kernels:
+// above 2^20 rows 23.5 / 18.3, from 2^19 to 2^20 2.7 / 3.6; compactions above
+// 2^20 rows 4.1 / 4.1.  Such a sort keeps one empty item in the plan (for
+// velo_batch_inject_unmet_wait).
+constexpr int SCHED_BIG_LOGN = 21;
+
+struct SchedBig {
+    RowKP::Cols c;
+    size_t n;
+    int logN;
+};
+
 template <int LOG_NT, int LOG_E>
 velo_status sched_launch(const SchedArgs& a, int sms, cudaStream_t st);
 
@@ -29,6 +45,7 @@ struct velo_batch {
     int log_nt = 9, log_e = 4;
     std::vector<velo::SchedStep> steps;
     std::vector<velo::SchedInst> insts;
+    std::vector<velo::SchedBig> big;    // sorts run by pass kernels
     std::vector<uint64_t*> zero_counts; // d_count of empty compactions
     void* dmem = nullptr;               // steps | insts | done | next | status | compaction scratch
     velo::SchedStep* d_steps = nullptr;
@@ -80,7 +97,11 @@ static velo_status batch_plan(velo_batch* b, const velo_batch_item* items, size_
         const int ntiles = in.logN > lt ? 1 << (in.logN - lt) : 1;
         in.ntiles = ntiles;
         std::vector<NetPass> passes;
-        if (it.kind == VELO_ITEM_SORT_KP) {
+        if (it.kind == VELO_ITEM_SORT_KP && in.logN >= SCHED_BIG_LOGN && b->log_nt == 8 && b->log_e == 4) {
+            b->big.push_back(SchedBig { { it.d_keys, it.d_payload }, it.n, in.logN });
+            per[i].push_back({ STEP_NOP, NetPass {} });
+            tiles[i].push_back(1);
+        } else if (it.kind == VELO_ITEM_SORT_KP) {
             if (np > 1)
                 plan_sort(in.logN, lt, lmax_sort, passes);
             const NetGeom g = NetGeom::trimmed(it.n, in.logN, lt, 1);
@@ -233,12 +254,17 @@ extern "C" velo_status velo_batch_launch(velo_batch* b, void* stream)
     a.total_items = b->total_items;
     a.timeout_ns = b->timeout_ns;
     a.nsteps = (int)b->steps.size();
+    velo_status rc = VELO_ESTATE;
 #define X(x, y)                                                                                                        \
     if (b->log_nt == x && b->log_e == y)                                                                               \
-        return sched_launch<x, y>(a, b->sms, st);
+        rc = sched_launch<x, y>(a, b->sms, st);
     VELO_FOR_SCHED_TUNES(X)
 #undef X
-    return einval("velo_batch_launch: bad configuration");
+    if (rc == VELO_ESTATE)
+        return einval("velo_batch_launch: bad configuration");
+    for (size_t i = 0; rc == VELO_OK && i < b->big.size(); i++)
+        rc = sort_kp_rows(b->big[i].c, b->big[i].n, b->big[i].logN, 1, st);
+    return rc;
 }
 
 extern "C" velo_status velo_batch_status(velo_batch* b, void* stream)

@@ -29,6 +29,7 @@ enum StepKind : uint32_t {
     STEP_COMPACT_COUNT = 2, // per-tile mark counts of a compaction
     STEP_COMPACT_SCAN = 3,  // exclusive scan of the tile counts (one tile)
     STEP_COMPACT_PASS = 4,  // ORCompact pass
+    STEP_NOP = 5,           // nothing (the instance runs outside the persistent launch)
 };
 
 struct SchedStep {
