@@ -420,7 +420,7 @@ extern "C" velo_status velo_ojoin_mn(const void* d_build_keys, const uint8_t* d_
     Rec3K2::Cols uc;
     for (int i = 0; i < 3; i++) {
         uc.w[i] = w[i];
-        uc.pad[i] = ~0ull;
+        uc.pad[i] = i < 2 ? ~0ull : 0ull; // as k_mn_pack pads
     }
     uc.mask[0] = ~0ull;
     uc.mask[1] = ~0ull;
@@ -429,7 +429,8 @@ extern "C" velo_status velo_ojoin_mn(const void* d_build_keys, const uint8_t* d_
     uc.mark_inv = 0;
     std::vector<NetPass> passes;
     plan_sort(logU, OP_LT, OP_LMAX, passes);
-    velo_status rc = launch_net12<Rec3K2>(uc, NetGeom { U, logU, 0 }, passes, nullptr, st);
+    velo_status rc = launch_net12<Rec3K2>(uc, NetGeom::trimmed(build_n + probe_n, logU, OP_LT, 0), passes, nullptr,
+                                          st); // every row has its row id in the key
     if (rc != VELO_OK)
         return rc;
 
@@ -864,7 +865,9 @@ extern "C" velo_status velo_ohash_join(const void* d_build_keys, const uint8_t* 
     c.mark_inv = 1; // kept rows (bit 63 clear) are marked
     std::vector<NetPass> passes;
     plan_sort(logR, OP_LT, OP_LMAX, passes);
-    velo_status rc = launch_net12<HjRec>(c, NetGeom { g.rows, logR, 0 }, passes, nullptr, st);
+    // every row's bin, side and row or slot number are its own
+    velo_status rc =
+        launch_net12<HjRec>(c, NetGeom::trimmed(build_n + probe_n + g.slots, logR, OP_LT, 0), passes, nullptr, st);
     if (rc != VELO_OK)
         return rc;
     const int nt = (int)(g.rows / MN_TS);
