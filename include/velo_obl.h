@@ -59,7 +59,8 @@ typedef enum velo_type {
 /* Tile configuration of the network kernels: tile = 2^tile_log2 rows per CTA
  * (11..13), threads = 256/512/1024.  NULL = defaults (velo_osort_kp and
  * velo_ocompact_kpm: 2048-row tiles of 256 threads up to 2^18 rows, 4096-row
- * tiles of 256 threads above). */
+ * tiles of 256 threads above; sorts of up to 512 or 1024 rows take a tile of
+ * that many). */
 typedef struct velo_tune {
     uint32_t tile_log2;
     uint32_t threads;

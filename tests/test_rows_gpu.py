@@ -13,9 +13,10 @@ pytestmark = pytest.mark.gpu
 INTEGER, BIGINT, DOUBLE, DATE, SMALLINT = 4, 5, 7, 10, 3
 
 
-# ---- trimmed sorts: one row around a tile, around 2^18 (the smaller tile's
-# ---- last size), in the last block of several phases, and in the three-CTA form
-@pytest.mark.parametrize("n", [2049, 4097, 6144, 6145, 12_289, (1 << 17) + 1, (1 << 18) - 2048, (1 << 18) + 1,
+# ---- trimmed sorts: one row around a tile (512 and 1024 rows for small sorts),
+# ---- around 2^18 (the smaller tile's last size), in the last block of several
+# ---- phases, and in the three-CTA form
+@pytest.mark.parametrize("n", [3, 511, 512, 513, 1023, 1024, 1025, 2049, 4097, 6144, 6145, 12_289, (1 << 17) + 1, (1 << 18) - 2048, (1 << 18) + 1,
                                3 << 17, (3 << 17) + 4096, (1 << 19) + 4095, (1 << 20) + 1, 1_572_865, (1 << 21) + 5])
 def test_trimmed_sort_and_padding(cuda, n):
     g = torch.Generator(device="cuda")

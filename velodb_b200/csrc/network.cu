@@ -42,6 +42,15 @@ static velo_status sort_dispatch(const typename R::Cols& c, size_t n, int logN, 
     return einval("unsupported tile configuration");
 }
 
+// Levels a fused global ORCompact pass of (key, payload, mark) rows takes: one
+// more than keeps 32 rows a segment where that makes it a single pass (2^20
+// rows 43.3 -> 37.1 us), else not (2^23 rows: 8 + 3 levels 216.7, 7 + 4 213.2)
+static int kpm_lmax(int logN, int lt)
+{
+    const int l = lt - 5 < 8 ? lt - 5 : 8;
+    return logN - lt == l + 1 ? l + 1 : l;
+}
+
 template <class R>
 static velo_status compact_dispatch(const typename R::Cols& c, size_t n, int logN, int log_nt, int log_e,
                                     uint32_t* counts, uint32_t* prefix, uint64_t* d_count, cudaStream_t st)
@@ -54,7 +63,7 @@ static velo_status compact_dispatch(const typename R::Cols& c, size_t n, int log
         velo_status rc = launch_count_scan<R>(c, n, logN, lt, counts, prefix, d_count, st);                            \
         if (rc != VELO_OK)                                                                                             \
             return rc;                                                                                                 \
-        plan_compact(logN, lt, lt - 5 < 8 ? lt - 5 : 8, passes);                                                       \
+        plan_compact(logN, lt, kpm_lmax(logN, lt), passes);                                                            \
         return launch_net<R, a, b>(c, g, passes, prefix, st);                                                          \
     }
     VELO_FOR_TUNES_COMPACT(X)
@@ -243,8 +252,22 @@ extern "C" const char* velo_last_error_text(void)
 constexpr int DEFAULT_SMALL_LOGN = 18;
 static int default_log_e(int logN) { return logN <= DEFAULT_SMALL_LOGN ? 3 : 4; }
 
+// Sorts of up to 1024 padded rows are one CTA whose time is its shared-memory
+// traffic and its levels' latency, so the tile holds no more rows than it has
+// to: 512 rows of 64 threads, 1024 of 128 (n = 300: 13.6 -> 10.6 us, n = 1000:
+// 16.4 -> 13.4 us a call against 2048 rows of 256; 256 threads x 4 rows 14.4).
+static velo_status sort_small(const RowKP::Cols& c, size_t n, int logN, cudaStream_t st)
+{
+    std::vector<NetPass> passes;
+    plan_sort(logN, 10, 6, passes); // the tile pass alone
+    return logN <= 9 ? launch_net<RowKP, 6, 3>(c, NetGeom(n, logN), passes, nullptr, st)
+                     : launch_net<RowKP, 7, 3>(c, NetGeom(n, logN), passes, nullptr, st);
+}
+
 velo_status velo::sort_kp_rows(const RowKP::Cols& c, size_t n, int logN, int fill, cudaStream_t st)
 {
+    if (logN <= 10)
+        return sort_small(c, n, logN, st);
     return sort_dispatch<RowKP>(c, n, logN, 8, default_log_e(logN), fill, st);
 }
 
@@ -268,6 +291,8 @@ extern "C" velo_status velo_osort_kp(uint64_t* d_keys, uint32_t* d_payload, size
     if (np == 1)
         return VELO_OK;
     RowKP::Cols c { d_keys, d_payload };
+    if (logN <= 10 && !(tune && tune->tile_log2))
+        return sort_small(c, n, logN, (cudaStream_t)stream);
     return sort_dispatch<RowKP>(c, n, logN, log_nt, log_e, 1, (cudaStream_t)stream);
 }
 
