@@ -727,7 +727,15 @@ __device__ bool dq_complete(const DqParams& a, DqShared& S)
     return false;
 }
 
-__global__ void __launch_bounds__(DQ_THREADS, 2) k_dq(DqParams a)
+// CTAs an SM; the instrumented build keeps the pass bodies as functions of up
+// to 235 registers, which two CTAs an SM have no room for
+#ifdef VELO_TRACE
+constexpr int DQ_CTAS = 1;
+#else
+constexpr int DQ_CTAS = 2;
+#endif
+
+__global__ void __launch_bounds__(DQ_THREADS, DQ_CTAS) k_dq(DqParams a)
 {
     extern __shared__ __align__(16) char sm[];
     __shared__ __align__(16) unsigned char s_args[DQ_STEP_ARG_MAX];
