@@ -97,10 +97,6 @@ def sort_passes(logn: int, lt: int, lmax: int) -> int:
     return p
 
 
-def compact_passes(logn: int, lt: int, lmax: int) -> int:
-    return 1 + (-(-(max(0, logn - lt)) // lmax) if logn > lt else 0)
-
-
 def rdm_psort(np_rows: int) -> int:
     """Pass count of the algorithmic-bytes model: T = 2^13, L = 8."""
     m = max(0, int(np.log2(np_rows)) - 13)
@@ -549,7 +545,14 @@ class Batched:
                 rows = min(npr, -(-it["n"] // (1 << lt)) * (1 << lt))
                 tot += 2 * rows * 12 * sort_passes(int(np.log2(npr)), lt, min(8, lt - 4))
             else:
-                tot += 2 * npr * 13 * compact_passes(int(np.log2(npr)), lt, lmax) + npr * 5
+                # the tile pass reads the tiles with rows and stores every
+                # tile; a fused pass works on its blocks with rows
+                logn = int(np.log2(npr))
+                tot += (-(-it["n"] // (1 << lt)) * (1 << lt) + npr) * 13 + npr * 5
+                b = lt
+                while b < logn:
+                    b = min(logn, b + lmax)
+                    tot += 2 * (-(-it["n"] // (1 << b)) << b) * 13
         return tot
 
     def check(self, orc):

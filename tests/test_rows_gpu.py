@@ -129,10 +129,14 @@ def test_join_topk_ends(cuda, nd, nf, price_hi, k):
     assert counts.tolist() == wc and np.array_equal(out.cpu().numpy(), want)
 
 
-# both routes back to request order (compaction when at most half the rows are
-# requests), repeated and out-of-range ids
+# both routes there (table and sorted requests merged when at least a quarter of
+# more than 4096 rows are table rows) and back to request order (compaction when
+# at most half the rows are requests), repeated and out-of-range ids
 @pytest.mark.parametrize("tn,rn", [(1, 1), (1, 4000), (5000, 5000), (5000, 4999), (5000, 5001), (4095, 1),
-                                   (100_000, 3), (70_001, 300_007), (300_007, 70_001)])
+                                   (100_000, 3), (70_001, 300_007), (300_007, 70_001), (1024, 3072), (1025, 3072),
+                                   (1024, 3073), (1023, 3074), (4097, 1), (8191, 1), (8192, 1), (4096, 4096),
+                                   (4097, 12_287), (100_000, 31_072), (524_289, 2048), (700_001, 349_000),
+                                   (1 << 20, 1 << 20), (524_288, 1_572_865)])
 def test_gather_routes(cuda, tn, rn):
     rng = np.random.default_rng(tn + rn)
     table = rng.integers(-2**63, 2**63 - 1, tn)
@@ -295,3 +299,39 @@ def test_compaction_level_rule(cuda, n):
     assert np.array_equal(capi.host_u64(k, c), keys[keep]) and np.array_equal(capi.host_u32(p, c), pay[keep])
     tail = capi.host_u64(k, cap)[c:]  # the other rows and the padding, re-routed
     assert np.array_equal(np.sort(tail), np.sort(np.concatenate([keys[~keep], np.full(cap - n, ~np.uint64(0))])))
+
+
+# blocks of padding alone are passed over: one and a few rows past a power of
+# two (whole blocks of every phase are padding), the last row of a block, and
+# the three-CTA form; the passes' results over all 2^k rows
+@pytest.mark.parametrize("n", [4097, 8191, (9 << 13) + 3, (1 << 17) + 5, 5 << 16, (5 << 16) + 1, (1 << 21) - (1 << 18),
+                               (1 << 20) + 4097, (5 << 19) + 1])
+def test_blocks_of_padding(cuda, orc, n):
+    rng = np.random.default_rng(n)
+    cap = capi.next_pow2(n)
+    rec, marks = np.full((cap, 16), 255, np.uint8), np.zeros(cap, np.uint8)
+    keys, pay = rng.integers(0, 2**63, n).astype(np.uint64), np.arange(n, dtype=np.uint32)
+    rec[:n, :8] = keys.view(np.uint8).reshape(n, 8)
+    rec[:n, 8:12] = pay.view(np.uint8).reshape(n, 4)
+    for density in (0.3, 1.0):
+        marks[:n] = rng.random(n) < density
+        want, wm, wc = orc.ocompact(rec, marks)
+        k, p, m = capi.to_dev_u64(keys, cap), capi.to_dev_u32(pay, cap), capi.to_dev_u8(marks[:n], cap)
+        count = int(capi.ocompact_kpm(k, p, m, n).item())
+        assert count == wc and np.array_equal(m.cpu().numpy(), wm)
+        assert np.array_equal(capi.host_u64(k), np.ascontiguousarray(want[:, :8]).view(np.uint64).reshape(-1))
+        assert np.array_equal(capi.host_u32(p), np.ascontiguousarray(want[:, 8:12]).view(np.uint32).reshape(-1))
+    for types, asc in (((BIGINT,), (True,)), ((INTEGER, DATE), (False, True)), ((BIGINT, DATE), (False, False))):
+        dts = {INTEGER: np.int32, BIGINT: np.int64, DATE: np.uint32}
+        cols = [rng.integers(0, 50, n).astype(dts[t]) for t in types]
+        cols[0][: n // 3] = np.iinfo(dts[types[0]]).max  # the padding's own key
+        want, widx = orc.bitonic_sort_cols(cols, types, asc, n)
+        dev = []
+        for c in cols:
+            x = np.zeros(cap, c.dtype)
+            x[:n] = c
+            dev.append(torch.from_numpy(x.view(np.int32) if x.dtype == np.uint32 else x).cuda())
+        idx = capi.sort_columns(dev, types, asc, n)
+        assert np.array_equal(idx.cpu().numpy(), widx), (types, asc)
+        for d, w in zip(dev, want):
+            assert np.array_equal(d.cpu().numpy(), w.view(d.cpu().numpy().dtype))

@@ -22,7 +22,7 @@
 // A predicate with price_hi = INT64_MAX leaves no order word free for a row
 // that fails, so it takes the record form: 16-byte records of next_pow2 rows,
 // sort on (key, tag), forward fill of the last dimension row, segmented sums,
-// top-k.  (1.5 M x 6 M rows: JOIN_FILL)
+// top-k.
 // Record layout of that form (2 u64 words):
 //   w0 = [63:32] key ^ 0x80000000 | [31] tag (0 dim, 1 fact) | [30] row passes
 //        its side's filter | [29] joined (set by fill) ; w1 = price (fact rows)

@@ -115,9 +115,10 @@ static velo_status batch_plan(velo_batch* b, const velo_batch_item* items, size_
             per[i].push_back({ STEP_COMPACT_SCAN, NetPass {} });
             tiles[i].push_back(1);
             plan_compact(in.logN, lt, lmax, passes);
+            const NetGeom g(it.n, in.logN);
             for (auto& p : passes) {
                 per[i].push_back({ STEP_COMPACT_PASS, p });
-                tiles[i].push_back((uint32_t)ntiles);
+                tiles[i].push_back((uint32_t)net_pass_tiles(g, p, lt));
             }
             scratch_u32 += (size_t)2 * ntiles + 1 + 64; // counts + prefix, 256-byte aligned below
         }

@@ -253,9 +253,10 @@ static velo_status sort_cols(const ColSpec& s, size_t n, int logN, uint64_t* wor
         std::vector<NetPass> passes;
         const int lt = LOG_NT + LOG_E;
         plan_sort(logN, lt, FORM == FORM_WORD ? (lt - 5 < 8 ? lt - 5 : 8) : 8, passes);
-        // every row is materialised by the pack kernel, so n = np here; the
-        // order of equal keys is seen, so the padding stays in the network
-        NetGeom g { np, logN, 0 };
+        // every row is materialised by the pack kernel; the order of equal keys
+        // is seen, so the padding stays in the network.  The compares are
+        // strict: blocks of padding alone stay in their order.
+        const NetGeom g = NetGeom::padded(n, logN);
         velo_status rc =
             launch_net<R, LOG_NT, LOG_E>(sort_cols_of((R*)nullptr, words, np), g, passes, nullptr, st);
         if (rc != VELO_OK)
