@@ -129,13 +129,15 @@ def test_join_topk_ends(cuda, nd, nf, price_hi, k):
     assert counts.tolist() == wc and np.array_equal(out.cpu().numpy(), want)
 
 
-# both routes there (table and sorted requests merged when at least a quarter of
-# more than 4096 rows are table rows) and back to request order (compaction when
-# at most half the rows are requests), repeated and out-of-range ids
+# both routes there (table and sorted requests merged when at least three eighths
+# of more than 2^18 rows are table rows) and back to request order (compaction when
+# at most an eighth of the rows are requests, half above 2^18), repeated and
+# out-of-range ids
 @pytest.mark.parametrize("tn,rn", [(1, 1), (1, 4000), (5000, 5000), (5000, 4999), (5000, 5001), (4095, 1),
                                    (100_000, 3), (70_001, 300_007), (300_007, 70_001), (1024, 3072), (1025, 3072),
                                    (1024, 3073), (1023, 3074), (4097, 1), (8191, 1), (8192, 1), (4096, 4096),
-                                   (4097, 12_287), (100_000, 31_072), (524_289, 2048), (700_001, 349_000),
+                                   (4097, 12_287), (100_000, 31_072), (98_304, 163_841), (98_303, 163_842), (262_143, 1),
+                                   (262_144, 1), (7000, 1000), (6999, 1001), (524_289, 2048), (700_001, 349_000),
                                    (1 << 20, 1 << 20), (524_288, 1_572_865)])
 def test_gather_routes(cuda, tn, rn):
     rng = np.random.default_rng(tn + rn)
