@@ -28,9 +28,7 @@
 
 namespace velo {
 
-constexpr int GB_LT = 12; // 4096-row tiles (CTA shape per record width: Tile12)
-// up to 8 fused global levels: 16 contiguous rows of 8-byte words fill a line
-constexpr int GB_LMAX = GB_LT - 4 < 8 ? GB_LT - 4 : 8;
+constexpr int GB_LT = 12; // compaction in 4096-row tiles (CTA shape per record width: Tile12)
 // compactions: up to 10 (4-row segments of a 32-byte sector)
 constexpr int GB_LMAX_COMPACT = GB_LT - 2;
 constexpr uint64_t GB_EXCL = 1ull << 63;
@@ -397,7 +395,7 @@ static velo_status gb_run(const GbScratch& s, const GbIn& in, size_t n, size_t b
     }
     const int logN = ilog2_floor(s.n_rec);
     // the sort leaves out the padding past the last tile; so do the later steps
-    const NetGeom geom = NetGeom::trimmed(n, logN, GB_LT, 0);
+    const NetGeom geom = NetGeom::trimmed(n, logN, sort_lt(logN), 0);
     const size_t m = geom.m;
     VELO_CUDA_TRY(cudaMemsetAsync(s.rejected, 0, 8, st), "cudaMemsetAsync");
     k_gb_pack<NS><<<gb_grid(n), 256, 0, st>>>(in, n, n, s.r[0], s.r[1], s.r[2], s.rejected);
@@ -412,9 +410,7 @@ static velo_status gb_run(const GbScratch& s, const GbIn& in, size_t n, size_t b
     rc.mark_bit = 63;
     rc.mark_inv = 1;
     rc.mark_word = 0;
-    std::vector<NetPass> passes;
-    plan_sort(logN, GB_LT, GB_LMAX, passes);
-    velo_status rc2 = launch_net12<typename T::Rec>(rc, geom, passes, nullptr, st);
+    velo_status rc2 = launch_sort<typename T::Rec>(rc, geom, st);
     if (rc2 != VELO_OK)
         return rc2;
 
@@ -437,7 +433,7 @@ static velo_status gb_run(const GbScratch& s, const GbIn& in, size_t n, size_t b
     rc2 = launch_count_scan<typename T::Grp>(gc, m, logN, GB_LT, s.counts, s.prefix, s.n_grp_rows, st);
     if (rc2 != VELO_OK)
         return rc2;
-    passes.clear();
+    std::vector<NetPass> passes;
     plan_compact(logN, GB_LT, GB_LMAX_COMPACT, passes);
     rc2 = launch_net12<typename T::Grp>(gc, NetGeom(m, logN), passes, s.prefix, st);
     if (rc2 != VELO_OK)
@@ -469,7 +465,7 @@ static velo_status gb_run_wide(const GbScratch& s, const GbIn& in, int with_coun
             done[dev] = 1;
     }
     const int logN = ilog2_floor(s.n_rec);
-    const NetGeom geom = NetGeom::trimmed(n, logN, GB_LT, 0);
+    const NetGeom geom = NetGeom::trimmed(n, logN, sort_lt(logN), 0);
     const size_t m = geom.m;
     unsigned long long* extra = s.rejected; // 3 words of its 256 bytes
     VELO_CUDA_TRY(cudaMemsetAsync(extra, 0, 24, st), "cudaMemsetAsync");
@@ -484,9 +480,7 @@ static velo_status gb_run_wide(const GbScratch& s, const GbIn& in, int with_coun
     rc.mark_bit = 0;
     rc.mark_inv = 0;
     rc.mark_word = 0;
-    std::vector<NetPass> passes;
-    plan_sort(logN, GB_LT, GB_LMAX, passes);
-    velo_status rc2 = launch_net12<typename T::Rec>(rc, geom, passes, nullptr, st);
+    velo_status rc2 = launch_sort<typename T::Rec>(rc, geom, st);
     if (rc2 != VELO_OK)
         return rc2;
     const int nts = (int)(m / SEG_TS);
@@ -507,7 +501,7 @@ static velo_status gb_run_wide(const GbScratch& s, const GbIn& in, int with_coun
     rc2 = launch_count_scan<typename T::Grp>(gc, m, logN, GB_LT, s.counts, s.prefix, s.n_grp_rows, st);
     if (rc2 != VELO_OK)
         return rc2;
-    passes.clear();
+    std::vector<NetPass> passes;
     plan_compact(logN, GB_LT, GB_LMAX_COMPACT, passes);
     rc2 = launch_net12<typename T::Grp>(gc, NetGeom(m, logN), passes, s.prefix, st);
     if (rc2 != VELO_OK)

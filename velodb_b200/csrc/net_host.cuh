@@ -98,6 +98,12 @@ struct Tile12 {
     static constexpr bool WIDE_COMPACT = R::WORDS >= 3;
 };
 
+template <int CM>
+struct Tile12<RowK12<CM>> {
+    static constexpr bool WIDE_SORT = false;
+    static constexpr bool WIDE_COMPACT = false;
+};
+
 template <class R>
 inline velo_status launch_net12(const typename R::Cols& c, const NetGeom& g, const std::vector<NetPass>& passes,
                                 const uint32_t* tile_prefix, cudaStream_t st)
@@ -106,6 +112,28 @@ inline velo_status launch_net12(const typename R::Cols& c, const NetGeom& g, con
     if (compact ? Tile12<R>::WIDE_COMPACT : Tile12<R>::WIDE_SORT)
         return launch_net<R, 9, 3>(c, g, passes, tile_prefix, st);
     return launch_net<R, 8, 4>(c, g, passes, tile_prefix, st);
+}
+
+// log2 of the tile of an operator's sort of 2^logN rows, 4096 rows or fewer a
+// tile: 2048 (256 threads x 8) up to 2^18 rows, where a pass is one short wave
+// and its time a CTA's latency, as in the plain sort (network.cu).  Against 4096
+// (us a call): ORDER BY (DOUBLE, DATE) of 5000 rows 59 -> 46, 50,000 94 -> 68,
+// 2^18 125 -> 96; GROUP BY of BIGINT keys with a sum 100 -> 88, 136 -> 113, 168
+// -> 145; PK-FK join 93 -> 81, 134 -> 113, 159 -> 136.  Plain sorts of 2^19
+// rows are faster with 4096 (109 against 123).
+constexpr int SORT_SMALL_LOGN = 18;
+inline int sort_lt(int logN) { return logN <= SORT_SMALL_LOGN ? 11 : 12; }
+
+// A whole sort in those tiles (a trimmed `g` is trimmed to sort_lt(g.logN))
+template <class R>
+inline velo_status launch_sort(const typename R::Cols& c, const NetGeom& g, cudaStream_t st)
+{
+    std::vector<NetPass> passes;
+    const int lt = sort_lt(g.logN);
+    plan_sort(g.logN, lt, lt - 4, passes);
+    if (lt == 11)
+        return launch_net<R, 8, 3>(c, g, passes, nullptr, st);
+    return launch_net12<R>(c, g, passes, nullptr, st);
 }
 
 // A whole bitonic sort of 2^logN pipeline records in 4096-row tiles (8192-row

@@ -5,6 +5,7 @@
 
 using JoinRec = velo::RowRec<2, 1, false, velo::KEY_FULL>;
 VELO_INSTANTIATE_NET(JoinRec, 8, 4)
+VELO_INSTANTIATE_NET(JoinRec, 8, 3)
 
 VELO_INSTANTIATE_NET(velo::RowU2, 8, 5)
 
@@ -12,5 +13,7 @@ VELO_INSTANTIATE_NET(velo::RowU2, 8, 5)
 using GbRec1 = velo::RowRec<1, 1, false, velo::KEY_FULL>;
 using GbRec3 = velo::RowRec<3, 1, false, velo::KEY_FULL>;
 VELO_INSTANTIATE_NET(GbRec1, 8, 4)
+VELO_INSTANTIATE_NET(GbRec1, 8, 3)
 VELO_INSTANTIATE_NET(GbRec3, 8, 4)
+VELO_INSTANTIATE_NET(GbRec3, 8, 3)
 VELO_INSTANTIATE_NET(GbRec3, 9, 3)

@@ -592,9 +592,7 @@ extern "C" velo_status velo_ojoin_pkfk(const void* d_build_keys, const uint8_t* 
     VELO_CUDA_TRY(cudaGetLastError(), "ojoin pack launch");
     // sort on (key, tag); the probe rows of a key are seen in the padded
     // network's order, so the padding stays in it
-    std::vector<NetPass> passes;
-    plan_sort(logR, OP_LT, OP_LMAX, passes);
-    velo_status rc = launch_net<RowK12<K12_KEY_TAG>, 8, 4>({ k, p }, NetGeom(n, logR), passes, nullptr, st);
+    velo_status rc = launch_sort<RowK12<K12_KEY_TAG>>({ k, p }, NetGeom(n, logR), st);
     if (rc != VELO_OK)
         return rc;
     // pairs, one word each, compacted to the front

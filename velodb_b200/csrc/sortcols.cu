@@ -241,7 +241,8 @@ static RowK12<K12_KEY>::Cols sort_cols_of(RowK12<K12_KEY>*, uint64_t* words, siz
     return { words, reinterpret_cast<uint32_t*>(words + np) };
 }
 
-template <class R, int KW, int FORM, int LOG_NT, int LOG_E>
+// (LOG_NT, LOG_E): CTA of the records with an index word
+template <class R, int KW, int FORM, int LOG_NT = 8, int LOG_E = 4>
 static velo_status sort_cols(const ColSpec& s, size_t n, int logN, uint64_t* words, int64_t* indices, cudaStream_t st)
 {
     const size_t np = (size_t)1 << logN;
@@ -250,15 +251,20 @@ static velo_status sort_cols(const ColSpec& s, size_t n, int logN, uint64_t* wor
     k_pack_cols<KW, FORM><<<blocks, threads, 0, st>>>(s, n, np, words);
     VELO_CUDA_TRY(cudaGetLastError(), "pack launch");
     if (np > 1) {
-        std::vector<NetPass> passes;
-        const int lt = LOG_NT + LOG_E;
-        plan_sort(logN, lt, FORM == FORM_WORD ? (lt - 5 < 8 ? lt - 5 : 8) : 8, passes);
         // every row is materialised by the pack kernel; the order of equal keys
         // is seen, so the padding stays in the network.  The compares are
         // strict: blocks of padding alone stay in their order.
         const NetGeom g = NetGeom::padded(n, logN);
-        velo_status rc =
-            launch_net<R, LOG_NT, LOG_E>(sort_cols_of((R*)nullptr, words, np), g, passes, nullptr, st);
+        const auto c = sort_cols_of((R*)nullptr, words, np);
+        velo_status rc;
+        if constexpr (FORM == FORM_WORD) {
+            std::vector<NetPass> passes;
+            const int lt = LOG_NT + LOG_E;
+            plan_sort(logN, lt, lt - 5 < 8 ? lt - 5 : 8, passes);
+            rc = launch_net<R, LOG_NT, LOG_E>(c, g, passes, nullptr, st);
+        } else {
+            rc = launch_sort<R>(c, g, st);
+        }
         if (rc != VELO_OK)
             return rc;
     }
@@ -339,11 +345,11 @@ extern "C" velo_status velo_sort_columns(void* const* d_cols, const uint32_t* ty
     cudaStream_t st = (cudaStream_t)stream;
     const int bits = key_bits(types, n_cols);
     if (bits <= 32)
-        return sort_cols<RowRec<1, 1, true, KEY_HI32>, 1, FORM_LOW, 8, 4>(s, n, logN, words, d_indices, st);
+        return sort_cols<RowRec<1, 1, true, KEY_HI32>, 1, FORM_LOW>(s, n, logN, words, d_indices, st);
     if (bits <= 64)
-        return sort_cols<RowK12<K12_KEY>, 1, FORM_K12, 8, 4>(s, n, logN, words, d_indices, st);
+        return sort_cols<RowK12<K12_KEY>, 1, FORM_K12>(s, n, logN, words, d_indices, st);
     if (bits <= 96)
-        return sort_cols<RowRec<2, 2, true, KEY_HI96>, 2, FORM_LOW, 8, 4>(s, n, logN, words, d_indices, st);
+        return sort_cols<RowRec<2, 2, true, KEY_HI96>, 2, FORM_LOW>(s, n, logN, words, d_indices, st);
     switch (kw) {
     case 2:
         return sort_cols<RowRec<3, 2>, 2, FORM_WORD, 8, 4>(s, n, logN, words, d_indices, st);
