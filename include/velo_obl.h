@@ -108,16 +108,19 @@ typedef struct velo_pass_time {
     float ms;
 } velo_pass_time;
 void velo_set_pass_timing(int on);
-/* Tune: run the in-tile merge passes of 4096-row sorts (key-payload rows and
- * two- or three-word records) as one persistent CTA per SM that prefetches
- * the next tile with bulk copies into a second shared-memory buffer while
- * the current tile's levels run (0 = off, the default).  Same network, same
- * results.  No reference counterpart. */
+/* Tune: run the in-tile merge passes of sorts in 4096-row tiles of 256 threads
+ * (12-byte rows and records of up to three words, padding left out or not) as
+ * one persistent CTA per SM that prefetches the next tile with bulk copies
+ * into a second shared-memory buffer while the current tile's levels run (0 =
+ * off, the default).  Same network, same results.  Sorts of up to 2^18 rows
+ * run smaller tiles by default, and the key sort of velo_filter_groupby has
+ * rows of its own: neither tune acts on them, nor on a command queue's or a
+ * batch's persistent kernel.  No reference counterpart. */
 void velo_set_merge_pipeline(int on);
 /* Tune: load the rows of each in-tile merge and fused global pass of sorts
- * in 4096-row tiles (key-payload rows, two- or three-word records) with one
- * 3-D tensor-map copy per word array into shared memory instead of
- * per-thread loads (0 = off, the default).  Same grid, same network, same
+ * in tiles of 4096 rows or more (the same rows) with one 3-D tensor-map copy
+ * per word array into shared memory instead of per-thread loads (0 = off, the
+ * default).  Same grid, same network, same
  * results.  The tensor maps cover the calling GPU's own arrays.  No
  * reference counterpart. */
 void velo_set_tensor_tile_loads(int on);

@@ -172,14 +172,15 @@ inline bool tma_passes_on(const typename R::Cols& c)
 
 // The bulk-copy merge pass (pipe.cuh) for this row type and tile shape, when
 // it is switched on (velo_set_merge_pipeline) and the word arrays allow bulk
-// copies; returns the grid (one CTA per SM) or 0 for the plain merge kernel.
+// copies; returns the most CTAs of a grid (one per SM) or 0 for the plain merge
+// kernel.
 template <class R, int LOG_NT, int LOG_E>
-inline unsigned merge_pipe_grid(const typename R::Cols& c, size_t ntiles, cudaStream_t)
+inline unsigned merge_pipe_grid(const typename R::Cols& c, size_t ntiles)
 {
 #ifdef VELO_TRACE
     return 0;
 #else
-    if constexpr (!pipe_capable<R, LOG_NT, LOG_E>() || Flip<R>::on) {
+    if constexpr (!pipe_capable<R, LOG_NT, LOG_E>()) {
         return 0;
     } else {
         if (!merge_pipe_on() || ntiles < 2 || !Stage<R>::aligned(c))
@@ -256,18 +257,16 @@ velo_status launch_net(const typename R::Cols& c, const NetGeom& g, const std::v
         return rc;
     const int lt = N::LT;
     const size_t grid = g.logN > lt ? ((size_t)1 << (g.logN - lt)) : 1;
-    const bool whole = g.m == (size_t)1 << g.logN; // not trimmed
     // the first pass follows whatever ran before it; the later ones overlap
     // their launch with the tail of the previous pass
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
-    // (the load tunes work on whole networks)
-    const unsigned pipe_grid = compact || !whole ? 0u : merge_pipe_grid<R, LOG_NT, LOG_E>(c, grid, st);
+    const unsigned pipe_grid = compact ? 0u : merge_pipe_grid<R, LOG_NT, LOG_E>(c, grid);
     int* pipe_fault = nullptr;
     if (pipe_grid)
         VELO_CUDA_TRY(cudaGetSymbolAddress((void**)&pipe_fault, s_pipe_fault), "cudaGetSymbolAddress");
-    const bool tma = !compact && whole && tma_passes_on<R, LOG_NT, LOG_E>(c);
+    const bool tma = !compact && tma_passes_on<R, LOG_NT, LOG_E>(c);
     int* tma_fault = tma ? tma_fault_word() : nullptr;
     PassTimer timer(st, passes.size());
     for (size_t i = 0; i < passes.size(); i++) {
@@ -279,12 +278,13 @@ velo_status launch_net(const typename R::Cols& c, const NetGeom& g, const std::v
         cfg.attrs = attr;
         cfg.numAttrs = (i > 0 && !timer.on()) ? 1 : 0;
         if (pipe_grid && passes[i].kind == P_SORT_MERGE) {
-            if constexpr (pipe_capable<R, LOG_NT, LOG_E>() && !Flip<R>::on) {
-                cfg.gridDim = dim3(pipe_grid);
+            if constexpr (pipe_capable<R, LOG_NT, LOG_E>()) {
+                const unsigned tiles = cfg.gridDim.x; // all of its rows are below g.m
+                cfg.gridDim = dim3(tiles < pipe_grid ? tiles : pipe_grid);
                 cfg.blockDim = dim3(1u << PIPE_LOG_NT);
                 cfg.dynamicSmemBytes = 2 * pipe_buf_bytes<R, PIPE_LOG_NT, PIPE_LOG_E>();
                 VELO_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_merge_pipe<R, PIPE_LOG_NT, PIPE_LOG_E>, c, g, passes[i].K,
-                                                 (int)grid, pipe_fault),
+                                                 (int)tiles, pipe_fault),
                               "network merge pass launch");
             }
         } else if (tma && (passes[i].kind == P_SORT_GLOBAL || passes[i].kind == P_SORT_MERGE)) {

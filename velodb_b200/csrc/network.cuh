@@ -611,8 +611,10 @@ struct Net {
         if constexpr (!std::is_void_v<ST>) {
             const int tp = tidpart(s);
 #pragma unroll
-            for (int e = 0; e < E; e++)
-                v[e] = ST::read(sm, T, tp | (e << s));
+            for (int e = 0; e < E; e++) {
+                const int l = tp | (e << s);
+                v[e] = is_global && gidx(l) >= Np ? R::pad(c) : ST::read(sm, T, l);
+            }
             // the staged tile is overwritten by the first transpose
             __syncthreads();
         } else {

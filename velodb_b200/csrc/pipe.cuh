@@ -94,23 +94,25 @@ struct Stage {
     static constexpr bool ok = false;
 };
 
-template <>
-struct Stage<RowKP> {
+template <int CM>
+struct Stage<RowK12<CM>> {
+    using R = RowK12<CM>;
     static constexpr bool ok = true;
     static constexpr size_t bytes(int T) { return (size_t)T * 12; }
-    __host__ static bool aligned(const RowKP::Cols& c)
+    __host__ static bool aligned(const typename R::Cols& c)
     {
         return ((uintptr_t)c.k % 16) == 0 && ((uintptr_t)c.p % 16) == 0;
     }
-    __device__ __forceinline__ static void issue(const RowKP::Cols& c, size_t base, int T, char* buf, uint64_t* bar)
+    __device__ __forceinline__ static void issue(const typename R::Cols& c, size_t base, int T, char* buf,
+                                                 uint64_t* bar)
     {
         bulk_g2s(buf, c.k + base, (uint32_t)T * 8, bar);
         bulk_g2s(buf + (size_t)T * 8, c.p + base, (uint32_t)T * 4, bar);
     }
-    __device__ __forceinline__ static RowKP read(const char* buf, int T, int r)
+    __device__ __forceinline__ static R read(const char* buf, int T, int r)
     {
         const uint64_t k = reinterpret_cast<const uint64_t*>(buf)[r];
-        return RowKP { lo32(k), hi32(k), reinterpret_cast<const uint32_t*>(buf + (size_t)T * 8)[r] };
+        return R { lo32(k), hi32(k), reinterpret_cast<const uint32_t*>(buf + (size_t)T * 8)[r] };
     }
 };
 
@@ -223,7 +225,9 @@ __global__ void __launch_bounds__(1 << LOG_NT, 1)
             v[e] = Stage<R>::read(buf, T, tp | (e << S0));
         __syncthreads(); // the staged tile is overwritten by the first transpose
         // levels LT-1 .. 0 of phase 2^K, direction fixed for the tile
-        const bool asc_c = ((cta_bits >> K) & 1) == 0;
+        const bool asc_c = (((cta_bits ^ g.dirx) >> K) & 1) == 0;
+        if constexpr (N::FLIP)
+            N::flip_all(v, asc_c);
         int s = S0;
         int b = LT - 1;
         while (b >= 0) {
@@ -232,9 +236,11 @@ __global__ void __launch_bounds__(1 << LOG_NT, 1)
                 N::template transpose<true, true>(v, s, ns, buf);
                 s = ns;
             }
-            N::bitonic_window(v, c, s, b, s, K, true, asc_c);
+            N::bitonic_window(v, c, s, b, s, K, true, N::FLIP || asc_c);
             b = s - 1;
         }
+        if constexpr (N::FLIP)
+            N::flip_all(v, asc_c);
         if (s != S0) {
             N::template transpose<true, true>(v, s, S0, buf);
             s = S0;

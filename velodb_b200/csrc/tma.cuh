@@ -13,7 +13,9 @@
 // fused global pass of L levels; an in-tile merge is C = LT, L = 0).  Viewed
 // as a 3-D array of one word array, (d0, 2^b_lo / d0, N / 2^b_lo) with
 // d0 = min(2^C, 256), that is one box (d0, 2^C / d0, 2^L) whose innermost
-// coordinate is 0, so every copy starts on a 16-byte boundary.
+// coordinate is 0, so every copy starts on a 16-byte boundary.  In a trimmed
+// network (NetGeom) a box may hold rows from m on: they lie inside the arrays of
+// 2^logN rows, and the pass takes padding in their place.
 //
 // A tensor copy wants its shared-memory destination on a 128-byte boundary
 // and its tensor map on a 64-byte one.  The kernel has no static shared
@@ -37,27 +39,29 @@ template <class R>
 struct TmaRows {
     static constexpr bool ok = false;
 };
-template <>
-struct TmaRows<RowKP> {
+template <int CM>
+struct TmaRows<RowK12<CM>> {
     static constexpr bool ok = true;
     static constexpr int NARR = 2;
-    static void arrays(const RowKP::Cols& c, void* (&base)[3], int (&es)[3])
+    static constexpr int row_bytes(int x) { return x == 0 ? 8 : 4; } // of array x
+    static void arrays(const typename RowK12<CM>::Cols& c, void* (&base)[3], int (&es)[3])
     {
         base[0] = c.k;
-        es[0] = 8;
+        es[0] = row_bytes(0);
         base[1] = c.p;
-        es[1] = 4;
+        es[1] = row_bytes(1);
     }
 };
 template <int W, int KW, bool S, int KM>
 struct TmaRows<RowRec<W, KW, S, KM>> {
     static constexpr bool ok = W <= 3;
     static constexpr int NARR = W;
+    static constexpr int row_bytes(int) { return 8; }
     static void arrays(const typename RowRec<W, KW, S, KM>::Cols& c, void* (&base)[3], int (&es)[3])
     {
         for (int x = 0; x < W && x < 3; x++) {
             base[x] = c.w[x];
-            es[x] = 8;
+            es[x] = row_bytes(x);
         }
     }
 };
@@ -143,8 +147,7 @@ __global__ void __launch_bounds__(1 << LOG_NT, MB)
 #pragma unroll
             for (int x = 0; x < NARR; x++) {
                 tma_load_3d(sm + off, &maps.m[x], 0, x1, x2, mbar);
-                // array x's rows: 4-byte payloads of key-payload rows, else words
-                off += (size_t)T * (x == 1 && std::is_same_v<R, RowKP> ? 4 : 8);
+                off += (size_t)T * TmaRows<R>::row_bytes(x);
             }
             if (!mbar_wait_bounded(mbar, 0, TMA_WAIT_NS))
                 code = TMA_FAULT_WAIT;
