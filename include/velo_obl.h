@@ -482,11 +482,14 @@ typedef struct velo_lineitem_pred {
     int32_t qty_lo, qty_hi;
 } velo_lineitem_pred;
 
-/* flags: the caller does not mind the filtered count being revealed (the
- * reference FilterCompactionOperator reads it back to the host,
- * src/operator/filter_compaction_operator.cpp:171-178).  Accepted and without
- * effect: no step needs the count on the host, with or without the flag the
- * whole pipeline is oblivious and never synchronises. */
+/* flags: the filtered count may be revealed (the reference
+ * FilterCompactionOperator reads it back to the host,
+ * src/operator/filter_compaction_operator.cpp:171-178): when few of many rows
+ * pass, the call compacts them and sorts next_pow2(filtered count) keys only,
+ * reading the count back to the host first.  Calls of up to 2^19 rows, and calls
+ * on a stream that is being captured, do not read it.  Without this flag the
+ * whole pipeline is oblivious and never synchronises.  The results are the
+ * same. */
 #define VELO_REVEAL_COUNT 1u
 
 /* Oblivious filter + GROUP BY (flag1, flag2) with exact int64 sums:

@@ -346,6 +346,48 @@ struct RowU2 {
     __device__ __forceinline__ static bool marked(const RowU2&) { return false; }
 };
 
+// A 32-bit word as a compaction row, marked unless it is ~0 (a pair of 16-bit
+// keys of rows of which one at least passes).
+struct RowW {
+    uint32_t k;
+    struct Cols {
+        uint32_t* k;
+    };
+    static constexpr int SMEM_BYTES = 4;
+    static constexpr int SWZ_BITS = 5;
+    static constexpr int SLOT_BYTES = 4;
+    __device__ __forceinline__ static RowW load(const Cols& c, size_t g)
+    {
+        VELO_TRACE_AT(TS_ROW_LOAD, c.k + g);
+        return RowW { __ldcg(c.k + g) };
+    }
+    __device__ __forceinline__ static void store(const Cols& c, size_t g, const RowW& r)
+    {
+        VELO_TRACE_AT(TS_ROW_STORE, c.k + g);
+        c.k[g] = r.k;
+    }
+    __device__ __forceinline__ static RowW pad(const Cols&) { return RowW { ~0u }; }
+    __device__ __forceinline__ static void sstore(char* sm, int, int i, const RowW& r)
+    {
+        reinterpret_cast<uint32_t*>(sm)[i] = r.k;
+    }
+    __device__ __forceinline__ static RowW sload(const char* sm, int, int i)
+    {
+        return RowW { reinterpret_cast<const uint32_t*>(sm)[i] };
+    }
+    __device__ __forceinline__ static void sstore_b(char* sm, int, uint32_t b, const RowW& r)
+    {
+        *reinterpret_cast<uint32_t*>(sm + b) = r.k;
+    }
+    __device__ __forceinline__ static RowW sload_b(const char* sm, int, uint32_t b)
+    {
+        return RowW { *reinterpret_cast<const uint32_t*>(sm + b) };
+    }
+    __device__ __forceinline__ static bool swap_pred(const RowW&, const RowW&, bool, const Cols&) { return false; }
+    __device__ __forceinline__ static void cswap(RowW& a, RowW& b, bool x) { xsel(x, a.k, b.k); }
+    __device__ __forceinline__ static bool marked(const RowW& r) { return r.k != ~0u; }
+};
+
 // (u64 key, u32 payload, u8 mark): compaction rows; ordered on (key, payload)
 // with the mark carried, strictly.
 struct RowKPM {

@@ -14,7 +14,8 @@
 //               once; then the smaller and the larger of (low lane i, high lane
 //               N - 1 - i) and one more merge, which leaves the lower half of
 //               all keys sorted in the low lane and the upper half in the high
-//               lane
+//               lane (with VELO_REVEAL_COUNT and few rows passing, of the words
+//               that hold such a row: reveal_words)
 //   3. groups   rows whose key differs from the one before are the groups, in
 //               key order; a prefix count ranks them and each of the first
 //               group_bound becomes a slot
@@ -23,7 +24,8 @@
 // (src/operator/filter_compaction_operator.cpp:65-184) and the sorted
 // segmented sums of obliviator/operator_2/enclave/
 // scalable_oblivious_join.c:221-262: the same groups, counts and sums.  The
-// order of the passes and every address depend on n and group_bound alone.
+// order of the passes and every address depend on n, group_bound and, only where
+// it is revealed, the number of passing rows.
 //
 // Why: sorting 16-byte records of next_pow2(n) rows took 1.74 ms of a 2.17 ms
 // call at 6,001,215 rows (ORCompact 0.31 ms, aggregation 0.29 ms).  The keys
@@ -36,9 +38,12 @@
 
 namespace velo {
 
-// 8192-word key tiles of 256 threads x 32 words (sort of 6 M keys: 320 us with
-// two selects an exchange more; 4096-word tiles 323, 512 threads 368 and 387)
-constexpr int LK_LOG_NT = 8, LK_LOG_E = 5, LK_LT = LK_LOG_NT + LK_LOG_E;
+// log2 of the key words a tile holds, 256 threads of 8, 16 or 32 words, for the
+// network over 2^log_words of them: small ones want more CTAs, large ones fewer
+// passes.  A call with 11 / 12 / 13 (us, 8 groups): 12,000 rows (2^13 words) 60 / 67
+// / 71, 70,001 (2^16) 78 / 86 / 107, 300,000 (2^18) 92 / 100 / 129, 1 M (2^19) 138 /
+// 131 / 146, 3 M (2^21) 281 / 256 / 261, 6 M (2^22) 542 / 436 / 421.
+static int lk_lt(int log_words) { return log_words <= 18 ? 11 : log_words <= 21 ? 12 : 13; }
 constexpr unsigned LK_MAX_BLOCKS = 148 * 8;
 // the sums: 8 slots a thread take 72 registers of sums
 constexpr int LK_SLOTS = 8, LKS_THREADS = 128, LKS_CTAS = 3;
@@ -83,11 +88,79 @@ __global__ void __launch_bounds__(LKS_THREADS, LKS_CTAS) k_li_sums(LiCols c, vel
     li_sums_body<LK_SLOTS, LKS_THREADS>(c, p, n, G, meta, out, d_counts, (int)blockIdx.y, blockIdx.x, gridDim.x, red);
 }
 
+// the sort of h key words, or the last merge of 2^logN words
+static velo_status lk_net(uint32_t* keys, size_t h, int logN, bool merge, cudaStream_t st)
+{
+    const int lt = merge && logN == 12 ? 12 : lk_lt(logN); // (4096 words: one pass)
+    std::vector<NetPass> passes;
+    if (merge)
+        plan_merge(logN, lt, lt - 4, logN, passes);
+    else
+        plan_sort(logN, lt, lt - 4, passes);
+    const RowU2::Cols c { keys };
+    const NetGeom g = merge ? NetGeom(h, logN) : NetGeom::trimmed(h, logN, lt, 0);
+    return lt == 11 ? launch_net<RowU2, 8, 3>(c, g, passes, nullptr, st)
+        : lt == 12  ? launch_net<RowU2, 8, 4>(c, g, passes, nullptr, st)
+                    : launch_net<RowU2, 8, 5>(c, g, passes, nullptr, st);
+}
+
+// the number of passing rows, by one CTA
+__global__ void __launch_bounds__(1024) k_li_rows(LkPlan q)
+{
+    VELO_TRACE_KERNEL(velo_site_hash("k_li_rows"));
+    __shared__ uint32_t tmp[33];
+    const uint32_t rows = lk_sum(q.n_pass, (int)q.nblk, tmp);
+    if (threadIdx.x == 0)
+        q.meta->rows = rows;
+}
+
+// With the count revealed (VELO_REVEAL_COUNT): when next_pow2(rows passing) is at
+// most half of the 2^logH key words, the words that hold such a row are compacted
+// to the front and `rows` words are sorted in the place of all h.  The count
+// costs a copy to the host (about 17 us), so calls below 2^19 words, whose whole
+// sort takes 45 us and less, do without it.
+// Revealed / not / 16-byte records compacted and sorted (us, 8 groups), 2 % of the
+// rows passing: 600,000 rows 114 / 114 / 133, 1 M 124 / 131 / 145, 3 M 182 / 255 /
+// 250, 6,001,215 261 / 420 / 405; 0.2 %: 96 / 131 / 109 at 1 M; 50 %: 435 / 420 /
+// 1,087 at 6,001,215.
+constexpr int LK_REVEAL_LOGH = 19;
+
+static velo_status reveal_words(const LiScratch& s, LkPlan& q, cudaStream_t st)
+{
+    // a stream that is being captured cannot be waited for
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    VELO_CUDA_TRY(cudaStreamIsCapturing(st, &cap), "cudaStreamIsCapturing");
+    if (cap != cudaStreamCaptureStatusNone)
+        return VELO_OK;
+    k_li_rows<<<1, 1024, 0, st>>>(q);
+    VELO_CUDA_TRY(cudaGetLastError(), "group-by count launch");
+    uint64_t rows = 0;
+    VELO_CUDA_TRY(cudaMemcpyAsync(&rows, &q.meta->rows, 8, cudaMemcpyDeviceToHost, st), "cudaMemcpyAsync");
+    VELO_CUDA_TRY(cudaStreamSynchronize(st), "cudaStreamSynchronize");
+    if (next_pow2(rows ? rows : 1) > (size_t)1 << (q.logH - 1))
+        return VELO_OK;
+    // tile counts and their scan in areas that no step of the group-by uses
+    uint32_t* counts = reinterpret_cast<uint32_t*>(s.runs);
+    uint32_t* prefix = reinterpret_cast<uint32_t*>(s.carry);
+    const RowW::Cols c { q.ka };
+    const int lt = q.logH <= 20 ? 12 : 13;
+    velo_status rc = launch_count_scan<RowW>(c, q.h, q.logH, lt, counts, prefix, nullptr, st);
+    if (rc != VELO_OK)
+        return rc;
+    std::vector<NetPass> passes;
+    plan_compact(q.logH, lt, 9, passes); // (8 or 16 words a segment)
+    const NetGeom g(q.h, q.logH);
+    rc = lt == 12 ? launch_net<RowW, 8, 4>(c, g, passes, prefix, st) : launch_net<RowW, 8, 5>(c, g, passes, prefix, st);
+    if (rc == VELO_OK)
+        lk_words(q, s, rows ? rows : 1, 12);
+    return rc;
+}
+
 static velo_status run_groupby(const LiScratch& s, const LiCols& c, size_t n, const velo_lineitem_pred& pred,
-                               uint32_t group_bound, int64_t* d_out, uint64_t* d_counts, cudaStream_t st)
+                               uint32_t group_bound, bool reveal, int64_t* d_out, uint64_t* d_counts, cudaStream_t st)
 {
     const int G = (int)group_bound;
-    const LkPlan q = lk_plan(s, n, LK_LT, LK_MAX_BLOCKS);
+    LkPlan q = lk_plan(s, n, 12, LK_MAX_BLOCKS);
     StageTimer tm(st);
 
     // 1. keys
@@ -95,27 +168,27 @@ static velo_status run_groupby(const LiScratch& s, const LiCols& c, size_t n, co
     VELO_CUDA_TRY(cudaGetLastError(), "group-by keys launch");
     tm.mark();
     // 2. sort both lanes, fold, merge
+    if (reveal && q.logH >= LK_REVEAL_LOGH) {
+        const velo_status rc = reveal_words(s, q, st);
+        if (rc != VELO_OK)
+            return rc;
+    }
     if (q.h > 1) {
-        std::vector<NetPass> passes;
-        plan_sort(q.logH, LK_LT, LK_LMAX, passes);
-        const velo_status rc = launch_net<RowU2, LK_LOG_NT, LK_LOG_E>(
-            RowU2::Cols { q.ka }, NetGeom::trimmed(q.h, q.logH, LK_LT, 0), passes, nullptr, st);
+        const velo_status rc = lk_net(q.ka, q.h, q.logH, false, st);
         if (rc != VELO_OK)
             return rc;
     }
     k_li_fold<<<(unsigned)(q.N / LK_ROWS < LK_MAX_BLOCKS ? q.N / LK_ROWS : LK_MAX_BLOCKS), LK_THREADS, 0, st>>>(q);
     VELO_CUDA_TRY(cudaGetLastError(), "group-by fold launch");
     {
-        std::vector<NetPass> passes;
-        plan_merge(q.logN, LK_LT, LK_LMAX, q.logN, passes);
-        const velo_status rc =
-            launch_net<RowU2, LK_LOG_NT, LK_LOG_E>(RowU2::Cols { q.kb }, NetGeom(q.N, q.logN), passes, nullptr, st);
+        const velo_status rc = lk_net(q.kb, q.N, q.logN, true, st);
         if (rc != VELO_OK)
             return rc;
     }
     tm.mark();
     // 3. the groups' keys in order
-    k_li_distinct<<<q.ntiles, LK_THREADS, 0, st>>>(q);
+    if (q.ntiles > 1)
+        k_li_distinct<<<q.ntiles, LK_THREADS, 0, st>>>(q);
     k_li_slots<<<q.ntiles, LK_THREADS, 0, st>>>(q, G);
     VELO_CUDA_TRY(cudaGetLastError(), "group-by slots launch");
     tm.mark();
@@ -159,6 +232,5 @@ extern "C" velo_status velo_filter_groupby(const velo_lineitem* cols, size_t n, 
     }
     cudaStream_t st = (cudaStream_t)stream;
     LiCols c { cols->qty, cols->price, cols->disc, cols->tax, cols->shipdate, cols->flag1, cols->flag2 };
-    (void)flags; // no step reads the filtered count back, revealed or not
-    return run_groupby(s, c, n, *pred, group_bound, d_out, d_counts, st);
+    return run_groupby(s, c, n, *pred, group_bound, (flags & VELO_REVEAL_COUNT) != 0, d_out, d_counts, st);
 }

@@ -177,7 +177,8 @@ __device__ __forceinline__ uint32_t lk_sum(const uint32_t* x, int n, uint32_t* t
     return total;
 }
 
-// step 3b: the first G first occurrences become the slots.  sm: LK_SM words
+// step 3b: the first G first occurrences become the slots (one tile counts its
+// own, without step 3a).  sm: LK_SM words
 struct LkSlotShared {
     unsigned long long rows;
     uint32_t slot[SEG_MAX_G];
@@ -200,12 +201,17 @@ __device__ __forceinline__ void li_slots_tile(const uint32_t* keys, size_t N, in
         f1 |= ((d >> 16) != 0 && (t.w[r] >> 16) != LK_NONE) ? 1u << r : 0u;
         p = t.w[r];
     }
-    uint32_t total;
-    const uint32_t ex0 = block_exclusive_scan(__popc(f0), x.tmp, &total);
-    const uint32_t ex1 = block_exclusive_scan(__popc(f1), x.tmp, &total);
-    const uint32_t all0 = lk_sum(cnt0, ntiles, x.tmp);
-    const uint32_t rank0 = lk_sum(cnt0, blk, x.tmp) + ex0;
-    const uint32_t rank1 = all0 + lk_sum(cnt1, blk, x.tmp) + ex1;
+    uint32_t all0, all1;
+    const uint32_t ex0 = block_exclusive_scan(__popc(f0), x.tmp, &all0);
+    const uint32_t ex1 = block_exclusive_scan(__popc(f1), x.tmp, &all1);
+    uint32_t rank0 = ex0;
+    uint32_t rank1 = ex1;
+    if (ntiles > 1) {
+        all0 = lk_sum(cnt0, ntiles, x.tmp);
+        rank0 += lk_sum(cnt0, blk, x.tmp);
+        rank1 += lk_sum(cnt1, blk, x.tmp);
+    }
+    rank1 += all0;
     for (int j = 0; j < G; j++) {
         uint32_t v = 0, r0 = rank0, r1 = rank1;
 #pragma unroll
@@ -223,7 +229,7 @@ __device__ __forceinline__ void li_slots_tile(const uint32_t* keys, size_t N, in
     if (blk == 0) {
         // the groups and rows in all; 0xFFFF, which the sort took for a row
         // that fails, is the last group if a passing row has it
-        const uint32_t distinct = all0 + lk_sum(cnt1, ntiles, x.tmp);
+        const uint32_t distinct = all0 + (ntiles > 1 ? lk_sum(cnt1, ntiles, x.tmp) : all1);
         const uint32_t ffff = lk_sum(n_ffff, nblk, x.tmp);
         uint64_t rows = 0;
         for (int i = threadIdx.x; i < nblk; i += LK_THREADS)
@@ -424,20 +430,26 @@ struct LkPlan {
     LkMeta* meta;
 };
 
-inline LkPlan lk_plan(const LiScratch& s, size_t n, int lt, unsigned max_blocks)
+// the key words that are sorted: h of them
+inline void lk_words(LkPlan& q, const LiScratch& s, size_t h, int lt)
 {
-    LkPlan q {};
-    q.h = (n + 1) / 2;
+    q.h = h;
     q.logH = ilog2_floor(next_pow2(q.h));
     q.logN = q.logH < lt ? lt : q.logH;
     q.N = (size_t)1 << q.logN;
     q.ntiles = (int)(q.N / LK_TS);
+    q.cnt0 = s.counts;
+    q.cnt1 = s.counts + q.ntiles;
+}
+
+inline LkPlan lk_plan(const LiScratch& s, size_t n, int lt, unsigned max_blocks)
+{
+    LkPlan q {};
+    lk_words(q, s, (n + 1) / 2, lt);
     const size_t want = (q.h + LK_ROWS - 1) / LK_ROWS;
     q.nblk = want < max_blocks ? (unsigned)want : max_blocks;
     q.ka = reinterpret_cast<uint32_t*>(s.w[0]);
     q.kb = reinterpret_cast<uint32_t*>(s.w[1]);
-    q.cnt0 = s.counts;
-    q.cnt1 = s.counts + q.ntiles;
     q.n_pass = s.prefix;
     q.n_ffff = s.tail_prefix;
     q.meta = reinterpret_cast<LkMeta*>(s.d_rows);

@@ -98,6 +98,10 @@ struct RowBytes<RowU2> {
     static constexpr int value = 4;
 };
 template <>
+struct RowBytes<RowW> {
+    static constexpr int value = 4;
+};
+template <>
 struct RowBytes<RowKPM> {
     static constexpr int value = 13;
 };

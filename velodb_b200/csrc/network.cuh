@@ -124,6 +124,14 @@ struct MarkAt<RowU2> {
     __device__ __forceinline__ static bool get(const RowU2::Cols&, size_t) { return false; }
 };
 template <>
+struct MarkAt<RowW> {
+    __device__ __forceinline__ static bool get(const RowW::Cols& c, size_t g)
+    {
+        VELO_TRACE_AT(TS_MARK_LOAD, c.k + g);
+        return __ldcg(c.k + g) != ~0u;
+    }
+};
+template <>
 struct MarkAt<RowKPM> {
     __device__ __forceinline__ static bool get(const RowKPM::Cols& c, size_t g)
     {
