@@ -156,6 +156,42 @@ def test_filter_groupby_trace_is_data_independent(T):
     assert_same_trace([trace_of(T, run(t)) for t in tabs])
 
 
+def test_revealed_filter_groupby_trace_depends_on_the_count_alone(T):
+    # VELO_REVEAL_COUNT: which rows pass, and with which keys, is not seen
+    n, rows, G = 600_001, 5000, 16
+    dt = dict(qty=torch.int32, price=torch.int64, disc=torch.int32, tax=torch.int32, shipdate=torch.int32,
+              flag1=torch.uint8, flag2=torch.uint8)
+    cols = {k: torch.empty(n, dtype=t, device="cuda") for k, t in dt.items()}
+    li = _lib.VeloLineitem(*[cols[k].data_ptr() for k in dt])
+    pred = _lib.VeloLineitemPred(0, 100, 0, 10, 1, 50)
+    sb = T.velo_filter_groupby_scratch_bytes(n, G)
+    scratch = torch.empty(sb, dtype=torch.uint8, device="cuda")
+    out = torch.empty((G, 6), dtype=torch.int64, device="cuda")
+    counts = torch.empty(2, dtype=torch.int64, device="cuda")
+
+    def run(seed, where, flags, passing=rows):
+        def f():
+            rng = np.random.default_rng(seed)
+            tab = W.lineitem(n, seed=seed)
+            tab["shipdate"][:] = 2000
+            tab["shipdate"][where(rng)[:passing]] = 7
+            tab["flag1"], tab["flag2"] = (rng.integers(0, flags, n).astype(np.uint8) for _ in range(2))
+            for key, v in tab.items():
+                cols[key].copy_(torch.from_numpy(v))
+            torch.cuda.synchronize()
+            assert T.velo_filter_groupby(C.byref(li), n, C.byref(pred), G, 1, out.data_ptr(), counts.data_ptr(),
+                                         scratch.data_ptr(), sb, None) == 0, T.velo_last_error_text()
+            torch.cuda.synchronize()
+            assert int(counts[0]) == passing
+        return f
+
+    anywhere, first = lambda rng: rng.permutation(n), lambda rng: np.arange(n)  # noqa: E731
+    traces = [trace_of(T, run(1, anywhere, 256)), trace_of(T, run(2, first, 1)),
+              trace_of(T, run(3, lambda rng: np.arange(n)[::-1], 3))]
+    assert_same_trace(traces)
+    assert trace_of(T, run(1, anywhere, 256, passing=9000))[0] != traces[0][0]
+
+
 # ---- join + group-by + top-k -----------------------------------------------------------
 
 def test_join_topk_trace_is_data_independent(T):

@@ -4,8 +4,8 @@
 //
 // Each instrumented global load or store folds (site, address) into a hash
 // chain kept per logical thread: logical thread = CTA work index * blockDim +
-// threadIdx, where the work index is blockIdx.x for ordinary kernels and the
-// claimed item for the persistent scheduler.  Chains continue across the
+// threadIdx, where the work index is the CTA's number in the grid for ordinary
+// kernels and the claimed item for the persistent scheduler.  Chains continue across the
 // launches of one stream.  Block 0 of every instrumented kernel appends
 // (kernel id, gridDim, blockDim, dynamic smem bytes) to an ordered launch log.
 // An oblivious operator run twice on different data of the same public size,
@@ -54,14 +54,14 @@ __device__ __forceinline__ void set_work(unsigned long long w)
 
 __device__ __forceinline__ void kernel_begin(uint32_t site)
 {
-    set_work(blockIdx.x);
-    if (blockIdx.x == 0 && threadIdx.x == 0 && g_launch) {
+    set_work(blockIdx.y * (unsigned long long)gridDim.x + blockIdx.x);
+    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0 && g_launch) {
         uint32_t dsmem;
         asm volatile("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dsmem));
         const unsigned long long i = atomicAdd(&g_nlaunch, 1ull);
         if (i < g_launch_cap) {
             g_launch[4 * i + 0] = site;
-            g_launch[4 * i + 1] = gridDim.x;
+            g_launch[4 * i + 1] = gridDim.x * (uint64_t)gridDim.y;
             g_launch[4 * i + 2] = blockDim.x;
             g_launch[4 * i + 3] = dsmem;
         }
