@@ -228,6 +228,33 @@ def test_join_topk_trace_is_data_independent(T):
     assert_same_trace([trace_of(T, run(d, f)) for d, f in sets])
 
 
+def test_join_topk_record_form_trace_is_data_independent(T):
+    # price_hi = 2^63 - 1 leaves no price free for the rows that fail: 16-byte records
+    nd, nf = 20_000, 80_000
+    sets = [W.join_tables(nd, nf, seed=s) for s in (11, 12, 13)]
+    sets[2][1]["fk"][:] = sets[2][0]["key"][0]  # every fact row on one key
+    names = ("key", "date", "fk", "price")
+    bufs = [torch.from_numpy(x.copy()).cuda() for x in (sets[0][0]["key"], sets[0][0]["date"], sets[0][1]["fk"],
+                                                        sets[0][1]["price"])]
+    tab = _lib.VeloJoinTables(bufs[0].data_ptr(), bufs[1].data_ptr(), nd, bufs[2].data_ptr(), bufs[3].data_ptr(), nf)
+    pred = _lib.VeloJoinPred(W.JOIN_PRED["date_hi"], 0, 2**63 - 1)
+    sb = T.velo_join_groupby_topk_scratch_bytes(nd, nf)
+    scratch = torch.empty(sb, dtype=torch.uint8, device="cuda")
+    out = torch.empty((10, 3), dtype=torch.int64, device="cuda")
+    counts = torch.empty(2, dtype=torch.int64, device="cuda")
+
+    def run(dim, fact):
+        def f():
+            for b, name in zip(bufs, names):
+                dev_copy(b, (dim if name in dim else fact)[name])
+            torch.cuda.synchronize()
+            assert T.velo_join_groupby_topk(C.byref(tab), C.byref(pred), 10, out.data_ptr(), counts.data_ptr(),
+                                            scratch.data_ptr(), sb, None) == 0, T.velo_last_error_text()
+        return f
+
+    assert_same_trace([trace_of(T, run(d, f)) for d, f in sets])
+
+
 # ---- batched persistent launch -----------------------------------------------------------
 
 def test_batched_launch_trace_is_data_independent(T):
@@ -330,6 +357,58 @@ def test_shuffle_gather_join_traces_are_data_independent(T):
         return f
 
     assert_same_trace([trace_of(T, join(x, mm)) for x, mm in ((6, False), (7, False), (8, True))])
+
+
+# the routes of the gather: union sorted whole or sorted requests merged with the
+# table, sorted back with or without a compaction before it
+@pytest.mark.parametrize("tn,rn", [(30_000, 4_000), (300_007, 70_001), (200_003, 250_001),
+                                   (100_003, 300_005), (100_003, 180_001)])
+def test_gather_traces_are_data_independent(T, tn, rn):
+    table = torch.empty(tn, dtype=torch.int64, device="cuda")
+    rids = torch.empty(rn, dtype=torch.int32, device="cuda")
+    out = torch.empty(rn, dtype=torch.int64, device="cuda")
+    gb = T.velo_ogather_scratch_bytes(tn, rn)
+    gs = torch.empty(gb, dtype=torch.uint8, device="cuda")
+
+    def gather(seed, dup):
+        def f():
+            rng = np.random.default_rng(seed)
+            dev_copy(table, rng.integers(0, 2**62, tn, dtype=np.int64))
+            r = np.full(rn, 17, np.int32) if dup else rng.integers(0, tn + 100, rn).astype(np.int32)
+            dev_copy(rids, r)
+            torch.cuda.synchronize()
+            assert T.velo_ogather_u64(table.data_ptr(), tn, rids.data_ptr(), rn, out.data_ptr(), gs.data_ptr(), gb,
+                                      None) == 0
+        return f
+
+    assert_same_trace([trace_of(T, gather(x, d)) for x, d in ((3, False), (4, False), (5, True))])
+
+
+# key bits: index in the key word (32, 96), as payload (64), in a word of its own
+@pytest.mark.parametrize("types", [(10,), (5,), (5, 10), (5, 5)])
+def test_sort_columns_trace_is_data_independent(T, types):
+    n = 70_001
+    cap = 1 << 17
+    dt = {5: np.int64, 10: np.int32}
+    cols = [torch.empty(cap, dtype=torch.from_numpy(np.empty(0, dt[t])).dtype, device="cuda") for t in types]
+    ptrs = (C.c_void_p * len(types))(*[c.data_ptr() for c in cols])
+    ty = (C.c_uint32 * len(types))(*types)
+    asc = (C.c_uint8 * len(types))(*[i % 2 for i in range(len(types))])
+    idx = torch.empty(cap, dtype=torch.int64, device="cuda")
+    sb = T.velo_sort_scratch_bytes(ty, len(types), n)
+    s = torch.empty(sb, dtype=torch.uint8, device="cuda")
+
+    def run(seed, span):
+        def f():
+            rng = np.random.default_rng(seed)
+            for c, t in zip(cols, types):
+                dev_copy(c, rng.integers(0, span, n).astype(dt[t]))
+            torch.cuda.synchronize()
+            assert T.velo_sort_columns(ptrs, ty, asc, len(types), n, cap, idx.data_ptr(), s.data_ptr(), sb,
+                                       None) == 0, T.velo_last_error_text()
+        return f
+
+    assert_same_trace([trace_of(T, run(x, sp)) for x, sp in ((1, 2**31 - 1), (2, 2**31 - 1), (3, 1))])
 
 
 def test_column_compaction_trace_is_data_independent(T):

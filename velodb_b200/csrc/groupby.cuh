@@ -96,6 +96,10 @@ __device__ __forceinline__ void li_fold_body(const uint32_t* in, size_t h, size_
     for (size_t i = blk * (size_t)LK_THREADS + threadIdx.x; VELO_GRID_COND(i, N);
          i += nblk * (size_t)LK_THREADS) {
         const size_t r = N - 1 - i;
+        if (i < h)
+            VELO_TRACE_AT(TS_LI_IN, in + i);
+        if (r < h)
+            VELO_TRACE_AT(TS_LI_IN, in + r);
         const uint32_t a = i < h ? in[i] & 0xFFFFu : LK_NONE;
         const uint32_t b = r < h ? in[r] >> 16 : LK_NONE;
         VELO_TRACE_AT(TS_LI_OUT, out + i);

@@ -112,10 +112,14 @@ __global__ void k_ogather_pack(const uint64_t* table, size_t tn_out, const uint3
     {
         uint64_t a;
         uint32_t b;
-        if (g < tn_out)
+        if (g < tn_out) {
+            VELO_TRACE_AT(TS_ROW_LOAD, table + g);
             ogather_table_row(table[g], g, a, b);
-        else
+        } else {
+            VELO_TRACE_AT(TS_ROW_LOAD, rids + (g - tn_out));
             ogather_request_row(rids[g - tn_out], tn, g - tn_out, a, b);
+        }
+        VELO_TRACE_AT(TS_ROW_STORE, k + g);
         k[g] = a;
         p[g] = b;
     }
@@ -132,11 +136,14 @@ __global__ void k_ogather_union(const uint64_t* table, size_t tn, const uint64_t
         uint64_t a = ~0ull;
         uint32_t b = ~0u;
         if (g < rn) {
+            VELO_TRACE_AT(TS_ROW_LOAD, rk + (rn - 1 - g));
             a = rk[rn - 1 - g];
             b = rp[rn - 1 - g];
         } else if (g < rn + tn) {
+            VELO_TRACE_AT(TS_ROW_LOAD, table + (g - rn));
             ogather_table_row(table[g - rn], g - rn, a, b);
         }
+        VELO_TRACE_AT(TS_ROW_STORE, k + g);
         k[g] = a;
         p[g] = b;
     }
@@ -146,7 +153,11 @@ __global__ void k_ogather_out(const uint64_t* k, const uint32_t* p, size_t rn, u
 {
     VELO_TRACE_KERNEL(velo_site_hash("k_ogather_out"));
     VELO_BLK_STRIDE(j, rn, blockIdx.x, gridDim.x)
-    out[j] = (k[j] << 32) | p[j];
+    {
+        VELO_TRACE_AT(TS_ROW_LOAD, k + j);
+        VELO_TRACE_AT(TS_ROW_STORE, out + j);
+        out[j] = (k[j] << 32) | p[j];
+    }
 }
 
 __global__ void k_ojoin_pack(const void* bk, const uint8_t* bm, size_t bn, const void* pk, const uint8_t* pm, size_t pn,
@@ -161,9 +172,11 @@ __global__ void k_ojoin_pack(const void* bk, const uint8_t* bm, size_t bn, const
         const size_t j = build ? g : g - bn;
         const void* keys = build ? bk : pk;
         const uint8_t* mask = build ? bm : pm;
+        VELO_TRACE_AT(TS_ROW_LOAD, static_cast<const char*>(keys) + j * (key64 ? 8 : 4));
         const uint64_t key = key64 ? ((uint64_t) static_cast<const int64_t*>(keys)[j] ^ 0x8000000000000000ull)
                                    : (uint64_t)((uint32_t) static_cast<const int32_t*>(keys)[j] ^ 0x80000000u);
         const bool valid = mask == nullptr || mask[j] != 0;
+        VELO_TRACE_AT(TS_ROW_STORE, k + g);
         k[g] = key;
         p[g] = (build ? 0u : OJ12_TAG) | (valid ? OJ12_VALID : 0u) | (uint32_t)j;
     }
@@ -175,6 +188,8 @@ __global__ void k_ojoin_out(const uint64_t* w, size_t pn, int64_t* ob, int64_t* 
     VELO_TRACE_KERNEL(velo_site_hash("k_ojoin_out"));
     VELO_BLK_STRIDE(i, pn, blockIdx.x, gridDim.x)
     {
+        VELO_TRACE_AT(TS_ROW_LOAD, w + i);
+        VELO_TRACE_AT(TS_ROW_STORE, ob + i);
         const uint64_t x = w[i];
         const bool j = x != ~0ull;
         ob[i] = j ? (int64_t)(x >> 30) : -1;
