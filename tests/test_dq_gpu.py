@@ -10,6 +10,7 @@ import numpy as np
 import pytest
 import torch
 
+from test_rows_gpu import ALL, join_expected, li_columns, li_expected
 from velodb_b200 import capi, workloads as W
 from velodb_b200._lib import VeloJoinPred, VeloJoinTables, VeloLineitem, VeloLineitemPred
 
@@ -150,6 +151,44 @@ def test_join_topk_matches_direct_path(pq, nd, nf, k):
     out2, counts2 = capi.join_groupby_topk(dt, W.JOIN_PRED, k)
     torch.cuda.synchronize()
     assert torch.equal(counts, counts2) and torch.equal(out, out2)
+
+
+# the queue's sums take 4 slots an item: one chunk, a last chunk of one slot, four
+# chunks; key 0xFFFF is also the mark of a row that fails; 256 keys overflow
+@pytest.mark.parametrize("n", [1, 4097, 32_769, 300_001])
+@pytest.mark.parametrize("flags,G", [((0xFFFF,), 1), ((0, 0xFFFF), 8), ((0x00FF, 0x0100, 0xFF00, 0xFFFF), 9),
+                                     (tuple(range(0, 65536, 257)), 1), (tuple(range(0, 65536, 257)), 16)])
+def test_filter_groupby_keys(pq, n, flags, G):
+    c = li_columns(n, n + G, flags)
+    d = capi.lineitem_to_device(c)
+    for pred in (ALL, W.LINEITEM_PRED, dict(ALL, qty_hi=0)):
+        cmd, keep, out, counts = groupby_cmd(d, n, pred, G)
+        ready()
+        pq.wait(pq.submit(cmd))
+        want, wc = li_expected(c, pred, G)
+        assert np.array_equal(out.cpu().numpy(), want) and counts.tolist() == wc
+
+
+# price_hi = INT64_MAX takes the record form, anything below the 12-byte form;
+# keys and prices at both ends, repeated and failing dimension rows
+@pytest.mark.parametrize("nd,nf", [(1, 1), (700, 1349), (1000, 3097), (40_000, 100_000)])
+@pytest.mark.parametrize("price_hi", [2**63 - 1, 2**63 - 2, 1000])
+@pytest.mark.parametrize("k", [1, 17, 300])
+def test_join_topk_ends(pq, nd, nf, price_hi, k):
+    rng = np.random.default_rng(nd + nf + k)
+    ends = np.array([-2**31, -2**31 + 1, -1, 0, 1, 2**31 - 2, 2**31 - 1])
+    keys = np.concatenate([ends, rng.integers(-2**31, 2**31, max(nd // 2, 1))]).astype(np.int32)
+    dk, fk = rng.choice(keys, nd), rng.choice(keys, nf)
+    dd = rng.integers(0, 2, nd).astype(np.int32)
+    pr = rng.choice(np.array([-2**40, -1, 0, 7, 999, 1000, 2**40, 2**63 - 1, 2**63 - 2, 2**63 - 3]), nf)
+    pred = dict(date_hi=1, price_hi=price_hi)
+    dt = capi.join_to_device(dict(key=dk, date=dd), dict(fk=fk, price=pr))
+    cmd, keep, out, counts = join_cmd(dt, pred, k)
+    ready()
+    pq.wait(pq.submit(cmd))
+    with np.errstate(over="ignore"):
+        want, wc = join_expected(dk, dd, fk, pr, pred, k)
+    assert counts.tolist() == wc and np.array_equal(out.cpu().numpy(), want)
 
 
 @pytest.mark.parametrize("key_type", [4, 5])  # INTEGER, BIGINT
