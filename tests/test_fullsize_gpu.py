@@ -201,3 +201,31 @@ def test_served_full_tables_alone_and_in_the_mix(full_tables, orc):
     assert st["peak_inflight"] > 1
     for a, p in zip(ra, rp):
         assert p.status == 0 and S.result_key(a) == S.result_key(p)
+
+
+def test_pkfk_join_of_more_than_2_30_rows(cuda):
+    # row ids no longer fit beside the tag of a 12-byte row: 24-byte records
+    bn, pn, step = 1 << 20, (1 << 30) + 5, 1 << 27
+    if torch.cuda.mem_get_info()[0] < 100 << 30:
+        pytest.skip("needs 100 GB of free device memory")
+    g = torch.Generator(device="cuda")
+    g.manual_seed(1)
+    bk = torch.randperm(bn, generator=g, device="cuda").to(torch.int32)
+    pk = torch.empty(pn, dtype=torch.int32, device="cuda")
+    for i in range(0, pn, step):
+        r = torch.arange(i, min(i + step, pn), device="cuda")
+        pk[i:i + step] = (r * 40_503 + 12_345) % (2 * bn)  # half of the keys have a build row
+    want = sum(int((pk[i:i + step] < bn).sum()) for i in range(0, pn, step))
+    ob, op, counts = capi.ojoin_pkfk(bk, None, pk, None, 4)
+    assert counts.tolist() == [want, 0]
+    seen = torch.zeros(pn, dtype=torch.uint8, device="cuda")
+    last = -1
+    for i in range(0, want, step):
+        j = min(i + step, want)
+        keys = pk[op[i:j]]
+        assert torch.equal(bk[ob[i:j]], keys)
+        assert int(keys[0]) >= last and bool((keys[1:] >= keys[:-1]).all())
+        last = int(keys[-1])
+        seen[op[i:j]] = 1
+    assert sum(int(seen[i:i + step].sum()) for i in range(0, pn, step)) == want  # every probe row once
+    assert all(bool((x[i:i + step] == -1).all()) for x in (ob, op) for i in range(want, pn, step))
