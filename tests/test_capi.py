@@ -76,6 +76,15 @@ def test_compact_scratch_size():
     assert L.velo_compact_scratch_bytes(1 << 23, C.byref(t)) == 2 * ((1 << 10) * 4) + 256
 
 
+def test_filter_groupby_scratch_size():
+    # callers' and servers' budgets are made for these sizes
+    L = velodb_b200.lib()
+    assert L.velo_filter_groupby_scratch_bytes(1, 1) == 100_608
+    assert L.velo_filter_groupby_scratch_bytes(4097, 8) == 202_240
+    assert L.velo_filter_groupby_scratch_bytes(6_001_215, 16) == 208_601_856
+    assert L.velo_filter_groupby_scratch_bytes(100, 17) == 0
+
+
 def test_queue_init_without_device_fails_cleanly():
     import torch
 

@@ -385,7 +385,6 @@ static size_t plan_join_records(B& b, const JoinScratch& s, const velo_join_tabl
     ja.aggs = s.aggs;
     ja.runs = s.runs;
     ja.carry = s.carry;
-    ja.tail_prefix = s.tail_prefix;
     ja.n_groups = s.n_groups;
     ja.out0 = s.cand[0];
     ja.out1 = s.cand[1];
@@ -437,7 +436,6 @@ static size_t plan_join_rows(B& b, const JoinScratch& s, const velo_join_tables*
     ja.aggs = s.aggs;
     ja.runs = s.runs;
     ja.carry = s.carry;
-    ja.tail_prefix = s.tail_prefix;
     ja.n_groups = s.unused;
     ja.ntiles = nt;
     b.step(DQ_K_JK_SUMMARY, (uint64_t)nt, ao);

@@ -170,6 +170,7 @@ struct DqLiArgs {
 constexpr int DQ_LK_SLOTS = 4;
 // 8192-word key tiles (256 threads x 32 words)
 constexpr int DQ_LK_LT = 13;
+static_assert(DQ_LK_LT <= LK_MIN_LOGN, "the scratch holds the merged words");
 
 struct DqJkArgs {
     const int32_t *dk, *dd, *ff;
@@ -209,7 +210,6 @@ struct DqJSegArgs {
     SegTileAgg* aggs;
     int64_t* runs;
     int64_t* carry;
-    uint32_t* tail_prefix;
     uint64_t* n_groups;
     uint64_t *out0, *out1;
     int ntiles;

@@ -251,7 +251,7 @@ __device__ void dq_run(const DqStep& step, const unsigned char* s_args, uint32_t
     }
     case DQ_K_JSEG_CARRIES: {
         const auto& A = dq_arg<DqJSegArgs>(s_args);
-        JSeg::carries(A.aggs, A.runs, A.ntiles, A.carry, A.tail_prefix, A.n_groups, sm);
+        JSeg::carries(A.aggs, A.runs, A.ntiles, A.carry, A.n_groups, sm);
         break;
     }
     case DQ_K_JSEG_EMIT_TOPK: {

@@ -343,7 +343,6 @@ struct RowU2 {
         a.k = lo;
     }
     __device__ __forceinline__ static void flip(RowU2& r, uint32_t m) { r.k ^= m; }
-    __device__ __forceinline__ static bool marked(const RowU2&) { return false; }
 };
 
 // A 32-bit word as a compaction row, marked unless it is ~0 (a pair of 16-bit
@@ -383,7 +382,6 @@ struct RowW {
     {
         return RowW { *reinterpret_cast<const uint32_t*>(sm + b) };
     }
-    __device__ __forceinline__ static bool swap_pred(const RowW&, const RowW&, bool, const Cols&) { return false; }
     __device__ __forceinline__ static void cswap(RowW& a, RowW& b, bool x) { xsel(x, a.k, b.k); }
     __device__ __forceinline__ static bool marked(const RowW& r) { return r.k != ~0u; }
 };
@@ -584,11 +582,8 @@ struct RowRec {
     __device__ __forceinline__ static bool swap_pred(const RowRec& a, const RowRec& b, bool desc, const Cols& c)
     {
         if constexpr (KM == KEY_HI32) {
-            const uint32_t x = hi32(a.w[0]), y = hi32(b.w[0]);
-            if constexpr (STRICT)
-                return x > y; // Flip
-            else
-                return (x > y) != desc;
+            static_assert(STRICT, "one compare for both directions (Flip)");
+            return hi32(a.w[0]) > hi32(b.w[0]);
         }
         if constexpr (KM == KEY_HI96)
             return gt_mask3(hi32(a.w[1]), lo32(a.w[0]), hi32(a.w[0]), hi32(b.w[1]), lo32(b.w[0]), hi32(b.w[0])) != 0u;

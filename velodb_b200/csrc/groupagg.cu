@@ -52,7 +52,6 @@ struct GbAgg {
         for (int s = 0; s < NS; s++)
             v[i + s] = ok ? (int64_t)w[1 + s] : 0;
     }
-    __device__ __forceinline__ static int64_t out_key_from(uint64_t key) { return (int64_t)(key & ~GB_EXCL); }
     __device__ __forceinline__ static uint64_t out_bits(uint64_t key) { return key & ~GB_EXCL; }
 };
 
@@ -75,7 +74,6 @@ struct GbAggWide {
         for (int s = 0; s < NS; s++)
             v[1 + s] = ok ? (int64_t)w[1 + s] : 0;
     }
-    __device__ __forceinline__ static int64_t out_key_from(uint64_t key) { return (int64_t)(key ^ (1ull << 63)); }
     __device__ __forceinline__ static uint64_t out_bits(uint64_t key) { return key; }
 };
 
@@ -210,11 +208,11 @@ __global__ void __launch_bounds__(SEG_THREADS) k_gbw_summary(typename GbTypesWid
 
 template <int NS>
 __global__ void __launch_bounds__(1024) k_gbw_carries(const SegTileAgg* aggs, const int64_t* runs, int ntiles,
-                                                      int64_t* carry_in, uint32_t* tail_prefix, uint64_t* n_groups)
+                                                      int64_t* carry_in, uint64_t* n_groups)
 {
     VELO_TRACE_KERNEL(velo_site_hash("k_gbw_carries"));
     extern __shared__ __align__(16) char sm[];
-    GbTypesWide<NS>::Seg::carries(aggs, runs, ntiles, carry_in, tail_prefix, n_groups, sm);
+    GbTypesWide<NS>::Seg::carries(aggs, runs, ntiles, carry_in, n_groups, sm);
 }
 
 template <int NS>
@@ -238,11 +236,11 @@ __global__ void __launch_bounds__(SEG_THREADS) k_gb_summary(typename GbTypes<NS,
 
 template <int NS, int CNT>
 __global__ void __launch_bounds__(1024) k_gb_carries(const SegTileAgg* aggs, const int64_t* runs, int ntiles,
-                                                     int64_t* carry_in, uint32_t* tail_prefix, uint64_t* n_groups)
+                                                     int64_t* carry_in, uint64_t* n_groups)
 {
     VELO_TRACE_KERNEL(velo_site_hash("k_gb_carries"));
     extern __shared__ __align__(16) char sm[];
-    GbTypes<NS, CNT>::Seg::carries(aggs, runs, ntiles, carry_in, tail_prefix, n_groups, sm);
+    GbTypes<NS, CNT>::Seg::carries(aggs, runs, ntiles, carry_in, n_groups, sm);
 }
 
 template <int NS, int CNT>
@@ -320,15 +318,14 @@ __global__ void k_gbw_out(GbwWords g, size_t bound, int n_sums, int with_count, 
 }
 
 struct GbScratch {
-    uint64_t* r[4];      // sort records
-    uint64_t* g[5];      // group records
+    uint64_t* r[3];      // sort records
+    uint64_t* g[4];      // group records
     uint32_t* counts;
     uint32_t* prefix;
     uint64_t* n_grp_rows;
     SegTileAgg* aggs;
     int64_t* runs;
     int64_t* carry;
-    uint32_t* tail_prefix;
     uint64_t* n_groups;
     unsigned long long* rejected;
     size_t n_rec;
@@ -349,9 +346,9 @@ static GbScratch gb_layout(char* base, size_t n)
         off += align_up(bytes ? bytes : 1, 256);
         return p;
     };
-    for (int i = 0; i < 4; i++)
+    for (int i = 0; i < 3; i++)
         s.r[i] = reinterpret_cast<uint64_t*>(take(np * 8));
-    for (int i = 0; i < 5; i++)
+    for (int i = 0; i < 4; i++)
         s.g[i] = reinterpret_cast<uint64_t*>(take(np * 8));
     s.counts = reinterpret_cast<uint32_t*>(take(ntc * 4));
     s.prefix = reinterpret_cast<uint32_t*>(take((ntc + 1) * 4));
@@ -361,7 +358,6 @@ static GbScratch gb_layout(char* base, size_t n)
     // count and two sums)
     s.runs = reinterpret_cast<int64_t*>(take(nts * 3 * 8));
     s.carry = reinterpret_cast<int64_t*>(take(nts * 3 * 8));
-    s.tail_prefix = reinterpret_cast<uint32_t*>(take(nts * 4));
     s.n_groups = reinterpret_cast<uint64_t*>(take(8));
     s.rejected = reinterpret_cast<unsigned long long*>(take(8));
     s.bytes = off;
@@ -426,7 +422,7 @@ static velo_status gb_run(const GbScratch& s, const GbIn& in, size_t n, size_t b
     gc.mark_word = 0;
     k_gb_summary<NS, CNT><<<nts, SEG_THREADS, Seg::SMEM_IN, st>>>(rc, s.aggs, s.runs);
     k_gb_carries<NS, CNT><<<1, 1024, (NS + CNT) * 1024 * 8 + 2 * 1024 * 4, st>>>(s.aggs, s.runs, nts, s.carry,
-                                                                                 s.tail_prefix, s.n_groups);
+                                                                                 s.n_groups);
     k_gb_emit_rows<NS, CNT><<<nts, SEG_THREADS, Seg::SMEM, st>>>(rc, nts, s.aggs, s.carry, gc);
     VELO_CUDA_TRY(cudaGetLastError(), "group-by aggregation launch");
 
@@ -495,7 +491,7 @@ static velo_status gb_run_wide(const GbScratch& s, const GbIn& in, int with_coun
     gc.mark_word = 1;
     k_gbw_summary<NS><<<nts, SEG_THREADS, Seg::SMEM_IN, st>>>(rc, s.aggs, s.runs);
     k_gbw_carries<NS><<<1, 1024, (1 + NS) * 1024 * 8 + 2 * 1024 * 4, st>>>(s.aggs, s.runs, nts, s.carry,
-                                                                           s.tail_prefix, s.n_groups);
+                                                                           s.n_groups);
     k_gbw_emit_rows<NS><<<nts, SEG_THREADS, Seg::SMEM, st>>>(rc, nts, s.aggs, s.carry, gc);
     VELO_CUDA_TRY(cudaGetLastError(), "group-by aggregation launch");
     rc2 = launch_count_scan<typename T::Grp>(gc, m, logN, GB_LT, s.counts, s.prefix, s.n_grp_rows, st);

@@ -139,18 +139,16 @@ static velo_status reveal_words(const LiScratch& s, LkPlan& q, cudaStream_t st)
     VELO_CUDA_TRY(cudaStreamSynchronize(st), "cudaStreamSynchronize");
     if (next_pow2(rows ? rows : 1) > (size_t)1 << (q.logH - 1))
         return VELO_OK;
-    // tile counts and their scan in areas that no step of the group-by uses
-    uint32_t* counts = reinterpret_cast<uint32_t*>(s.runs);
-    uint32_t* prefix = reinterpret_cast<uint32_t*>(s.carry);
     const RowW::Cols c { q.ka };
-    const int lt = q.logH <= 20 ? 12 : 13;
-    velo_status rc = launch_count_scan<RowW>(c, q.h, q.logH, lt, counts, prefix, nullptr, st);
+    const int lt = q.logH <= 20 ? LK_COMPACT_LT : 13;
+    velo_status rc = launch_count_scan<RowW>(c, q.h, q.logH, lt, s.tile_counts, s.tile_prefix, nullptr, st);
     if (rc != VELO_OK)
         return rc;
     std::vector<NetPass> passes;
     plan_compact(q.logH, lt, 9, passes); // (8 or 16 words a segment)
     const NetGeom g(q.h, q.logH);
-    rc = lt == 12 ? launch_net<RowW, 8, 4>(c, g, passes, prefix, st) : launch_net<RowW, 8, 5>(c, g, passes, prefix, st);
+    rc = lt == LK_COMPACT_LT ? launch_net<RowW, 8, 4>(c, g, passes, s.tile_prefix, st)
+                             : launch_net<RowW, 8, 5>(c, g, passes, s.tile_prefix, st);
     if (rc == VELO_OK)
         lk_words(q, s, rows ? rows : 1, 12);
     return rc;

@@ -11,7 +11,6 @@
 
 namespace velo {
 
-constexpr int LI_LT = 12; // scratch is sized in 4096-row tiles
 // output values of a group: count, sum qty, sum price, sum price*(100-disc),
 // sum price*(100-disc)*(100+tax)
 constexpr int LI_V = 5;
@@ -32,13 +31,12 @@ constexpr int LK_TS = 4096;   // key words of a tile of the group search
 constexpr int LK_LMAX = 9;
 constexpr uint32_t LK_NONE = 0xFFFFu;
 
-// the words the later steps share (in the 256 bytes of LiScratch::d_rows)
+// the words the later steps share
 struct LkMeta {
     uint64_t rows;            // rows passing the filter
     uint64_t groups;          // distinct keys among them
     uint32_t slot[SEG_MAX_G]; // key + 1 of group j, 0 past the last group
 };
-static_assert(sizeof(LkMeta) <= 256, "fits the 256-byte aligned area of d_rows");
 
 __device__ __forceinline__ bool li_pass(const velo_lineitem_pred& p, int32_t q, int32_t d, int32_t s)
 {
@@ -367,62 +365,62 @@ __device__ __forceinline__ void li_sums_body(const LiCols& c, const velo_lineite
 }
 
 struct LiScratch {
-    uint64_t* w[3];
-    uint32_t* counts;
-    uint32_t* prefix;
-    uint64_t* d_rows;
-    SegTileAgg* aggs;
-    int64_t* runs;
-    int64_t* carry;
-    uint32_t* tail_prefix;
-    int64_t* tile_out;
-    uint64_t* n_groups;
+    uint32_t* ka;          // key words of step 1, 2^logH words
+    uint32_t* kb;          // merged key words, N words
+    uint32_t* cnt;         // first occurrences: low lanes, then high lanes of N / LK_TS tiles
+    uint32_t *n_pass, *n_ffff; // counts of the blocks of step 1
+    uint32_t *tile_counts, *tile_prefix; // marked words of a compaction's tiles and their scan
+    LkMeta* meta;
     size_t bytes;
-    size_t n_rec;
-    int ntiles_c;
-    int ntiles_s;
 };
 
-// Partition of the scratch buffer (offsets 256-byte aligned).
+constexpr int LK_MIN_LOGN = 13; // merged key words: at least the queue's tile
+constexpr int LK_COMPACT_LT = 12; // the smallest tile of a compaction
+
+// What a caller has to bring: the size for the 24-byte records and slot vectors
+// that the query used to move.  The steps need a sixth of it; budgets and
+// admission by this size stay what they are.
+inline size_t li_bytes(size_t n, uint32_t G)
+{
+    size_t rows = next_pow2(n);
+    rows = rows < 4096 ? 4096 : rows;
+    const size_t tiles = rows / SEG_TS;
+    auto area = [](size_t b) { return align_up(b, 256); };
+    return 3 * area(rows * 8) + area(rows / 2048 * 4) + area((rows / 2048 + 1) * 4) + 2 * area(8)
+        + area(tiles * sizeof(SegTileAgg)) + 2 * area(tiles * LI_V * 8) + area(tiles * 4)
+        + area(tiles * G * (1 + LI_V) * 8);
+}
+
+// Partition of the scratch buffer (offsets 256-byte aligned); every area sized
+// for the largest geometry that lk_words makes of n rows
 inline LiScratch li_layout(char* base, size_t n, uint32_t G)
 {
     LiScratch s {};
-    const size_t np = next_pow2(n);
-    size_t n_rec = np;
-    if (n_rec < (size_t)SEG_TS)
-        n_rec = SEG_TS;
-    if (n_rec < ((size_t)1 << LI_LT))
-        n_rec = (size_t)1 << LI_LT;
-    s.n_rec = n_rec;
-    s.ntiles_c = (int)(n_rec >> LI_LT);
-    s.ntiles_s = (int)(n_rec / SEG_TS);
+    const size_t h = (n + 1) / 2;
+    const size_t ph = next_pow2(h);
+    const size_t N = ph < ((size_t)1 << LK_MIN_LOGN) ? (size_t)1 << LK_MIN_LOGN : ph;
+    const size_t nblk = (h + LK_ROWS - 1) / LK_ROWS;
+    const size_t ctiles = (ph >> LK_COMPACT_LT) + 1;
     size_t off = 0;
-    auto take = [&](size_t bytes) {
+    auto take = [&](size_t words) {
         char* p = base ? base + off : nullptr;
-        off += align_up(bytes, 256);
-        return p;
+        off += align_up(words * 4, 256);
+        return reinterpret_cast<uint32_t*>(p);
     };
-    for (int i = 0; i < 3; i++)
-        s.w[i] = reinterpret_cast<uint64_t*>(take(n_rec * 8));
-    // room for the tile counts of 2^(LI_LT-1)-row tiles: the persistent
-    // command queue compacts three-word records in 2048-row tiles
-    const size_t cnt_tiles = n_rec >> (LI_LT - 1);
-    s.counts = reinterpret_cast<uint32_t*>(take(cnt_tiles * 4));
-    s.prefix = reinterpret_cast<uint32_t*>(take((cnt_tiles + 1) * 4));
-    s.d_rows = reinterpret_cast<uint64_t*>(take(8));
-    s.aggs = reinterpret_cast<SegTileAgg*>(take((size_t)s.ntiles_s * sizeof(SegTileAgg)));
-    s.runs = reinterpret_cast<int64_t*>(take((size_t)s.ntiles_s * LI_V * 8));
-    s.carry = reinterpret_cast<int64_t*>(take((size_t)s.ntiles_s * LI_V * 8));
-    s.tail_prefix = reinterpret_cast<uint32_t*>(take((size_t)s.ntiles_s * 4));
-    s.tile_out = reinterpret_cast<int64_t*>(take((size_t)s.ntiles_s * G * (1 + LI_V) * 8));
-    s.n_groups = reinterpret_cast<uint64_t*>(take(8));
-    s.bytes = off;
+    s.ka = take(ph);
+    s.kb = take(N);
+    s.cnt = take(2 * (N / LK_TS));
+    s.n_pass = take(nblk);
+    s.n_ffff = take(nblk);
+    s.tile_counts = take(ctiles);
+    s.tile_prefix = take(ctiles + 1);
+    s.meta = reinterpret_cast<LkMeta*>(take((sizeof(LkMeta) + 3) / 4));
+    const size_t size = li_bytes(n, G);
+    s.bytes = off > size ? off : size;
     return s;
 }
 
-// Geometry and scratch of one query with key tiles of 2^lt words: the key words
-// in w[0], the merged ones from w[1] on (w[1] and w[2] are adjacent and hold 16
-// bytes a row of at least 4096 rows); the counts in the tile arrays.
+// Geometry and scratch of one query with key tiles of 2^lt words
 struct LkPlan {
     size_t h; // key words
     int logH;
@@ -434,7 +432,8 @@ struct LkPlan {
     LkMeta* meta;
 };
 
-// the key words that are sorted: h of them
+// the key words that are sorted: h of them, merged in tiles of 2^lt words
+// (lt <= LK_MIN_LOGN)
 inline void lk_words(LkPlan& q, const LiScratch& s, size_t h, int lt)
 {
     q.h = h;
@@ -442,8 +441,8 @@ inline void lk_words(LkPlan& q, const LiScratch& s, size_t h, int lt)
     q.logN = q.logH < lt ? lt : q.logH;
     q.N = (size_t)1 << q.logN;
     q.ntiles = (int)(q.N / LK_TS);
-    q.cnt0 = s.counts;
-    q.cnt1 = s.counts + q.ntiles;
+    q.cnt0 = s.cnt;
+    q.cnt1 = s.cnt + q.ntiles;
 }
 
 inline LkPlan lk_plan(const LiScratch& s, size_t n, int lt, unsigned max_blocks)
@@ -452,11 +451,11 @@ inline LkPlan lk_plan(const LiScratch& s, size_t n, int lt, unsigned max_blocks)
     lk_words(q, s, (n + 1) / 2, lt);
     const size_t want = (q.h + LK_ROWS - 1) / LK_ROWS;
     q.nblk = want < max_blocks ? (unsigned)want : max_blocks;
-    q.ka = reinterpret_cast<uint32_t*>(s.w[0]);
-    q.kb = reinterpret_cast<uint32_t*>(s.w[1]);
-    q.n_pass = s.prefix;
-    q.n_ffff = s.tail_prefix;
-    q.meta = reinterpret_cast<LkMeta*>(s.d_rows);
+    q.ka = s.ka;
+    q.kb = s.kb;
+    q.n_pass = s.n_pass;
+    q.n_ffff = s.n_ffff;
+    q.meta = s.meta;
     return q;
 }
 

@@ -85,11 +85,11 @@ __global__ void __launch_bounds__(SEG_THREADS) k_jseg_summary(JRec::Cols c, SegT
 }
 
 __global__ void __launch_bounds__(1024) k_jseg_carries(const SegTileAgg* aggs, const int64_t* runs, int ntiles,
-                                                       int64_t* carry_in, uint32_t* tail_prefix, uint64_t* n_groups)
+                                                       int64_t* carry_in, uint64_t* n_groups)
 {
     VELO_TRACE_KERNEL(velo_site_hash("k_jseg_carries"));
     extern __shared__ __align__(16) char sm[];
-    JSeg::carries(aggs, runs, ntiles, carry_in, tail_prefix, n_groups, sm);
+    JSeg::carries(aggs, runs, ntiles, carry_in, n_groups, sm);
 }
 
 __global__ void __launch_bounds__(SEG_THREADS, 5) k_jseg_emit_topk(JRec::Cols c, int ntiles, const SegTileAgg* aggs,
@@ -196,7 +196,7 @@ static velo_status join_records(const JoinScratch& s, const velo_join_tables* t,
     const int nts = (int)(s.n_rec / SEG_TS);
     k_jseg_summary<<<nts, SEG_THREADS, JSeg::SMEM_IN, st>>>(uc, s.aggs, s.runs);
     k_jseg_carries<<<1, 1024, JoinAgg::V * 1024 * 8 + 2 * 1024 * 4, st>>>(s.aggs, s.runs, nts, s.carry,
-                                                                            s.tail_prefix, s.n_groups);
+                                                                            s.n_groups);
     const size_t topk_smem = cand == 16 ? JSEG_TOPK16_SMEM : JSEG_TOPK_SMEM;
     k_jseg_emit_topk<<<nts, SEG_THREADS, topk_smem, st>>>(uc, nts, s.aggs, s.carry, cand, s.cand[0], s.cand[1]);
     VELO_CUDA_TRY(cudaGetLastError(), "join group-by launch");
@@ -232,8 +232,7 @@ static velo_status join_rows(const JoinScratch& s, const velo_join_tables* t, co
     const int nt = (int)((n + JK_TS - 1) / JK_TS);
     const int nts = (int)next_pow2((size_t)nt);
     k_jk_summary<<<nt, JK_THREADS, 0, st>>>(k, p, n, s.aggs, s.runs);
-    k_jseg_carries<<<1, 1024, JoinAgg::V * 1024 * 8 + 2 * 1024 * 4, st>>>(s.aggs, s.runs, nt, s.carry, s.tail_prefix,
-                                                                            s.unused);
+    k_jseg_carries<<<1, 1024, JoinAgg::V * 1024 * 8 + 2 * 1024 * 4, st>>>(s.aggs, s.runs, nt, s.carry, s.unused);
     k_jk_emit_topk<<<nts, JK_THREADS, cand == 16 ? JK_EMIT16_SMEM : JK_EMIT_SMEM, st>>>(
         k, p, n, nt, s.aggs, s.carry, cand, s.cand[0], s.cand[1], s.n_groups, s.n_joined);
     VELO_CUDA_TRY(cudaGetLastError(), "join group-by launch");

@@ -35,7 +35,6 @@ struct JoinAgg {
         v[0] = ok ? (int64_t)w[1] : 0;
         v[1] = ok ? 1 : 0;
     }
-    __device__ __forceinline__ static int64_t out_key_from(uint64_t key) { return (int64_t)(key >> 32); }
     __device__ __forceinline__ static uint64_t out_bits(uint64_t key) { return key >> 32; }
 };
 using JSeg = SegAgg<JoinAgg>;
@@ -624,7 +623,6 @@ struct JoinScratch {
     SegTileAgg* aggs;
     int64_t* runs;
     int64_t* carry;
-    uint32_t* tail_prefix;
     uint64_t* n_groups;
     uint64_t* unused; // the group count of the carry scan, which the 12-byte form does not use
     size_t bytes, n_rec;
@@ -658,7 +656,6 @@ inline JoinScratch join_layout(char* base, size_t nd, size_t nf)
     s.aggs = reinterpret_cast<SegTileAgg*>(take(nts * sizeof(SegTileAgg)));
     s.runs = reinterpret_cast<int64_t*>(take(nts * JoinAgg::V * 8));
     s.carry = reinterpret_cast<int64_t*>(take(nts * JoinAgg::V * 8));
-    s.tail_prefix = reinterpret_cast<uint32_t*>(take(nts * 4));
     s.n_groups = reinterpret_cast<uint64_t*>(take(8));
     s.unused = base ? s.n_groups + 1 : nullptr; // in the 256 bytes of n_groups
     s.bytes = off;

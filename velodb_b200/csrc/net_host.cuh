@@ -79,6 +79,35 @@ inline velo_status ensure_smem(Kern kern, size_t bytes, int (&done)[64])
     return VELO_OK;
 }
 
+// The networks that a row type runs in a tile shape; launch_net compiles the
+// kernels of these alone.
+template <class R, int LOG_NT, int LOG_E>
+struct NetUse {
+    static constexpr bool sort = true, compact = true;
+};
+// 12-byte rows: compacted by the gather in one shape, key-ordered ones never
+template <int CM, int LOG_NT, int LOG_E>
+struct NetUse<RowK12<CM>, LOG_NT, LOG_E> {
+    static constexpr bool sort = true, compact = CM == K12_ALL && LOG_NT == 8 && LOG_E == 4;
+};
+// strict records are sorted alone
+template <int W, int KW, int KM, int LOG_NT, int LOG_E>
+struct NetUse<RowRec<W, KW, true, KM>, LOG_NT, LOG_E> {
+    static constexpr bool sort = true, compact = false;
+};
+template <int LOG_NT, int LOG_E>
+struct NetUse<RowU2, LOG_NT, LOG_E> {
+    static constexpr bool sort = true, compact = false;
+};
+template <int LOG_NT, int LOG_E>
+struct NetUse<RowW, LOG_NT, LOG_E> {
+    static constexpr bool sort = false, compact = true;
+};
+template <int LOG_NT, int LOG_E>
+struct NetUse<RowKPM, LOG_NT, LOG_E> {
+    static constexpr bool sort = false, compact = true;
+};
+
 // Launches `passes` (all bitonic or all ORCompact kinds) over the tiles; one
 // kernel launch per pass.  Defined in net_impl.cuh and explicitly
 // instantiated per row type and tile configuration (net_inst_*.cu).

@@ -17,22 +17,16 @@ namespace velo {
 // against 0.22 ms, 2^23 1.65 ms against 1.45 ms).
 template <class R, int LOG_NT>
 constexpr int net_min_blocks() { return LOG_NT <= 8 ? 2 : 1; }
-// rows of at most 12 bytes, and two-word records keyed on 32 bits (the
-// group-by's: 2^23-row sort 1.78 -> 1.63 ms), in both the in-tile and the
-// global kernels.  Two-word records compared on a whole word (the join's
-// union) only in the global kernel and the merge kernel: their tile sort
-// needs 128 registers (2^23 union sort: tile 353 -> 390 us at 85), while
-// their global passes (56.4 -> 53.2 us a pass) and merges (73.9 -> 71.6 us)
-// gain from the third CTA.
+// rows of at most 12 bytes, in both the in-tile and the global kernels.
+// Two-word records compared on a whole word (the join's record form, GROUP BY)
+// or on 96 bits (ORDER BY) only in the global kernel and the merge kernel: their
+// tile sort needs 128 registers (2^23 rows on a whole word: tile 353 -> 390 us at
+// 85), while their global passes (56.4 -> 53.2 us a pass) and merges (73.9 ->
+// 71.6 us) gain from the third CTA.
 template <class R>
 struct NetWide {
     static constexpr bool ok = sizeof(R) <= 12;
     static constexpr bool ok_global = ok;
-};
-template <bool S>
-struct NetWide<RowRec<2, 1, S, KEY_HI32>> {
-    static constexpr bool ok = true;
-    static constexpr bool ok_global = true;
 };
 template <bool S>
 struct NetWide<RowRec<2, 1, S, KEY_FULL>> {
@@ -159,7 +153,7 @@ constexpr bool tma_capable()
 #ifdef VELO_TRACE
     return false;
 #else
-    return TmaRows<R>::ok && Stage<R>::ok && LOG_NT + LOG_E >= 12;
+    return NetUse<R, LOG_NT, LOG_E>::sort && TmaRows<R>::ok && Stage<R>::ok && LOG_NT + LOG_E >= 12;
 #endif
 }
 // ... and are switched on (velo_set_tensor_tile_loads), and the word arrays
@@ -223,26 +217,35 @@ velo_status launch_net(const typename R::Cols& c, const NetGeom& g, const std::v
     constexpr int MBG = net_has_wide_global<R, LOG_NT>() ? 3 : MB;
     const bool wide = MBW != MB && g.logN >= NET_WIDE_LOGN;
     const bool wide_g = MBG != MB && g.logN >= NET_WIDE_LOGN;
-    auto k_local = wide ? k_sort_pass<R, LOG_NT, LOG_E, N::PK_LOCAL, MBW> : k_sort_pass<R, LOG_NT, LOG_E, N::PK_LOCAL, MB>;
+    using Use = NetUse<R, LOG_NT, LOG_E>;
+    using Kern = void (*)(typename R::Cols, NetGeom, NetPass, const uint32_t*);
+    Kern k_local = nullptr, k_merge = nullptr, k_global = nullptr, k_comp = nullptr, k_comp_g = nullptr;
     // record sorts run their in-tile merges as a kernel of their own, compiled
-    // without the tile-sort code: join union merges 76.5 -> 73.8 us, group-by
-    // merges 65.6 -> 62.1 us; key-payload rows keep the shared kernel (2^24
-    // merges 111.1 -> 112.9 us with the split)
+    // without the tile-sort code: two-word merges 76.5 -> 73.8 us; 12-byte rows
+    // keep the shared kernel (2^24 merges 111.1 -> 112.9 us with the split)
     constexpr bool split_merge = sizeof(R) != 12;
-    // the merges of records that keep a two-CTA tile sort (compared on a
-    // whole word) take the global kernel's three-CTA budget from 2^21 rows:
-    // 80 registers, a few spilled, join union merges 73.9 -> 71.6 us
-    auto k_merge = !split_merge ? k_local
-        : wide                  ? k_sort_pass<R, LOG_NT, LOG_E, N::PK_MERGE, MBW>
-        : wide_g                ? k_sort_pass<R, LOG_NT, LOG_E, N::PK_MERGE, MBG>
-                                : k_sort_pass<R, LOG_NT, LOG_E, N::PK_MERGE, MB>;
-    auto k_global = wide_g ? k_sort_pass<R, LOG_NT, LOG_E, N::PK_GLOBAL, MBG>
-                           : k_sort_pass<R, LOG_NT, LOG_E, N::PK_GLOBAL, MB>;
+    if constexpr (Use::sort) {
+        k_local = wide ? k_sort_pass<R, LOG_NT, LOG_E, N::PK_LOCAL, MBW> : k_sort_pass<R, LOG_NT, LOG_E, N::PK_LOCAL, MB>;
+        k_merge = k_local;
+        // the merges of records that keep a two-CTA tile sort (compared on a
+        // whole word) take the global kernel's three-CTA budget from 2^21 rows:
+        // 80 registers, a few spilled, 73.9 -> 71.6 us
+        if constexpr (split_merge)
+            k_merge = wide ? k_sort_pass<R, LOG_NT, LOG_E, N::PK_MERGE, MBW>
+                : wide_g   ? k_sort_pass<R, LOG_NT, LOG_E, N::PK_MERGE, MBG>
+                           : k_sort_pass<R, LOG_NT, LOG_E, N::PK_MERGE, MB>;
+        k_global = wide_g ? k_sort_pass<R, LOG_NT, LOG_E, N::PK_GLOBAL, MBG>
+                          : k_sort_pass<R, LOG_NT, LOG_E, N::PK_GLOBAL, MB>;
+    }
     // ORCompact's tile pass and fused global passes are separate kernels too,
-    // each compiled without the other's code: join compaction tile pass
+    // each compiled without the other's code: 2^23 two-word records, tile pass
     // 98.3 -> 94.2 us, global passes 69.6 -> 65.0 us
-    auto k_comp = k_compact_pass<R, LOG_NT, LOG_E, N::PK_LOCAL>;
-    auto k_comp_g = k_compact_pass<R, LOG_NT, LOG_E, N::PK_GLOBAL>;
+    if constexpr (Use::compact) {
+        k_comp = k_compact_pass<R, LOG_NT, LOG_E, N::PK_LOCAL>;
+        k_comp_g = k_compact_pass<R, LOG_NT, LOG_E, N::PK_GLOBAL>;
+    }
+    if (compact ? !Use::compact : !Use::sort)
+        return einval("a network this row type does not run");
     const size_t smem = compact ? N::smem_bytes_compact() : N::smem_bytes_sort();
     if (smem > MAX_SMEM_BYTES)
         return einval("tile configuration needs more shared memory than a CTA can have");

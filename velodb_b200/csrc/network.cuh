@@ -120,10 +120,6 @@ struct MarkAt<RowK12<CM>> {
     }
 };
 template <>
-struct MarkAt<RowU2> {
-    __device__ __forceinline__ static bool get(const RowU2::Cols&, size_t) { return false; }
-};
-template <>
 struct MarkAt<RowW> {
     __device__ __forceinline__ static bool get(const RowW::Cols& c, size_t g)
     {

@@ -134,7 +134,6 @@ struct SegFlagInCount<A, std::void_t<decltype(A::FLAG_IN_COUNT)>> {
 //      static uint64_t key(const uint64_t* w)      -- run key (includes validity)
 //      static bool valid(const uint64_t* w)
 //      static void values(const uint64_t* w, int64_t (&v)[V], const Params&)  -- zero when invalid
-//      static int64_t out_key_from(uint64_t key)
 template <class Agg>
 struct SegAgg {
     static constexpr int W = Agg::W;
@@ -238,7 +237,7 @@ struct SegAgg {
 
     // pass B: one CTA of 1024 threads
     __device__ static void carries(const SegTileAgg* aggs, const int64_t* tail_runs, int ntiles, int64_t* carry_in,
-                                   uint32_t* tail_prefix, uint64_t* n_groups, char* smem)
+                                   uint64_t* n_groups, char* smem)
     {
         // Rounds of blockDim.x consecutive tiles (coalesced loads, all issued
         // at once), each a block-wide segmented scan chained to the previous
@@ -246,7 +245,6 @@ struct SegAgg {
         //   run_out(t) = tail_runs[t] + (t continues t-1's run and is one run
         //                ? run_out(t-1) : 0)       (the run crossing t's end)
         //   carry_in[t] = t's first run continues t-1's last ? run_out(t-1) : 0
-        //   tail_prefix[t] = groups ending in tiles before t
         const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
         int64_t* wv = reinterpret_cast<int64_t*>(smem);                 // [V][32] warp prefixes
         uint32_t* wc = reinterpret_cast<uint32_t*>(smem + (size_t)V * 32 * 8);  // [32]
@@ -335,20 +333,17 @@ struct SegAgg {
                 for (int i = 0; i < V; i++)
                     ez[i] = __shfl_up_sync(0xFFFFFFFFu, z[i], 1);
                 int eg = __shfl_up_sync(0xFFFFFFFFu, g ? 1 : 0, 1);
-                uint32_t ed = __shfl_up_sync(0xFFFFFFFFu, d, 1);
                 if (lane == 0) {
 #pragma unroll
                     for (int i = 0; i < V; i++)
                         ez[i] = 0;
                     eg = 0;
-                    ed = 0;
                 }
                 __syncwarp();
                 if (lane < nw) {
 #pragma unroll
                     for (int i = 0; i < V; i++)
                         wv[i * 32 + lane] = eg ? ez[i] : run_prev[i] + ez[i];
-                    wc[lane] = cnt_prev + ed;
                 }
                 if (lane == nw - 1) {
 #pragma unroll
@@ -367,13 +362,11 @@ struct SegAgg {
                 if (lane == 0)
                     pr[i] = wp; // run_out(t - 1)
             }
-            const uint32_t cin = wc[warp] + c - cnt;
             if (in) {
                 VELO_TRACE_AT(TS_SEG_META, carry_in + (size_t)t * V);
 #pragma unroll
                 for (int i = 0; i < V; i++)
                     carry_in[(size_t)t * V + i] = joins ? pr[i] : 0;
-                tail_prefix[t] = cin;
             }
 #pragma unroll
             for (int i = 0; i < V; i++)
