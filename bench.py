@@ -83,13 +83,6 @@ def hbm_peak():
 PIPE_LMAX = 8
 
 
-def sorted_rows(n: int) -> dict:
-    """Rows the passes of a sort of n rows work on, by log2 of the padded size:
-    whole 4096-row tiles, the padding past the last one left out."""
-    return {max(0, (n - 1).bit_length()): -(-n // 4096) * 4096}
-
-
-
 def sort_passes(logn: int, lt: int, lmax: int) -> int:
     p = 1
     for k in range(lt + 1, logn + 1):
@@ -190,7 +183,6 @@ class JoinTopK:
         self.in_bytes = sum(v.numel() * v.element_size() for v in self.pinned.values())
         self.np_rows = 1 << int(np.ceil(np.log2(self.n)))
         self.rec_bytes = 12
-        self.pass_rows = sorted_rows(self.n)
         self.flush_l2 = False  # inputs (84 MB) plus union rows (90 MB) exceed the 126 MB L2
         self.kernel = ("k_sort_pass<RowKP,8,4,PK,3> (union sort: 7.5 M 12-byte rows, 4096-row tiles, three CTAs "
                        "per SM)")
@@ -306,7 +298,6 @@ class GroupBy:
         self.in_bytes = sum(v.numel() * v.element_size() for v in self.pinned.values())
         self.np_rows = 1 << int(np.ceil(np.log2(self.n)))
         self.rec_bytes = 4  # a pair of 16-bit group keys
-        self.pass_rows = sorted_rows((self.n + 1) // 2)
         self.flush_l2 = False  # inputs (156 MB) exceed the 126 MB L2
         self.kernel = "k_sort_pass<RowU2,8,5,PK> (sort stage: 3 M pairs of 16-bit keys, 8192-word tiles)"
 
@@ -609,16 +600,12 @@ def warm(torch, fn, warmup, min_s=SOAK_S):
 PASS_KINDS = ("tile_sort", "merge", "global", "compact_tile", "compact_global")
 
 
-def pass_roofline(torch, capi, run, peak, reps=3, reset=None, pass_rows=None):
+def pass_roofline(torch, capi, run, peak, reps=3, reset=None):
     """Every network pass of `run` timed on its own (the library's pass timer:
     CUDA events around each pass, on the pass's stream) and grouped by pass
-    kind.  Algorithmic bytes of a pass: every row it works on read and written
-    once, 2 x rows x row bytes (pass_rows: rows by log2 of the padded size where
-    the sorts leave padding out)."""
-    def bytes_of(kind, lg, rb):
-        trimmed = (pass_rows or {}).get(lg) if kind in ("tile_sort", "merge", "global") else None
-        return 2 * (trimmed or 1 << lg) * rb
-
+    kind.  Algorithmic bytes of a pass: the rows it reads and the rows it writes
+    (the pass timer's counts: padding that a pass leaves out is not among them)
+    times the bytes of a row."""
     rows = []
     for _ in range(reps):
         if reset is not None:
@@ -628,12 +615,13 @@ def pass_roofline(torch, capi, run, peak, reps=3, reset=None, pass_rows=None):
         try:
             run()
             torch.cuda.synchronize()
-            rows.extend(capi.last_pass_times())
+            rows.extend((k, lg, (r + w) * rb, ms)
+                        for (k, lg, rb, ms), (r, w) in zip(capi.last_pass_times(), capi.last_pass_rows()))
         finally:
             capi.set_pass_timing(False)
     out = {}
     for kind in PASS_KINDS:
-        xs = [(bytes_of(k, lg, rb), ms) for (k, lg, rb, ms) in rows if k == kind and ms > 0]
+        xs = [(b, ms) for (k, _, b, ms) in rows if k == kind and ms > 0]
         if not xs:
             continue
         byt = sum(b for b, _ in xs)
@@ -643,13 +631,13 @@ def pass_roofline(torch, capi, run, peak, reps=3, reset=None, pass_rows=None):
                      "achieved_gbs": byt / (t / 1e3) / 1e9, "frac": byt / (t / 1e3) / 1e9 / peak,
                      "min_frac": min(fr), "max_frac": max(fr)}
     # the dominant sort: the sort passes of the largest padded size
-    sorts = [(lg, rb, ms) for (k, lg, rb, ms) in rows if k in ("tile_sort", "merge", "global") and ms > 0]
+    sorts = [(lg, b, ms) for (k, lg, b, ms) in rows if k in ("tile_sort", "merge", "global") and ms > 0]
     dom = None
     if sorts:
         lg_max = max(lg for lg, _, _ in sorts)
-        xs = [(bytes_of("merge", lg, rb), ms) for lg, rb, ms in sorts if lg == lg_max]
+        xs = [(b, ms) for lg, b, ms in sorts if lg == lg_max]
         dom = {"launches_per_step": len(xs) // reps, "avg_launch_us": sum(m for _, m in xs) / len(xs) * 1e3,
-               "algorithmic_bytes_per_launch": xs[0][0], "log2_rows": lg_max}
+               "algorithmic_bytes_per_launch": sum(b for b, _ in xs) / len(xs), "log2_rows": lg_max}
     return out, dom
 
 
@@ -785,7 +773,7 @@ def roofline_of(torch, capi, wl, peak, peak_kind):
 
         def run():
             wl.capi.osort_kp(wl.k, wl.p, wl.n)
-    kinds, dom = pass_roofline(torch, capi, run, peak, reset=reset, pass_rows=getattr(wl, "pass_rows", None))
+    kinds, dom = pass_roofline(torch, capi, run, peak, reset=reset)
     if dom is None:
         return None
     achieved = dom["algorithmic_bytes_per_launch"] / (dom["avg_launch_us"] / 1e6) / 1e9

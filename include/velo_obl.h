@@ -132,6 +132,10 @@ void velo_set_tensor_tile_loads(int on);
 int velo_tensor_tile_status(void);
 void velo_pass_times_clear(void);
 int velo_last_pass_times(velo_pass_time* out, int capacity);
+/* Rows read and rows written by each of those passes, in the same order: two
+ * numbers a pass, `capacity` passes at most (a pass over fewer than 2^log_n rows
+ * leaves padding out). */
+int velo_last_pass_rows(uint64_t* out, int capacity);
 
 /* ------------------------------------------------------------------------ */
 /* Bitonic network sort                                                     */

@@ -235,3 +235,33 @@ def test_sort_columns_order_by_known_answers(cuda, orc):
         torch.cuda.synchronize()
         outs = [t.cpu().numpy().view(np.asarray(c).dtype)[:n] for t, c in zip(dcols, cols)]
         assert check(outs, idx.cpu().numpy()[:n])
+
+
+def passes_of(fn):
+    """(kind, log2 rows, rows read, rows written) of the call's network passes."""
+    capi.set_pass_timing(True)
+    try:
+        capi.clear_pass_times()
+        fn()
+        return [(k, lg, r, w) for (k, lg, _, _), (r, w) in zip(capi.last_pass_times(), capi.last_pass_rows())]
+    finally:
+        capi.set_pass_timing(False)
+
+
+def test_pass_rows_leave_out_padding(cuda):
+    # 300,001 rows: 74 tiles of 4096; the tile pass writes padding up to 2^19
+    n, cap = 300_001, 1 << 19
+    k, p, m = (torch.zeros(cap, dtype=t, device="cuda") for t in (torch.int64, torch.int32, torch.uint8))
+    got = passes_of(lambda: capi.osort_kp(k, p, n))
+    assert got[0] == ("tile_sort", 19, n, cap)
+    assert len(got) > 8 and all(x[1:] == (19, 74 * 4096, 74 * 4096) for x in got[1:])
+    got = passes_of(lambda: capi.ocompact_kpm(k, p, m, n))
+    assert got == [("compact_tile", 19, n, cap), ("compact_global", 19, cap, cap)]
+    # the group keys, two a word, in 8192-word tiles; the last merge works on all 2^22
+    n = 6_001_215
+    d = capi.lineitem_to_device(W.lineitem())
+    h, tiles = (n + 1) // 2, -(-n // 16384)
+    got = passes_of(lambda: capi.filter_groupby(d, n, W.LINEITEM_PRED, 8))
+    assert got[0] == ("tile_sort", 22, h, tiles * 8192)
+    assert got[-2:] == [("global", 22, 1 << 22, 1 << 22), ("merge", 22, 1 << 22, 1 << 22)]
+    assert all(x[2:] == (tiles * 8192, tiles * 8192) for x in got[1:-2])

@@ -24,6 +24,7 @@ PROTOS = {
     "velo_tensor_tile_status": (i32, []),
     "velo_pass_times_clear": (None, []),
     "velo_last_pass_times": (i32, [vp, i32]),
+    "velo_last_pass_rows": (i32, [vp, i32]),
     "velo_trace_enabled": (i32, []),
     "velo_trace_begin": (i32, [u64, u64]),
     "velo_trace_end": (i32, [vp, vp, vp, u64, vp]),

@@ -80,6 +80,13 @@ def last_pass_times() -> list:
              float(buf[i].ms)) for i in range(n)]
 
 
+def last_pass_rows() -> list:
+    """(rows read, rows written) of the same passes (velo_last_pass_rows)."""
+    buf = np.zeros((1024, 2), dtype=np.uint64)
+    n = int(lib().velo_last_pass_rows(buf.ctypes.data, 1024))
+    return [(int(r), int(w)) for r, w in buf[:n]]
+
+
 def to_dev_u64(a: np.ndarray, capacity: int | None = None, device="cuda") -> torch.Tensor:
     """Upload a uint64 array into an int64 device tensor of `capacity` rows."""
     cap = len(a) if capacity is None else capacity

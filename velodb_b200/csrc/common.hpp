@@ -86,7 +86,7 @@ void store_stage_times(const float* ms, int n);
 bool pass_timing_on();
 // merge passes with bulk-copy prefetch (velo_set_merge_pipeline)
 bool merge_pipe_on();
-void store_pass_time(int kind, int log_n, int row_bytes, float ms);
+void store_pass_time(int kind, int log_n, int row_bytes, float ms, uint64_t rows_read, uint64_t rows_written);
 
 class StageTimer {
 public:

@@ -118,14 +118,16 @@ public:
         if (on_)
             cudaEventRecord(ev_[i + 1], st_);
     }
-    void finish(const std::vector<NetPass>& passes, int log_n, int row_bytes)
+    void finish(const std::vector<NetPass>& passes, const NetGeom& g, int lt, int row_bytes)
     {
         if (!on_ || cudaEventSynchronize(ev_.back()) != cudaSuccess)
             return;
         for (size_t i = 0; i < passes.size(); i++) {
             float ms = 0.f;
             cudaEventElapsedTime(&ms, ev_[i], ev_[i + 1]);
-            store_pass_time(passes[i].kind, log_n, row_bytes, ms);
+            size_t read, written;
+            net_pass_rows(g, passes[i], lt, &read, &written);
+            store_pass_time(passes[i].kind, g.logN, row_bytes, ms, read, written);
         }
     }
     ~PassTimer()
@@ -326,7 +328,7 @@ velo_status launch_net(const typename R::Cols& c, const NetGeom& g, const std::v
         }
         timer.mark(i);
     }
-    timer.finish(passes, g.logN, RowBytes<R>::value);
+    timer.finish(passes, g, lt, RowBytes<R>::value);
     return VELO_OK;
 }
 

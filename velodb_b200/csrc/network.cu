@@ -113,14 +113,18 @@ extern "C" int velo_last_stage_times(float* ms, int capacity)
 static std::atomic<int> g_pass_timing { 0 };
 constexpr int PASS_LOG_CAP = 1024;
 static thread_local velo_pass_time g_pass_log[PASS_LOG_CAP];
+static thread_local uint64_t g_pass_rows[2 * PASS_LOG_CAP];
 static thread_local int g_pass_n = 0;
 
 bool velo::pass_timing_on() { return g_pass_timing.load(std::memory_order_relaxed) != 0; }
 
-void velo::store_pass_time(int kind, int log_n, int row_bytes, float ms)
+void velo::store_pass_time(int kind, int log_n, int row_bytes, float ms, uint64_t rows_read, uint64_t rows_written)
 {
-    if (g_pass_n < PASS_LOG_CAP)
-        g_pass_log[g_pass_n++] = velo_pass_time { (uint32_t)kind, (uint32_t)log_n, (uint32_t)row_bytes, ms };
+    if (g_pass_n >= PASS_LOG_CAP)
+        return;
+    g_pass_rows[2 * g_pass_n] = rows_read;
+    g_pass_rows[2 * g_pass_n + 1] = rows_written;
+    g_pass_log[g_pass_n++] = velo_pass_time { (uint32_t)kind, (uint32_t)log_n, (uint32_t)row_bytes, ms };
 }
 
 extern "C" void velo_set_pass_timing(int on)
@@ -234,6 +238,14 @@ extern "C" int velo_last_pass_times(velo_pass_time* out, int capacity)
     const int n = capacity < g_pass_n ? capacity : g_pass_n;
     for (int i = 0; out && i < n; i++)
         out[i] = g_pass_log[i];
+    return out ? n : g_pass_n;
+}
+
+extern "C" int velo_last_pass_rows(uint64_t* out, int capacity)
+{
+    const int n = capacity < g_pass_n ? capacity : g_pass_n;
+    for (int i = 0; out && i < 2 * n; i++)
+        out[i] = g_pass_rows[i];
     return out ? n : g_pass_n;
 }
 

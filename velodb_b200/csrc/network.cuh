@@ -108,6 +108,16 @@ __host__ __device__ inline size_t net_pass_tiles(const NetGeom& g, const NetPass
     return round_up_log2(m, p.kind == P_SORT_GLOBAL ? p.b_hi + 1 : lt) >> lt;
 }
 
+// Rows that pass `p` reads and writes (tiles as above)
+inline void net_pass_rows(const NetGeom& g, const NetPass& p, int lt, size_t* read, size_t* written)
+{
+    const size_t rows = g.logN <= lt ? (size_t)1 << g.logN : net_pass_tiles(g, p, lt) << lt;
+    const bool first = p.kind == P_SORT_TILE || p.kind == P_COMPACT_TILE;
+    const size_t in = first ? g.n : g.m;
+    *read = rows < in ? rows : in;
+    *written = first || rows < g.m ? rows : g.m;
+}
+
 // mark of the row stored at global index g (count pass)
 template <class R>
 struct MarkAt;
