@@ -58,9 +58,9 @@ FALLBACK_HBM_GBS = 6650.0
 METRIC = "obliv sort & join Mrows/s (frac of HBM peak); p50/p99 latency served vs plain"
 
 # DRAM bytes (read + write) per launch of the dominant kernel from one ncu
-# capture of the same pipeline (the mean over its sort passes), or None when
-# no capture of that launch exists.
-TRAFFIC = {"groupby": None, "sort": 12.65e6, "join": None, "batch": None}
+# capture of the same pipeline (the mean of a tile sort, a global pass and a
+# merge of its sort), or None when no capture of that launch exists.
+TRAFFIC = {"groupby": 12.06e6, "sort_2^20": 12.65e6, "sort_2^24": 343.8e6, "join": 121.4e6}
 
 # warm-up runs at least this long (seconds) so that the clock samples taken
 # from the end of the warm-up through the timed steps show the GPU under load
@@ -756,7 +756,9 @@ def measure(torch, capi, wl, args, world, device, peak, peak_kind, with_e2e=True
         res["e2e"] = e2e
     rdm = wl.rdm_bytes()
     res["rdm"] = {"bytes_per_step": int(rdm), "achieved_gbs": rdm / (ms / 1e3) / 1e9,
-                  "frac_of_hbm": rdm / (ms / 1e3) / 1e9 / peak, "peak_kind": peak_kind}
+                  "frac_of_hbm": rdm / (ms / 1e3) / 1e9 / peak, "peak_kind": peak_kind,
+                  "what": "bytes of the model pipeline (24-byte records, every step over next_pow2(n) rows); a "
+                          "pipeline that moves fewer bytes reads above 1, and says nothing about the HBM it uses"}
     res["gpu_launches"] = int(wl.launches() * args.steps)
     return res
 
@@ -779,7 +781,7 @@ def roofline_of(torch, capi, wl, peak, peak_kind):
     achieved = dom["algorithmic_bytes_per_launch"] / (dom["avg_launch_us"] / 1e6) / 1e9
     return {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
             "peak_kind": f"{peak_kind} (MEASURED_PEAKS.json hbm_gbs)" if peak_kind == "measured" else "fallback",
-            "traffic": TRAFFIC.get(wl.key), "kernel": wl.kernel, "avg_launch_us": dom["avg_launch_us"],
+            "traffic": TRAFFIC.get(f"sort_2^{int(np.log2(wl.n))}" if isinstance(wl, SortKP) else wl.key), "kernel": wl.kernel, "avg_launch_us": dom["avg_launch_us"],
             "launches_per_step": dom["launches_per_step"],
             "algorithmic_bytes_per_launch": dom["algorithmic_bytes_per_launch"],
             "timing": "each pass bracketed by CUDA events on its stream (library pass timer), mean of 3 runs",

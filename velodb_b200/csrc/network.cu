@@ -266,8 +266,8 @@ static int default_log_e(int logN) { return logN <= DEFAULT_SMALL_LOGN ? 3 : 4; 
 
 // Sorts of up to 1024 padded rows are one CTA whose time is its shared-memory
 // traffic and its levels' latency, so the tile holds no more rows than it has
-// to: 512 rows of 64 threads, 1024 of 128 (n = 300: 13.6 -> 10.6 us, n = 1000:
-// 16.4 -> 13.4 us a call against 2048 rows of 256; 256 threads x 4 rows 14.4).
+// to: 512 rows of 64 threads, 1024 of 128 (n = 500: 10.8 -> 8.4 us, n = 1000: 13.8
+// -> 10.3 us a call against 2048 rows of 256).
 static velo_status sort_small(const RowKP::Cols& c, size_t n, int logN, cudaStream_t st)
 {
     std::vector<NetPass> passes;
