@@ -593,12 +593,8 @@ struct RowRec {
             ka[x] = KM == KEY_FULL ? a.w[x] : (a.w[x] & c.mask[x]);
             kb[x] = KM == KEY_FULL ? b.w[x] : (b.w[x] & c.mask[x]);
         }
-        if constexpr (KW == 1) {
-            if constexpr (STRICT)
-                return desc ? ka[0] < kb[0] : ka[0] > kb[0];
-            else
-                return (ka[0] > kb[0]) != desc;
-        }
+        if constexpr (KW == 1)
+            return STRICT ? ka[0] > kb[0] : (ka[0] > kb[0]) != desc; // (strict: Flip)
         if constexpr (STRICT) {
             const uint32_t gt = key_gt_mask<KW>(ka, kb);
             const uint32_t lt = key_gt_mask<KW>(kb, ka);
@@ -613,7 +609,7 @@ struct RowRec {
             r.w[0] ^= (uint64_t)m << 32;
         } else {
             r.w[0] ^= ((uint64_t)m << 32) | m;
-            if constexpr (W > 1)
+            if constexpr (KM == KEY_HI96)
                 r.w[1] ^= (uint64_t)m << 32;
         }
     }
@@ -643,10 +639,10 @@ template <>
 struct Flip<RowU2> {
     static constexpr bool on = true;
 };
-// strict records keyed on the high half of a word, the low half of the last
-// one being payload
-template <int W>
-struct Flip<RowRec<W, 1, true, KEY_HI32>> {
+// strict records keyed on bits of word 0 (masked, or its high half), or on word 0
+// and the high half of word 1
+template <int W, int KM>
+struct Flip<RowRec<W, 1, true, KM>> {
     static constexpr bool on = true;
 };
 template <>
