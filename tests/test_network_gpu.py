@@ -265,3 +265,22 @@ def test_pass_rows_leave_out_padding(cuda):
     assert got[0] == ("tile_sort", 22, h, tiles * 8192)
     assert got[-2:] == [("global", 22, 1 << 22, 1 << 22), ("merge", 22, 1 << 22, 1 << 22)]
     assert all(x[2:] == (tiles * 8192, tiles * 8192) for x in got[1:-2])
+
+
+# one wave of 128 tiles: all of them, in a trimmed sort where more than three
+# quarters hold rows (393,216 = 96 tiles)
+@pytest.mark.parametrize("n,whole", [(300_001, False), (393_216, False), (393_217, True), (500_000, True)])
+def test_sorts_of_one_wave(cuda, n, whole):
+    keys, pay = W.sort_kp(n, seed=n)
+    cap = 1 << 19
+    k, p = capi.to_dev_u64(keys, cap), capi.to_dev_u32(pay, cap)
+    rows = cap if whole else -(-n // 4096) * 4096
+    got = passes_of(lambda: capi.osort_kp(k, p, n))
+    assert all(x[3] == rows for x in got[1:])
+    o = np.lexsort((pay, keys))
+    assert np.array_equal(capi.host_u64(k, n), keys[o]) and np.array_equal(capi.host_u32(p, n), pay[o])
+    assert bool((k[n:] == -1).all()) and bool((p[n:] == -1).all())
+    w = capi.to_dev_u64(keys, cap)
+    got = passes_of(lambda: capi.osort_records([w], n, 2**64 - 1))
+    assert all(x[3] == cap for x in got)
+    assert np.array_equal(capi.host_u64(w, n), np.sort(keys))

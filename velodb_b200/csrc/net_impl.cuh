@@ -207,12 +207,13 @@ inline unsigned merge_pipe_grid(const typename R::Cols& c, size_t ntiles)
 }
 
 template <class R, int LOG_NT, int LOG_E>
-velo_status launch_net(const typename R::Cols& c, const NetGeom& g, const std::vector<NetPass>& passes,
+velo_status launch_net(const typename R::Cols& c, const NetGeom& geom, const std::vector<NetPass>& passes,
                        const uint32_t* tile_prefix, cudaStream_t st)
 {
     using N = Net<R, LOG_NT, LOG_E>;
     if (passes.empty())
         return VELO_OK;
+    const NetGeom g = net_launch_geom(geom, passes, N::LT);
     const bool compact = passes[0].kind == P_COMPACT_TILE || passes[0].kind == P_COMPACT_GLOBAL;
     constexpr int MB = net_min_blocks<R, LOG_NT>();
     constexpr int MBW = net_has_wide<R, LOG_NT>() ? 3 : MB;
