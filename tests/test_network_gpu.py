@@ -267,20 +267,35 @@ def test_pass_rows_leave_out_padding(cuda):
     assert all(x[2:] == (tiles * 8192, tiles * 8192) for x in got[1:-2])
 
 
-# one wave of 128 tiles: all of them, in a trimmed sort where more than three
-# quarters hold rows (393,216 = 96 tiles)
-@pytest.mark.parametrize("n,whole", [(300_001, False), (393_216, False), (393_217, True), (500_000, True)])
-def test_sorts_of_one_wave(cuda, n, whole):
+# one wave of 128 tiles: record sorts work on all of them, as do GROUP BY INTEGER
+# where more than 96 tiles (393,216 rows) hold rows and plain sorts where more than
+# 112 (458,752) do
+@pytest.mark.parametrize("n,whole,plain", [(262_145, 0, 0), (300_001, 0, 0), (393_216, 0, 0), (393_217, 1, 0),
+                                           (458_752, 1, 0), (458_753, 1, 1), (520_000, 1, 1), (1 << 19, 1, 1)])
+def test_sorts_of_one_wave(cuda, n, whole, plain):
     keys, pay = W.sort_kp(n, seed=n)
     cap = 1 << 19
-    k, p = capi.to_dev_u64(keys, cap), capi.to_dev_u32(pay, cap)
-    rows = cap if whole else -(-n // 4096) * 4096
-    got = passes_of(lambda: capi.osort_kp(k, p, n))
-    assert all(x[3] == rows for x in got[1:])
-    o = np.lexsort((pay, keys))
-    assert np.array_equal(capi.host_u64(k, n), keys[o]) and np.array_equal(capi.host_u32(p, n), pay[o])
-    assert bool((k[n:] == -1).all()) and bool((p[n:] == -1).all())
     w = capi.to_dev_u64(keys, cap)
     got = passes_of(lambda: capi.osort_records([w], n, 2**64 - 1))
     assert all(x[3] == cap for x in got)
-    assert np.array_equal(capi.host_u64(w, n), np.sort(keys))
+    assert np.array_equal(capi.host_u64(w, n), np.sort(keys)) and bool((w[n:] == -1).all())
+    k, p = capi.to_dev_u64(keys, cap), capi.to_dev_u32(pay, cap)
+    got = passes_of(lambda: capi.osort_kp(k, p, n))
+    assert all(x[3] == (cap if plain else -(-n // 4096) * 4096) for x in got[1:])
+    o = np.lexsort((pay, keys))
+    assert np.array_equal(capi.host_u64(k, n), keys[o]) and np.array_equal(capi.host_u32(p, n), pay[o])
+    assert bool((k[n:] == -1).all()) and bool((p[n:] == -1).all())
+    gk = (keys % np.uint64(1000)).astype(np.int32)
+    d = torch.from_numpy(gk).cuda()
+    v = torch.from_numpy(pay.astype(np.int64)).cuda()
+    out = []
+    got = passes_of(lambda: out.extend(capi.ogroupby(d, 4, n, sums=[v])))
+    rows = cap if whole else -(-n // 4096) * 4096
+    assert all(x[3] == rows for x in got if not x[0].startswith("compact"))
+    uk, inv = np.unique(gk, return_inverse=True)
+    s = np.zeros(len(uk), np.int64)
+    np.add.at(s, inv, pay.astype(np.int64))
+    m = len(uk)
+    assert out[3].tolist() == [m, 0] and np.array_equal(out[0].cpu().numpy()[:m], uk)
+    assert np.array_equal(out[1][0].cpu().numpy()[:m], s)
+    assert np.array_equal(out[2].cpu().numpy()[:m], np.bincount(inv))

@@ -43,6 +43,15 @@ constexpr bool net_has_wide() { return LOG_NT <= 8 && NetWide<R>::ok; }
 template <class R, int LOG_NT>
 constexpr bool net_has_wide_global() { return LOG_NT <= 8 && NetWide<R>::ok_global; }
 constexpr int NET_WIDE_LOGN = 21; // sorts of 2^21 rows and more take the three-CTA form
+// Grids of up to 296 CTAs fit on 148 SMs two by two.  Passes overlap their launch
+// with the tail of the one before, so where a pass's registers leave room for a
+// third CTA, its CTAs crowd the SMs that came free first and the others idle.  For
+// records of one word, whose global passes take 80 registers (96 before the loads
+// of a tile pass changed), a request for more shared memory than a third of an SM
+// has keeps it at two (us a call with 96 registers / 80 / 80 and this): 1 M rows 165 /
+// 171 / 155, 300,000 103 / 105 / 97.
+constexpr unsigned NET_TWO_CTA_GRID = 2 * 148;
+constexpr size_t NET_TWO_CTA_SMEM = 77 * 1024;
 
 // Passes of one sequence are launched with programmatic stream serialization:
 // the next pass may be launched while this one drains, and waits here until
@@ -207,13 +216,12 @@ inline unsigned merge_pipe_grid(const typename R::Cols& c, size_t ntiles)
 }
 
 template <class R, int LOG_NT, int LOG_E>
-velo_status launch_net(const typename R::Cols& c, const NetGeom& geom, const std::vector<NetPass>& passes,
+velo_status launch_net(const typename R::Cols& c, const NetGeom& g, const std::vector<NetPass>& passes,
                        const uint32_t* tile_prefix, cudaStream_t st)
 {
     using N = Net<R, LOG_NT, LOG_E>;
     if (passes.empty())
         return VELO_OK;
-    const NetGeom g = net_launch_geom(geom, passes, N::LT);
     const bool compact = passes[0].kind == P_COMPACT_TILE || passes[0].kind == P_COMPACT_GLOBAL;
     constexpr int MB = net_min_blocks<R, LOG_NT>();
     constexpr int MBW = net_has_wide<R, LOG_NT>() ? 3 : MB;
@@ -284,6 +292,9 @@ velo_status launch_net(const typename R::Cols& c, const NetGeom& geom, const std
         cfg.gridDim = dim3((unsigned)net_pass_tiles(g, passes[i], lt));
         cfg.blockDim = dim3(1u << LOG_NT);
         cfg.dynamicSmemBytes = smem;
+        // no third CTA on an SM where two on each hold the whole grid
+        if (sizeof(R) == 8 && LOG_NT == 8 && !compact && cfg.gridDim.x <= NET_TWO_CTA_GRID && smem < NET_TWO_CTA_SMEM)
+            cfg.dynamicSmemBytes = NET_TWO_CTA_SMEM;
         cfg.stream = st;
         cfg.attrs = attr;
         cfg.numAttrs = (i > 0 && !timer.on()) ? 1 : 0;

@@ -14,7 +14,6 @@
 #pragma once
 
 #include <type_traits>
-#include <vector>
 
 #include "engine.cuh"
 
@@ -109,28 +108,22 @@ __host__ __device__ inline size_t net_pass_tiles(const NetGeom& g, const NetPass
     return round_up_log2(m, p.kind == P_SORT_GLOBAL ? p.b_hi + 1 : lt) >> lt;
 }
 
-// The geometry in which the passes of a sort are launched.  A grid of up to 128
-// CTAs is one wave: leaving CTAs out shortens no pass, and the passes, which
-// overlap their launch with the tail of the one before, then find free SMs and
-// run two CTAs on some of them.  So a sort of at most 128 tiles works on all of
-// them, a trimmed one where more than three quarters of 128 hold rows (the whole
-// network needs a tile pass and arrays of 2^logN rows, which every sort has).
-// us a call without / with: records of one word, 300,000 rows 117 / 105, 400,000
-// 126 / 105, three words 200 / 177; ORDER BY (DOUBLE, DATE) 300,000 157 / 139;
-// PK-FK join of 400,000 rows 185 / 171; plain sort 500,000 114 / 108, 300,000 108 /
-// 108; GROUP BY INTEGER 500,000 202 / 182, 300,000 176 / 177.
-constexpr int NET_WAVE_LOG = 7;
-inline NetGeom net_launch_geom(const NetGeom& g, const std::vector<NetPass>& passes, int lt)
+// A sort's geometry on all of its tiles where they are 128, one wave: leaving CTAs
+// out shortens no pass there, and the passes, which overlap their launch with the
+// tail of the one before, then find free SMs and run two CTAs on some of them.  A
+// trimmed sort takes the whole network (its arrays hold 2^logN rows) where more
+// than `eighths` of the tiles hold rows.  Calls on several streams at once pay for
+// the padding, so only the sorts do this that leaving it out had made slower than
+// sorting it (us a call, before that / without this / with it): records of one
+// word, 400,000 rows 103 / 126 / 97, two words 134 / 141 / 125, three words 192 / 200 /
+// 177; GROUP BY INTEGER (6 eighths) 500,000 187 / 202 / 182, 300,000 187 / 176 / 177;
+// plain sort (7) 520,000 116 / 128 / 108, 400,000 116 / 114 / 114.
+inline NetGeom net_one_wave(const NetGeom& g, int lt, int eighths = 0)
 {
     const size_t np = (size_t)1 << g.logN;
-    if (passes[0].kind > P_SORT_GLOBAL || g.logN <= lt || g.logN - lt > NET_WAVE_LOG)
+    if (g.logN - lt != 7 || (g.m < np && g.m <= np / 8 * eighths))
         return g;
-    NetGeom w = g;
-    if (g.m < np) {
-        if (passes[0].kind != P_SORT_TILE || g.logN - lt < NET_WAVE_LOG || g.m <= np / 4 * 3)
-            return g;
-        w = NetGeom(g.n, g.logN);
-    }
+    NetGeom w(g.n, g.logN);
     w.live = np;
     return w;
 }

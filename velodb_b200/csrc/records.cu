@@ -27,12 +27,11 @@ static velo_status rec_sort(uint64_t* const* words, uint64_t mask, size_t n, int
     c.mark_inv = 0;
     c.mark_word = 0;
     std::vector<NetPass> passes;
-    NetGeom g { n, logN, 0 };
 #define X(a, b)                                                                                                        \
     if (log_nt == a && log_e == b) {                                                                                   \
         const int lt = a + b;                                                                                          \
         plan_sort(logN, lt, lt - 4 < 8 ? lt - 4 : 8, passes);                                                          \
-        return launch_net<R, a, b>(c, g, passes, nullptr, st);                                                         \
+        return launch_net<R, a, b>(c, net_one_wave(NetGeom(n, logN), lt), passes, nullptr, st);                        \
     }
     VELO_FOR_REC_TUNES(X)
 #undef X
