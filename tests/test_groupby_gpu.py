@@ -164,14 +164,15 @@ def test_revealed_count_in_a_captured_stream(cuda):
     assert torch.equal(out, want[0]) and torch.equal(counts, want[1])
 
 
-# key words at the edges of the tile rule (2^11, 2^12 of one tile; 2^18 | 2^19 and
-# 2^21 | 2^22 of the next tile)
-@pytest.mark.parametrize("words", [2047, 2048, 2049, 4096, 4097, 1 << 18, (1 << 18) + 1, 1 << 21, (1 << 21) + 1])
+# key words at the edges of the tile rules (2^11, 2^12 of one tile; with the count
+# revealed 2^18 | 2^19 and 2^21 | 2^22 of the next tile)
+@pytest.mark.parametrize("words", [2047, 2048, 2049, 4096, 4097, 8193, 1 << 18, (1 << 18) + 1, 1 << 21, (1 << 21) + 1])
 @pytest.mark.parametrize("odd", [0, 1])
-def test_filter_groupby_key_tiles(cuda, words, odd):
+@pytest.mark.parametrize("reveal", [False, True])
+def test_filter_groupby_key_tiles(cuda, words, odd, reveal):
     n = 2 * words - odd
     c = rows_passing(n, n - n // 5, tuple(range(0, 65536, 4369)), seed=n)
-    out, counts = run_gpu(c, ANY, 16)
+    out, counts = run_gpu(c, ANY, 16, reveal)
     key = c["flag1"].astype(np.int64) * 256 + c["flag2"]
     ok = c["shipdate"] == 10
     keys, num = np.unique(key[ok], return_counts=True)

@@ -39,11 +39,20 @@
 namespace velo {
 
 // log2 of the key words a tile holds, 256 threads of 8, 16 or 32 words, for the
-// network over 2^log_words of them: small ones want more CTAs, large ones fewer
-// passes.  A call with 11 / 12 / 13 (us, 8 groups): 12,000 rows (2^13 words) 60 / 67
-// / 71, 70,001 (2^16) 78 / 86 / 107, 300,000 (2^18) 92 / 100 / 129, 1 M (2^19) 138 /
-// 131 / 146, 3 M (2^21) 281 / 256 / 261, 6 M (2^22) 542 / 436 / 421.
-static int lk_lt(int log_words) { return log_words <= 18 ? 11 : log_words <= 21 ? 12 : 13; }
+// network over 2^log_words of them.  One tile of up to 4096 words is no larger than
+// it has to be (a call of 5,000 rows 59 -> 44 us).  Beyond that smaller tiles shorten
+// a call, but their passes are more work: with the count revealed, where a call
+// waits for its own result, 2048 words up to 2^18 and 4096 up to 2^21 (with 11 / 12 /
+// 13, us, 8 groups: 12,000 rows 60 / 67 / 71, 70,001 78 / 86 / 107, 300,000 92 / 100 /
+// 129, 1 M 138 / 131 / 146, 3 M 281 / 256 / 261, 6 M 542 / 436 / 421); else 8192, which
+// serves more queries a second on several streams (16 streams, 2^14..2^18 rows:
+// 12,400 against 11,700).
+static int lk_lt(int log_words, bool reveal)
+{
+    if (log_words <= 12)
+        return log_words <= 11 ? 11 : 12;
+    return !reveal || log_words > 21 ? 13 : log_words <= 18 ? 11 : 12;
+}
 constexpr unsigned LK_MAX_BLOCKS = 148 * 8;
 // the sums: 8 slots a thread take 72 registers of sums
 constexpr int LK_SLOTS = 8, LKS_THREADS = 128, LKS_CTAS = 3;
@@ -89,9 +98,9 @@ __global__ void __launch_bounds__(LKS_THREADS, LKS_CTAS) k_li_sums(LiCols c, vel
 }
 
 // the sort of h key words, or the last merge of 2^logN words
-static velo_status lk_net(uint32_t* keys, size_t h, int logN, bool merge, cudaStream_t st)
+static velo_status lk_net(uint32_t* keys, size_t h, int logN, bool merge, bool reveal, cudaStream_t st)
 {
-    const int lt = merge && logN == 12 ? 12 : lk_lt(logN); // (4096 words: one pass)
+    const int lt = lk_lt(logN, reveal);
     std::vector<NetPass> passes;
     if (merge)
         plan_merge(logN, lt, lt - 4, logN, passes);
@@ -172,14 +181,14 @@ static velo_status run_groupby(const LiScratch& s, const LiCols& c, size_t n, co
             return rc;
     }
     if (q.h > 1) {
-        const velo_status rc = lk_net(q.ka, q.h, q.logH, false, st);
+        const velo_status rc = lk_net(q.ka, q.h, q.logH, false, reveal, st);
         if (rc != VELO_OK)
             return rc;
     }
     k_li_fold<<<(unsigned)(q.N / LK_ROWS < LK_MAX_BLOCKS ? q.N / LK_ROWS : LK_MAX_BLOCKS), LK_THREADS, 0, st>>>(q);
     VELO_CUDA_TRY(cudaGetLastError(), "group-by fold launch");
     {
-        const velo_status rc = lk_net(q.kb, q.N, q.logN, true, st);
+        const velo_status rc = lk_net(q.kb, q.N, q.logN, true, reveal, st);
         if (rc != VELO_OK)
             return rc;
     }
