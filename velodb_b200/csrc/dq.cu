@@ -302,7 +302,9 @@ velo_status dq_plan_filter_groupby(DqPlan& p, const velo_lineitem* cols, size_t 
     a.c = c;
     a.p = *pred;
     a.n = n;
-    a.q = lk_plan(s, n, DQ_LK_LT, 0xFFFFFFFFu);
+    // up to 4096 key words: one search tile, half of a key tile
+    const int lt = (n + 1) / 2 <= (size_t)LK_TS ? ilog2_floor(LK_TS) : DQ_LK_LT;
+    a.q = lk_plan(s, n, lt, 0xFFFFFFFFu);
     a.out = d_out;
     a.d_counts = d_counts;
     a.G = (int)group_bound;
@@ -320,7 +322,8 @@ velo_status dq_plan_filter_groupby(DqPlan& p, const velo_lineitem* cols, size_t 
     std::vector<NetPass> mp;
     plan_merge(q.logN, DQ_LK_LT, LK_LMAX, q.logN, mp);
     b.net<RowU2>(DQ_K_SORT_U2, RowU2::Cols { q.kb }, NetGeom(q.N, q.logN), nullptr, mp, DQ_LK_LT);
-    b.step(DQ_K_LI_DISTINCT, (uint64_t)q.ntiles, ao);
+    if (q.ntiles > 1)
+        b.step(DQ_K_LI_DISTINCT, (uint64_t)q.ntiles, ao);
     b.step(DQ_K_LI_SLOTS, (uint64_t)q.ntiles, ao);
     b.step(DQ_K_LI_SUMS, (n + DQ_ELEM_ITEM - 1) / DQ_ELEM_ITEM * (uint64_t)a.chunks, ao);
     return VELO_OK;

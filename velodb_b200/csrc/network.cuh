@@ -658,7 +658,7 @@ struct Net {
                 const size_t gi = gidx(tp | (e << s));
                 if (first)
                     v[e] = (gi < g.n) ? R::load(c, gi) : R::pad(c);
-                else if (SORT && is_global)
+                else if (SORT && (is_global || PK == PK_ANY)) // (PK_ANY: a merge of less than a tile)
                     v[e] = (gi < Np) ? R::load(c, gi) : R::pad(c);
                 else
                     v[e] = R::load(c, gi);
