@@ -40,7 +40,7 @@ namespace velo {
 
 // log2 of the key words a tile holds, 256 threads of 8, 16 or 32 words, for the
 // network over 2^log_words of them.  One tile of up to 4096 words is no larger than
-// it has to be (a call of 5,000 rows 59 -> 44 us).  Beyond that smaller tiles shorten
+// it has to be (a call of 5,000 rows 59 -> 47 us).  Beyond that smaller tiles shorten
 // a call, but their passes are more work: with the count revealed, where a call
 // waits for its own result, 2048 words up to 2^18 and 4096 up to 2^21 (with 11 / 12 /
 // 13, us, 8 groups: 12,000 rows 60 / 67 / 71, 70,001 78 / 86 / 107, 300,000 92 / 100 /
@@ -126,11 +126,11 @@ __global__ void __launch_bounds__(1024) k_li_rows(LkPlan q)
 // With the count revealed (VELO_REVEAL_COUNT): when next_pow2(rows passing) is at
 // most half of the 2^logH key words, the words that hold such a row are compacted
 // to the front and `rows` words are sorted in the place of all h.  The count
-// costs a copy to the host (about 17 us), so calls below 2^19 words, whose whole
-// sort takes 45 us and less, do without it.
+// costs a copy to the host (about 17 us), so calls of at most 2^18 words, whose
+// whole sort takes 45 us and less in small tiles, do without it.
 // Revealed / not / 16-byte records compacted and sorted (us, 8 groups), 2 % of the
-// rows passing: 600,000 rows 114 / 114 / 133, 1 M 124 / 131 / 145, 3 M 182 / 255 /
-// 250, 6,001,215 261 / 420 / 405; 0.2 %: 96 / 131 / 109 at 1 M; 50 %: 435 / 420 /
+// rows passing: 600,000 rows 113 / 142 / 133, 1 M 119 / 146 / 145, 3 M 172 / 258 /
+// 250, 6,001,215 262 / 420 / 405; 0.2 %: 94 / 146 / 109 at 1 M; 50 %: 435 / 420 /
 // 1,087 at 6,001,215.
 constexpr int LK_REVEAL_LOGH = 19;
 
