@@ -172,7 +172,7 @@ __device__ void dq_run(const DqStep& step, const unsigned char* s_args, uint32_t
     // ---- filter + group-by
     case DQ_K_SORT_U2: {
         const auto& A = dq_arg<DqNetArgs<RowU2>>(s_args);
-        NetU2::run<true>(A.c, A.g, step.pass, nullptr, (int)tile, sm);
+        NetU2::run<true, NetU2::PK_PART>(A.c, A.g, step.pass, nullptr, (int)tile, sm);
         break;
     }
     case DQ_K_LI_KEYS: {

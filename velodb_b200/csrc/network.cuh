@@ -110,14 +110,16 @@ __host__ __device__ inline size_t net_pass_tiles(const NetGeom& g, const NetPass
 
 // A sort's geometry on all of its tiles where they are 128, one wave: leaving CTAs
 // out shortens no pass there, and the passes, which overlap their launch with the
-// tail of the one before, then find free SMs and run two CTAs on some of them.  A
-// trimmed sort takes the whole network (its arrays hold 2^logN rows) where more
-// than `eighths` of the tiles hold rows.  Calls on several streams at once pay for
-// the padding, so only the sorts do this that leaving it out had made slower than
-// sorting it (us a call, before that / without this / with it): records of one
-// word, 400,000 rows 103 / 126 / 97, two words 134 / 141 / 125, three words 192 / 200 /
-// 177; GROUP BY INTEGER (6 eighths) 500,000 187 / 202 / 182, 300,000 187 / 176 / 177;
-// plain sort (7) 520,000 116 / 128 / 108, 400,000 116 / 114 / 114.
+// tail of the one before, then find free SMs and run two CTAs on some of them (the
+// more so with an odd number of tiles, whose global passes hold CTAs without a
+// pair).  A trimmed sort takes the whole network (its arrays hold 2^logN rows)
+// where more than `eighths` of the tiles hold rows.  Calls on several streams at
+// once pay for the padding, so only the sorts do this that leaving it out had made
+// slower than sorting it (us a call, before that / without this / with it): records
+// of one word, 98 tiles 103 / 126 / 97, two words 134 / 141 / 125, three words 192 / 200 /
+// 177; GROUP BY INTEGER (5 eighths) 85 tiles 188 / 198 / 178, 127 188 / 203 / 180, 73 188 /
+// 173 / 175; hash join (5) 66 k x 131 k 456 / 469 / 446; plain sort (6) 97 tiles 116 / 126 /
+// 107, 127 116 / 128 / 107, 94 116 / 111 / 107.
 inline NetGeom net_one_wave(const NetGeom& g, int lt, int eighths = 0)
 {
     const size_t np = (size_t)1 << g.logN;
@@ -598,8 +600,9 @@ struct Net {
     // ST (not void): the pass's rows are already in shared memory in local
     // row order, staged by a tensor-map tile load; ST::read(sm, T, l) reads
     // row l (merge and fused global passes only)
-    // PK_MERGE: the in-tile merges alone (no tile-sort code)
-    enum : int { PK_ANY = 0, PK_LOCAL = 1, PK_GLOBAL = 2, PK_MERGE = 3 };
+    // PK_MERGE: the in-tile merges alone (no tile-sort code); PK_PART: as PK_ANY,
+    // merges of less than a tile among them
+    enum : int { PK_ANY = 0, PK_LOCAL = 1, PK_GLOBAL = 2, PK_MERGE = 3, PK_PART = 4 };
     template <bool SORT, int PK = PK_ANY, bool WIDE = false, class ST = void>
     __device__ static void run(const Cols& c, const NetGeom& g, const NetPass& p, const uint32_t* tile_prefix,
                                int cta, char* sm)
@@ -658,7 +661,7 @@ struct Net {
                 const size_t gi = gidx(tp | (e << s));
                 if (first)
                     v[e] = (gi < g.n) ? R::load(c, gi) : R::pad(c);
-                else if (SORT && (is_global || PK == PK_ANY)) // (PK_ANY: a merge of less than a tile)
+                else if (SORT && (is_global || PK == PK_PART))
                     v[e] = (gi < Np) ? R::load(c, gi) : R::pad(c);
                 else
                     v[e] = R::load(c, gi);
