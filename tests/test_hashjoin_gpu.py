@@ -73,3 +73,20 @@ def test_hash_join_reports_bin_overflow(cuda, orc):
     probe = np.full(200_000, dim["key"][7], np.int32)  # one hot key: its bin overflows
     _, _, cnt = run(dim["key"], None, probe, None)
     assert int(cnt[2]) > 0
+
+
+# 2^19 rows with the padding of the bins: the sort works on all of its 128 tiles
+@pytest.mark.parametrize("nd,nf", [(61_166, 122_334), (65_601, 131_203), (74_274, 148_548)])
+def test_hash_join_sort_of_one_wave(cuda, orc, nd, nf):
+    dim, fact = W.join_tables(nd, nf, seed=nd)
+    check(orc, dim["key"], None, fact["fk"], None)
+    bk, pk = (torch.from_numpy(x).cuda() for x in (dim["key"], fact["fk"]))
+    capi.set_pass_timing(True)
+    try:
+        capi.clear_pass_times()
+        capi.ohash_join(bk, None, pk, None, INTEGER)
+        passes = list(zip(capi.last_pass_times(), capi.last_pass_rows()))
+    finally:
+        capi.set_pass_timing(False)
+    sort = [(t[1], rows[1]) for t, rows in passes if not t[0].startswith("compact")]
+    assert all(w == 1 << lg for lg, w in sort if lg == 19)

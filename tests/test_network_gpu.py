@@ -268,10 +268,10 @@ def test_pass_rows_leave_out_padding(cuda):
 
 
 # one wave of 128 tiles: record sorts work on all of them, as do GROUP BY INTEGER
-# where more than 96 tiles (393,216 rows) hold rows and plain sorts where more than
-# 112 (458,752) do
-@pytest.mark.parametrize("n,whole,plain", [(262_145, 0, 0), (300_001, 0, 0), (393_216, 0, 0), (393_217, 1, 0),
-                                           (458_752, 1, 0), (458_753, 1, 1), (520_000, 1, 1), (1 << 19, 1, 1)])
+# where more than 80 tiles (327,680 rows) hold rows and plain sorts where more than
+# 96 (393,216) do
+@pytest.mark.parametrize("n,whole,plain", [(262_145, 0, 0), (300_001, 0, 0), (327_680, 0, 0), (327_681, 1, 0),
+                                           (393_216, 1, 0), (393_217, 1, 1), (520_000, 1, 1), (1 << 19, 1, 1)])
 def test_sorts_of_one_wave(cuda, n, whole, plain):
     keys, pay = W.sort_kp(n, seed=n)
     cap = 1 << 19

@@ -406,7 +406,7 @@ static velo_status gb_run(const GbScratch& s, const GbIn& in, size_t n, size_t b
     rc.mark_bit = 63;
     rc.mark_inv = 1;
     rc.mark_word = 0;
-    velo_status rc2 = launch_sort<typename T::Rec>(rc, net_one_wave(geom, sort_lt(logN), 6), st);
+    velo_status rc2 = launch_sort<typename T::Rec>(rc, net_one_wave(geom, sort_lt(logN), 5), st);
     if (rc2 != VELO_OK)
         return rc2;
 

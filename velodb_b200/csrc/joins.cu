@@ -867,7 +867,8 @@ extern "C" velo_status velo_ohash_join(const void* d_build_keys, const uint8_t* 
     plan_sort(logR, OP_LT, OP_LMAX, passes);
     // every row's bin, side and row or slot number are its own
     velo_status rc =
-        launch_net12<HjRec>(c, NetGeom::trimmed(build_n + probe_n + g.slots, logR, OP_LT, 0), passes, nullptr, st);
+        launch_net12<HjRec>(c, net_one_wave(NetGeom::trimmed(build_n + probe_n + g.slots, logR, OP_LT, 0), OP_LT, 5),
+                            passes, nullptr, st);
     if (rc != VELO_OK)
         return rc;
     const int nt = (int)(g.rows / MN_TS);

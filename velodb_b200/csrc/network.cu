@@ -35,7 +35,7 @@ static velo_status sort_dispatch(const typename R::Cols& c, size_t n, int logN, 
     if (log_nt == a && log_e == b) {                                                                                   \
         const int lt = a + b;                                                                                          \
         plan_sort(logN, lt, lt - 4 < 8 ? lt - 4 : 8, passes);                                                          \
-        return launch_net<R, a, b>(c, net_one_wave(NetGeom::trimmed(n, logN, lt, fill), lt, 7), passes, nullptr, st);  \
+        return launch_net<R, a, b>(c, net_one_wave(NetGeom::trimmed(n, logN, lt, fill), lt, 6), passes, nullptr, st);  \
     }
     VELO_FOR_TUNES(X)
 #undef X
